@@ -47,7 +47,7 @@ LIB_SOURCES = [
     "pr.cu",
     "mis.cu",
 ]
-HEADERS = ["gft_internal.h", "gen_common.h", "traverse.cuh", "frontier.cuh", "job.cuh"]
+HEADERS = ["gft_internal.h", "gen_common.h", "traverse.cuh", "frontier.cuh", "job.cuh", "pr_pull.cuh"]
 CLI_SOURCE = "cli_main.cpp"
 
 NVCC_FLAGS = [

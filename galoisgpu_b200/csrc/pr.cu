@@ -1,5 +1,7 @@
-// pr.cu -- PageRank by residual push (gft_pr): the reference's apps/pr on
-// the engine's frontier core.
+// pr.cu -- PageRank (gft_pr): the reference's apps/pr on the engine's
+// frontier core.  A graph whose edges prove symmetric takes pulled sweeps
+// (pr_pull.cuh); a directed one, and a call with an iteration limit, takes
+// the residual pushes below.
 //
 // The reference (apps/pr/kernel.cu) keeps a rank and a residual per vertex:
 //   init   rank = 1 - ALPHA; every vertex adds (float)(1.0 / outdeg) to its
@@ -33,6 +35,7 @@
 
 #include "frontier.cuh"
 #include "gft_internal.h"
+#include "pr_pull.cuh"
 
 namespace gft {
 namespace dev {
@@ -312,6 +315,99 @@ const void *pr_kernel_for(int block)
     return nullptr;
 }
 
+// The pull path (pr_pull.cuh).  *done says whether it has written the ranks:
+// a graph that is not symmetric, or whose renumbered rows find no room in
+// device memory, is left to the pushes.
+gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t timeout_ms, cudaStream_t stream,
+                    gft_stats *stats, bool *done)
+{
+    *done = false;
+    const uint64_t n = G.nnodes, m = G.nedges;
+    // Quads of the renumbered rows: at most deg / 4 + 3/4 per row with edges,
+    // padded by at most 1/8.
+    const uint64_t quads = (m / 4 + std::min(n, m)) * 9 / 8 + 64;
+    if (quads >> 32) return GFT_OK;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    const size_t vec = (n + 8) * 4;
+    const size_t o_st = take(sizeof(dev::PullState)), o_perm = take(vec), o_num = take(vec), o_inv = take(vec),
+                 o_x0 = take(vec), o_x1 = take(vec), o_y0 = take(vec), o_y1 = take(vec), o_quads = take(quads * 16);
+    if (e->scratch.ensure(off) != GFT_OK) {
+        clear_error();
+        return GFT_OK;
+    }
+    char *base = static_cast<char *>(e->scratch.ptr);
+    dev::PullParams p{};
+    p.row_start = G.row_start;
+    p.edge_dst = G.edge_dst;
+    p.nnodes = G.nnodes;
+    p.nedges = G.nedges;
+    p.rank = d_rank;
+    p.perm = reinterpret_cast<uint32_t *>(base + o_perm);
+    p.number = reinterpret_cast<uint32_t *>(base + o_num);
+    p.inv_deg = reinterpret_cast<float *>(base + o_inv);
+    p.x[0] = reinterpret_cast<float *>(base + o_x0);
+    p.x[1] = reinterpret_cast<float *>(base + o_x1);
+    p.y[0] = reinterpret_cast<float *>(base + o_y0);
+    p.y[1] = reinterpret_cast<float *>(base + o_y1);
+    p.quads = reinterpret_cast<uint4 *>(base + o_quads);
+    p.st = reinterpret_cast<dev::PullState *>(base + o_st);
+    p.ctl = reinterpret_cast<TraversalCtl *>(e->ctl.ptr);
+    p.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
+    // A small graph's sweep is a few microseconds: CTAs without work only
+    // lengthen its barrier.
+    const int blocks = (int)std::min<uint64_t>(e->sms, (n + m / 4) / 2048 + 1);
+    const size_t hub_bytes = dev::kPullHub * sizeof(float);
+    const void *kern = (const void *)dev::pr_sweeps;
+    GFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hub_bytes));
+    GFT_CUDA_TRY(cudaMemsetAsync(e->ctl.ptr, 0, sizeof(TraversalCtl), stream));
+    GFT_CUDA_TRY(cudaMemsetAsync(p.st, 0, sizeof(dev::PullState), stream));
+    GFT_CUDA_TRY(cudaEventRecord(e->ev0, stream));
+    dev::pr_sample<<<dev::kPullSamples / 8, 256, 0, stream>>>(p);
+    GFT_CUDA_TRY(cudaGetLastError());
+    const int vblocks = (int)std::min<uint64_t>(2 * (uint64_t)e->sms, n / dev::kPullTile + 1);
+    dev::pr_classes<<<vblocks, 1024, 0, stream>>>(p);
+    GFT_CUDA_TRY(cudaGetLastError());
+    dev::pr_place<<<vblocks, 1024, 0, stream>>>(p);
+    GFT_CUDA_TRY(cudaGetLastError());
+    dev::pr_relabel<<<(int)std::min<uint64_t>(3 * (uint64_t)e->sms, (n + m / 4) / 1024 + 1), 512, 0, stream>>>(p);
+    GFT_CUDA_TRY(cudaGetLastError());
+    void *args[] = {&p};
+    GFT_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(dev::kPullBlock), args, hub_bytes, stream));
+    GFT_CUDA_TRY(cudaEventRecord(e->ev1, stream));
+    TraversalCtl *h = reinterpret_cast<TraversalCtl *>(e->host_ctl);
+    const size_t cold = offsetof(TraversalCtl, error);
+    unsigned asymmetric = 0;
+    GFT_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<char *>(h) + cold, reinterpret_cast<char *>(e->ctl.ptr) + cold,
+                                 sizeof(TraversalCtl) - cold, cudaMemcpyDeviceToHost, stream));
+    GFT_CUDA_TRY(cudaMemcpyAsync(h, &p.st->asymmetric, sizeof asymmetric, cudaMemcpyDeviceToHost, stream));
+    GFT_CUDA_TRY(cudaStreamSynchronize(stream));
+    memcpy(&asymmetric, h, sizeof asymmetric);
+    if (h->error)
+        return fail((gft_status)h->error, "gft_pr: device reported %s (site %u)", gft_status_string((gft_status)h->error),
+                    h->error_where);
+    if (asymmetric) return GFT_OK;
+    *done = true;
+    if (stats) {
+        memset(stats, 0, sizeof *stats);
+        float ms = 0;
+        cudaEventElapsedTime(&ms, e->ev0, e->ev1);
+        stats->levels = h->levels;
+        stats->iterations = h->iterations;
+        stats->vertices_reached = G.nnodes;
+        stats->edges_scanned = h->edges;
+        stats->pushes = h->pushes;
+        stats->kernel_ms = ms;
+        stats->grid_blocks = blocks;
+        stats->block_threads = dev::kPullBlock;
+    }
+    return GFT_OK;
+}
+
 gft_status run_pr(gft_engine *e, const gft_graph *g, float *d_rank, uint32_t max_iterations, const gft_tuning *tune,
                   cudaStream_t stream, gft_stats *stats)
 {
@@ -325,6 +421,14 @@ gft_status run_pr(gft_engine *e, const gft_graph *g, float *d_rank, uint32_t max
     if (!kern) return fail(GFT_ERR_INVALID_ARG, "gft_pr: block_threads must be 256, 512 or 1024");
     DeviceScope device_scope(e->device);
     GFT_CUDA_TRY(device_scope.err);
+    const uint32_t timeout_ms = (tune && tune->timeout_ms) ? tune->timeout_ms : 20000;
+    // A call that asks for so many rounds gets rounds of pushes: their partial
+    // sums are what the reference's -x option prints.
+    if (max_iterations == UINT32_MAX && G.nnodes && G.nedges) {
+        bool done = false;
+        GFT_TRY(run_pull(e, G, d_rank, timeout_ms, stream, stats, &done));
+        if (done) return GFT_OK;
+    }
     LaunchShape shape;
     GFT_TRY(resolve_shape(e, kern, block, bps, 0, &shape));
     const uint32_t n = G.nnodes;
@@ -351,7 +455,7 @@ gft_status run_pr(gft_engine *e, const gft_graph *g, float *d_rank, uint32_t max
     p.hub_degree = hub;
     p.qcap = n;
     p.ctl = reinterpret_cast<TraversalCtl *>(e->ctl.ptr);
-    p.timeout_ns = (unsigned long long)((tune && tune->timeout_ms) ? tune->timeout_ms : 20000) * 1000000ull;
+    p.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
     p.skip_block = -1;
     p.vec_ok = (uintptr_t)G.edge_dst % 16 == 0;
     p.nedges = G.nedges;

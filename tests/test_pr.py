@@ -144,3 +144,65 @@ def test_pr_cli_and_dropin_match_reference(gft, tmp_path, key):
     dropin = ROOT / "oracle" / "_ref" / "pr_gft"
     if dropin.exists():
         assert close(_run_pr_cli(dropin, key, tmp_path, gft), PR_VALUES[key])
+
+
+def _pull_cases():
+    """Symmetric graphs at the pull path's edges: rows of 0..40 edges (every
+    number of lanes per row and its padding), rows around the sizes a warp and
+    a whole CTA sum, duplicate edges, self loops."""
+    rng = np.random.default_rng(5)
+    n = 900
+    pairs = [(int(u), int(v)) for u in range(41) for v in rng.choice(np.arange(41, n), size=u, replace=False)]
+    yield "rows0to40", n, pairs
+    yield "pair", 2, [(0, 1)]
+    yield "lonely", 5, []
+    yield "dups_loops", 40, [(int(a), int(b)) for a, b in rng.integers(0, 40, size=(300, 2))]
+    for leaves in (127, 128, 2047, 2048, 4096, 9000, 70000):
+        yield f"star{leaves}", leaves + 3, [(1, i) for i in range(2, leaves + 2)]
+
+
+def _csr(n, src, dst):
+    order = np.argsort(src, kind="stable")
+    return np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint32), dst[order].astype(np.uint32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", list(_pull_cases()), ids=lambda c: c[0])
+def test_gpu_pr_pulled_rows(gft, engine, case):
+    """Ranks against the 64-bit solution of the rank equation.  A sweep ends
+    the iteration once no rank moves by more than 1e-6 of max(1, rank), and
+    the remaining error is below 1.3 times the last move (the sweeps gain a
+    factor 0.56); a rank's own 32-bit rounding adds less than 1e-6."""
+    _, n, pairs = case
+    a = np.array(pairs, dtype=np.int64).reshape(-1, 2)
+    src, dst = np.concatenate([a[:, 0], a[:, 1]]), np.concatenate([a[:, 1], a[:, 0]])
+    rs, ed = _csr(n, src, dst)
+    deg = np.diff(rs.astype(np.int64)).astype(np.float64)
+    want = np.full(n, 0.15)
+    for _ in range(250):
+        y = want / np.maximum(deg, 1)
+        want = 0.15 + 0.85 * np.bincount(dst, weights=y[src], minlength=n) if len(src) else want
+    for symmetric in (False, True):
+        dg = gft.CSRGraph(rs, ed).copy_to_gpu()
+        dg.symmetric = symmetric
+        got = engine.pr(dg)["out"].cpu().numpy().astype(np.float64)
+        assert np.all(np.abs(got - want) <= 2.5e-6 * np.maximum(1.0, want))
+
+
+@pytest.mark.gpu
+def test_gpu_pr_pushes_on_graphs_that_are_not_symmetric(gft, orc, engine):
+    """A directed graph with hubs, a symmetric one with a single edge
+    doubled in one direction (every edge still has a reverse), and a marked
+    directed one all take the pushes and match the oracle."""
+    rng = np.random.default_rng(6)
+    n, m = 20000, 160000
+    src = (n * rng.random(m) ** 3).astype(np.int64)
+    dst = (n * rng.random(m) ** 2).astype(np.int64)
+    g = gft.CSRGraph(*_csr(n, src, dst))
+    s2, d2 = np.concatenate([src, dst, src[:1]]), np.concatenate([dst, src, dst[:1]])
+    for graph, mark in ((g, False), (gft.CSRGraph(*_csr(n, s2, d2)), False), (g, True)):
+        dg = graph.copy_to_gpu()
+        dg.symmetric = mark
+        r = engine.pr(dg)
+        want, _ = orc.pr(graph.row_start, graph.edge_dst)
+        assert close(r["out"].cpu().numpy(), want)
