@@ -39,24 +39,31 @@ namespace dev {
 constexpr uint32_t kCcHubDegree = 2048;  // vertices with at least this many edges are split into chunks
 constexpr uint32_t kCcHubChunk = 2048;
 
-// Root of x.  Parent links are read from L2 (other SMs change them) and
-// halved on the way: label[x] <- label[label[x]], an ancestor of x at the
-// time of the read and therefore forever (trees only grow at the root).
+// A vertex that was x's root.  Parent links are read through L1: every find
+// ends at a root, most of them at the giant component's, and reads of one
+// address from all SMs queue up in its L2 slice (RMAT-23, whole call: 1.39 ms
+// with reads from L2, 0.54 ms through L1).  An SM may so see a link that has changed
+// since, but it is still one to an ancestor (trees only grow at the root), and
+// cc_union finds out by its compare-and-swap.  Links are halved on the way:
+// label[x] <- label[label[x]], an ancestor of x at the time of the read and
+// therefore forever.
 __device__ __forceinline__ uint32_t cc_find(uint32_t *label, uint32_t x)
 {
-    uint32_t p = __ldcg(label + x);
+    uint32_t p = __ldca(label + x);
     while (p != x) {
-        const uint32_t g = __ldcg(label + p);
+        const uint32_t g = __ldca(label + p);
         if (g == p) return p;
         label[x] = g;
         x = g;
-        p = __ldcg(label + x);
+        p = __ldca(label + x);
     }
     return x;
 }
 
 // Joins the components of u and v; the larger root is linked under the
-// smaller one.
+// smaller one.  When b is no longer a root the swap returns its parent,
+// which is smaller, so the union ends; when a no longer is, b's tree hangs
+// below a, in a's component all the same.
 __device__ __forceinline__ void cc_union(uint32_t *label, uint32_t u, uint32_t v)
 {
     uint32_t a = cc_find(label, u), b = cc_find(label, v);
@@ -196,7 +203,7 @@ __global__ void cc_flatten(uint32_t *label, uint32_t n)
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     for (uint32_t v = tid; v < n; v += nthreads) {
         uint32_t r = v, p;
-        while ((p = __ldcg(label + r)) != r) r = p;
+        while ((p = __ldca(label + r)) != r) r = p;
         label[v] = r;
     }
 }
@@ -234,7 +241,7 @@ __global__ void cc_compress(uint32_t *label, uint32_t n, unsigned long long *cou
     unsigned long long roots = 0;
     for (uint32_t v = tid; v < n; v += nthreads) {
         uint32_t r = v, p;
-        while ((p = __ldcg(label + r)) != r) r = p;
+        while ((p = __ldca(label + r)) != r) r = p;
         label[v] = r;
         roots += r == v;
     }
