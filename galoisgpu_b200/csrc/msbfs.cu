@@ -24,6 +24,12 @@
 //             ones together.  Uses v's out-edges as its in-edges, so it
 //             requires a symmetric graph (flag GFT_MSBFS_SYMMETRIC); without
 //             the flag every level runs top-down.
+// In either direction a vertex of kHubDegree edges or more goes to a hub list,
+// whose edges all warps of the grid then take in kHubEdges-edge chunks: with
+// one warp per vertex most of a level was the grid waiting for the largest
+// ones (256 sources on RMAT-20, levels of eight sources read back: 4.79 ->
+// 1.52 ms, with the frontier rows reduced by one instruction per word
+// instead of five shuffles, and the source set-up by a CTA instead of a thread).
 #include <string.h>
 
 #include <algorithm>
@@ -35,6 +41,8 @@ namespace gft {
 namespace dev {
 
 constexpr uint32_t kThreadDegree = 32;  // bottom-up: larger vertices are scanned by the whole warp
+constexpr uint32_t kHubDegree = 1024;   // either direction: larger vertices are scanned by the whole grid
+constexpr uint32_t kHubEdges = 512;     // edges of a hub per warp step
 
 // A row of WP words of source bits.
 template <int WP>
@@ -111,6 +119,8 @@ struct MsParams {
     uint32_t *queue[2];        // frontier vertices per level
     uint32_t *touched;         // top-down: vertices given new bits
     uint32_t *tstamp;          // top-down: level + 1 at which v was last touched
+    uint2 *hubs;               // (vertex, first chunk) of the level's hubs
+    uint32_t hub_cap;
     uint32_t symmetric;
     uint32_t alpha;            // bottom-up when m_f * alpha > nedges
     TraversalCtl *ctl;
@@ -126,6 +136,99 @@ __device__ __forceinline__ Bits<WP> all_sources(uint32_t k)
     for (int i = 0; i < WP; i++)
         b.w[i] = 32u * (i + 1) <= k ? ~0u : (32u * i >= k ? 0u : (1u << (k % 32)) - 1u);
     return b;
+}
+
+// The sources that `need` lacks and that stand in frontier rows of the edges
+// [s, e), gathered by the whole warp; ends once all of them are found.  The
+// same result in every lane.
+template <int WP>
+__device__ __forceinline__ Bits<WP> warp_gather(const MsParams &p, const uint32_t *F, uint32_t s, uint32_t e,
+                                                const Bits<WP> &need, unsigned lane)
+{
+    constexpr int kFly = WP >= 8 ? 2 : 4;  // rows a lane has in flight
+    Bits<WP> a;
+    a.clear();
+    for (uint32_t b = s; b < e; b += 32 * kFly) {
+        uint32_t u[kFly];
+#pragma unroll
+        for (int k = 0; k < kFly; k++) {
+            const uint32_t i = b + 32 * k + lane;
+            u[k] = i < e ? __ldcs(p.edge_dst + i) : 0xFFFFFFFFu;
+        }
+        Bits<WP> f[kFly];
+#pragma unroll
+        for (int k = 0; k < kFly; k++) {
+            f[k].clear();
+            if (u[k] != 0xFFFFFFFFu) f[k] = ld_row<WP>(F, u[k]);
+        }
+#pragma unroll
+        for (int w = 0; w < WP; w++) {
+            uint32_t x = 0;
+#pragma unroll
+            for (int k = 0; k < kFly; k++) x |= f[k].w[w];
+            a.w[w] |= __reduce_or_sync(kFull, x & need.w[w]);
+        }
+        if (a.covers(need)) break;  // warp uniform after the reduction
+    }
+    return a;
+}
+
+// Top-down: ORs the frontier row of u into next[v] for the edges [s, e),
+// `step` edges apart per turn of the warp.
+template <int WP>
+__device__ __forceinline__ void warp_scatter(const MsParams &p, const Bits<WP> &fu, uint32_t s, uint32_t e,
+                                             uint32_t step, uint32_t stamp, WarpQueue &tq, unsigned lane)
+{
+    for (uint32_t eb = s; eb < e; eb += step) {  // warp-uniform trip count
+        const uint32_t ei = eb + lane;
+        bool touched = false;
+        uint32_t v = 0;
+        if (ei < e) {
+            v = __ldcs(p.edge_dst + ei);
+            const Bits<WP> sv = ld_row<WP>(p.seen, v);
+#pragma unroll
+            for (int w = 0; w < WP; w++) {
+                const uint32_t b = fu.w[w] & ~sv.w[w];
+                if (b) {
+                    atomicOr(p.next + (size_t)v * WP + w, b);
+                    touched = true;
+                }
+            }
+            touched = touched && atomicExch(p.tstamp + v, stamp) != stamp;
+        }
+        tq.push(touched, v, lane);
+    }
+}
+
+// Puts v on the level's hub list.
+__device__ __forceinline__ void list_hub(const MsParams &p, unsigned long long *hub_ctr, uint32_t v, uint32_t deg)
+{
+    const unsigned nch = (deg + kHubEdges - 1) / kHubEdges;
+    const unsigned long long old = atomicAdd(hub_ctr, (1ull << 32) | nch);
+    const unsigned h = (unsigned)(old >> 32);
+    if (h < p.hub_cap) p.hubs[h] = make_uint2(v, (unsigned)old);
+    else raise_error(&p.ctl->error, &p.ctl->error_where, GFT_ERR_OVERFLOW, h);
+}
+
+// Calls f(vertex, first edge, end) for each chunk of the hub list, chunks
+// dealt to the grid's warps in turn.
+template <class F>
+__device__ __forceinline__ void for_hub_chunks(const MsParams &p, unsigned long long hv, unsigned gwarp,
+                                               unsigned nwarps, F &&f)
+{
+    const unsigned nh = (unsigned)(hv >> 32), nc = (unsigned)hv;
+    for (unsigned c = gwarp; c < nc; c += nwarps) {
+        unsigned lo = 0, hi = nh;
+        while (hi - lo > 1) {
+            const unsigned mid = (lo + hi) >> 1;
+            if (__ldcg(&p.hubs[mid].y) <= c) lo = mid;
+            else hi = mid;
+        }
+        const uint2 hb = __ldcg(p.hubs + lo);
+        const uint32_t s = __ldg(p.row_start + hb.x), e = __ldg(p.row_start + hb.x + 1);
+        const uint32_t at = s + (c - hb.y) * kHubEdges;
+        f(hb.x, at, min(e, at + kHubEdges));
+    }
 }
 
 template <int WP>
@@ -156,24 +259,28 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
         p.planes[i] = 0;
     }
     if (!gs.sync()) return;
-    if (tid == 0) {
-        for (uint32_t i = 0; i < p.k; i++) {
-            const uint32_t s = p.sources[i];
-            p.seen[(size_t)s * WP + i / 32] |= 1u << (i % 32);
-            p.planes[(size_t)s * WP + i / 32] |= 1u << (i % 32);
-        }
-        uint32_t nq0 = 0;
+    if (blockIdx.x == 0) {  // a thread per source; k <= 256
+        __shared__ uint32_t s_src[256];
+        __shared__ unsigned s_n;
+        const uint32_t i = threadIdx.x;
+        if (i < p.k) s_src[i] = p.sources[i];
+        if (i == 0) s_n = 0;
+        __syncthreads();
         unsigned long long mf = 0;
-        for (uint32_t i = 0; i < p.k; i++) {
-            const uint32_t s = p.sources[i];
+        if (i < p.k) {
+            const uint32_t s = s_src[i];
+            atomicOr(p.seen + (size_t)s * WP + i / 32, 1u << (i % 32));
+            atomicOr(p.planes + (size_t)s * WP + i / 32, 1u << (i % 32));
             bool dup = false;
-            for (uint32_t j = 0; j < i; j++) dup |= p.sources[j] == s;
-            if (dup) continue;
-            p.queue[0][nq0++] = s;
-            mf += p.row_start[s + 1] - p.row_start[s];
+            for (uint32_t j = 0; j < i; j++) dup |= s_src[j] == s;
+            if (!dup) {
+                p.queue[0][atomicAdd(&s_n, 1u)] = s;
+                mf = p.row_start[s + 1] - p.row_start[s];
+            }
         }
-        *u32_of(ctl->qlen[0]) = nq0;
-        ctl->hub[0].v = mf;
+        warp_add_u64(&ctl->hub[0].v, mf, lane);
+        __syncthreads();
+        if (i == 0) *u32_of(ctl->qlen[0]) = s_n;
     }
     if (!gs.sync()) return;
 
@@ -192,7 +299,9 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
             *u32_of(ctl->qlen[rslot]) = 0;
             *u32_of(ctl->claim[rslot]) = 0;
             ctl->hub[rslot].v = 0;
+            ctl->handoff[rslot].v = 0;
         }
+        unsigned long long *hub_ctr = &ctl->handoff[slot].v;  // (hubs << 32) | chunks of this level
         const uint32_t *F = p.planes + (size_t)L * plane_words;
         uint32_t *Fn = p.planes + (size_t)(L + 1) * plane_words;
         nq.queue = ((L + 1) & 1) ? p.queue[1] : p.queue[0];  // no dynamic index: keeps p out of local memory
@@ -218,6 +327,11 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                         e = __ldg(p.row_start + v + 1);
                     }
                 }
+                const bool hub = e - s >= kHubDegree;
+                if (hub) {  // its row is written after the hub phase
+                    list_hub(p, hub_ctr, v, e - s);
+                    e = s;
+                }
                 const bool heavy = e - s > kThreadDegree;
                 if (!heavy) {  // this thread's own vertex, kStep edges at a time
                     for (uint32_t i = s; i < e; i += kStep) {
@@ -240,26 +354,14 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                     const int j = __ffs(hm) - 1;
                     hm &= hm - 1;
                     const uint32_t sj = __shfl_sync(kFull, s, j), ej = __shfl_sync(kFull, e, j);
-                    Bits<WP> nj, a;
+                    Bits<WP> nj;
 #pragma unroll
                     for (int w = 0; w < WP; w++) nj.w[w] = __shfl_sync(kFull, need.w[w], j);
-                    a.clear();
-                    for (uint32_t b = sj; b < ej; b += 32) {
-                        if (b + lane < ej) {
-                            const Bits<WP> f = ld_row<WP>(F, __ldcs(p.edge_dst + b + lane));
-#pragma unroll
-                            for (int w = 0; w < WP; w++) a.w[w] |= f.w[w] & nj.w[w];
-                        }
-#pragma unroll
-                        for (int w = 0; w < WP; w++)
-#pragma unroll
-                            for (int o = 16; o > 0; o >>= 1) a.w[w] |= __shfl_xor_sync(kFull, a.w[w], o);
-                        if (a.covers(nj)) break;  // warp uniform after the reduction
-                    }
+                    const Bits<WP> a = warp_gather<WP>(p, F, sj, ej, nj, lane);
                     if ((int)lane == j) acc = a;
                 }
                 const bool got = acc.any();
-                if (v < n) {
+                if (v < n && !hub) {
                     st_row<WP>(Fn, v, acc);
                     if (got) {
                         Bits<WP> s2;
@@ -271,35 +373,63 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                 }
                 nq.push(got, v, lane);
             }
+            if (!gs.sync()) return;
+            const unsigned long long hv = ld_relaxed_u64(hub_ctr);
+            if (hv) {
+                for_hub_chunks(p, hv, gwarp, nwarps, [&](uint32_t v, uint32_t s, uint32_t e) {
+                    const Bits<WP> sv = ld_row<WP>(p.seen, v);
+                    Bits<WP> need;
+#pragma unroll
+                    for (int i = 0; i < WP; i++) need.w[i] = all.w[i] & ~sv.w[i];
+                    const Bits<WP> a = warp_gather<WP>(p, F, s, e, need, lane);
+#pragma unroll
+                    for (int i = 0; i < WP; i++)
+                        if (lane == i && a.w[i]) atomicOr(p.next + (size_t)v * WP + i, a.w[i]);
+                });
+                if (!gs.sync()) return;
+                const unsigned nh = (unsigned)(hv >> 32);
+                for (unsigned b = gwarp * 32; b < nh; b += nwarps * 32) {  // warp-uniform trip count
+                    bool got = false;
+                    uint32_t v = 0;
+                    if (b + lane < nh) {
+                        v = __ldcg(&p.hubs[b + lane].x);
+                        const Bits<WP> nb = ld_row<WP>(p.next, v);  // the sources it lacked
+                        got = nb.any();
+                        st_row<WP>(Fn, v, nb);
+                        if (got) {
+                            Bits<WP> z, sv = ld_row<WP>(p.seen, v);
+                            z.clear();
+                            st_row<WP>(p.next, v, z);
+#pragma unroll
+                            for (int i = 0; i < WP; i++) sv.w[i] |= nb.w[i];
+                            st_row<WP>(p.seen, v, sv);
+                            my_mf += __ldg(p.row_start + v + 1) - __ldg(p.row_start + v);
+                        }
+                    }
+                    nq.push(got, v, lane);
+                }
+            }
         } else {
             // Top-down: clear the next plane, expand, commit.
             for (size_t i = tid; i < plane_words; i += nthreads) Fn[i] = 0;
             if (!gs.sync()) return;
             const uint32_t *q = (L & 1) ? p.queue[1] : p.queue[0];
-            for (uint32_t qi = gwarp; qi < nf; qi += nwarps) {
+            // A frontier of fewer vertices than warps gives each vertex
+            // several warps.
+            const unsigned share = max(1u, nwarps / nf);
+            for (uint32_t qi = gwarp / share; qi < nf; qi += nwarps / share) {
                 const uint32_t u = __ldcg(q + qi);
-                const Bits<WP> fu = ld_row<WP>(F, u);
                 const uint32_t s = __ldg(p.row_start + u), e = __ldg(p.row_start + u + 1);
-                for (uint32_t eb = s; eb < e; eb += 32) {  // warp-uniform trip count
-                    const uint32_t ei = eb + lane;
-                    bool touched = false;
-                    uint32_t v = 0;
-                    if (ei < e) {
-                        v = __ldcs(p.edge_dst + ei);
-                        const Bits<WP> sv = ld_row<WP>(p.seen, v);
-#pragma unroll
-                        for (int w = 0; w < WP; w++) {
-                            const uint32_t b = fu.w[w] & ~sv.w[w];
-                            if (b) {
-                                atomicOr(p.next + (size_t)v * WP + w, b);
-                                touched = true;
-                            }
-                        }
-                        touched = touched && atomicExch(p.tstamp + v, L + 1) != L + 1;
-                    }
-                    tq.push(touched, v, lane);
+                if ((e - s) / kHubDegree >= share) {
+                    if (lane == 0 && gwarp % share == 0) list_hub(p, hub_ctr, u, e - s);
+                    continue;
                 }
+                warp_scatter<WP>(p, ld_row<WP>(F, u), s + gwarp % share * 32, e, 32 * share, L + 1, tq, lane);
             }
+            if (!gs.sync()) return;
+            for_hub_chunks(p, ld_relaxed_u64(hub_ctr), gwarp, nwarps, [&](uint32_t u, uint32_t s, uint32_t e) {
+                warp_scatter<WP>(p, ld_row<WP>(F, u), s, e, 32, L + 1, tq, lane);
+            });
             tq.flush(lane);
             if (!gs.sync()) return;
             const uint32_t nt = ld_relaxed_u32(u32_of(ctl->claim[slot]));
@@ -419,6 +549,8 @@ gft_status gft_msbfs(gft_engine *e, const gft_graph *g, const uint32_t *h_source
     const size_t o_seen = take(vwords * 4), o_next = take(vwords * 4), o_q0 = take((size_t)G.nnodes * 4),
                  o_q1 = take((size_t)G.nnodes * 4), o_t = take((size_t)G.nnodes * 4),
                  o_ts = take((size_t)G.nnodes * 4), o_src = take((size_t)k * 4);
+    const uint32_t hub_cap = G.nedges / dev::kHubDegree + 1;
+    const size_t o_hubs = take((size_t)hub_cap * sizeof(uint2));
     GFT_TRY(e->scratch.ensure(off));
     char *base = static_cast<char *>(e->scratch.ptr);
     const void *kern = msbfs_kernel_for(WP);
@@ -439,6 +571,8 @@ gft_status gft_msbfs(gft_engine *e, const gft_graph *g, const uint32_t *h_source
     p.queue[1] = reinterpret_cast<uint32_t *>(base + o_q1);
     p.touched = reinterpret_cast<uint32_t *>(base + o_t);
     p.tstamp = reinterpret_cast<uint32_t *>(base + o_ts);
+    p.hubs = reinterpret_cast<uint2 *>(base + o_hubs);
+    p.hub_cap = hub_cap;
     p.symmetric = (flags & GFT_MSBFS_SYMMETRIC) ? 1u : 0u;
     // Bottom-up once the frontier's edges exceed 1/64 of the graph's: a
     // bottom-up level checks a vertex's rows only until its sources are

@@ -65,3 +65,24 @@ def test_msbfs_sources_in_small_components(gft, orc, engine, k):
     r = engine.msbfs(dg, srcs, max_levels=24, symmetric=True)
     for i, s in enumerate(srcs):
         np.testing.assert_array_equal(r["levels_of"](i).cpu().numpy(), orc.bfs(rs, dst, s))
+
+
+@pytest.mark.parametrize("k", [3, 40, 100, 256])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_msbfs_hub_phase(gft, orc, engine, k, symmetric):
+    """Two hubs of more edges than one warp takes (at, just below and above a
+    multiple of the hub chunk), reached from leaves and as sources, in both
+    directions."""
+    n = 6000
+    pairs = [(0, i) for i in range(2, 2 + 3072)] + [(1, i) for i in range(2500, 2500 + 1023)]
+    pairs += [(i, i + 1) for i in range(4000, n - 1)] + [(2, 4000)]
+    a = np.array(pairs)
+    src, dst = np.concatenate([a[:, 0], a[:, 1]]), np.concatenate([a[:, 1], a[:, 0]])
+    order = np.argsort(src, kind="stable")
+    rs = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint32)
+    g = gft.CSRGraph(rs, dst[order].astype(np.uint32))
+    dg = g.copy_to_gpu()
+    srcs = [0, 1, 3000] + [int(x) for x in np.random.default_rng(k).integers(0, 4100, size=k - 3)]
+    r = engine.msbfs(dg, srcs, max_levels=2100, symmetric=symmetric)
+    for i in {0, 1, 2, k // 2, k - 1}:
+        np.testing.assert_array_equal(r["levels_of"](i).cpu().numpy(), orc.bfs(rs, g.edge_dst, srcs[i]))
