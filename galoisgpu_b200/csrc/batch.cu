@@ -5,12 +5,14 @@
 // query (skelapp/skel.cu:139-151, apps/sssp/kernel.cu:426-454).  Most queries
 // of a mixed batch are small or high-diameter and cannot keep 148 SMs busy,
 // so one launch runs them side by side in two phases:
-//   phase 1: queries on graphs of at least `group_min_nodes` vertices run on
-//            groups of `group` consecutive CTAs (GridMode over the group,
-//            control block in global memory, one per group); the launch is
-//            cooperative whenever there are such queries, so a group is
-//            co-resident and its bounded barrier cannot wait on a CTA that
-//            never starts;
+//   phase 1: large queries run on groups of consecutive CTAs (GridMode over
+//            the group, control block in global memory, one per group); the
+//            launch is cooperative whenever there are such queries, so a group
+//            is co-resident and its bounded barrier cannot wait on a CTA that
+//            never starts.  By default each query gets CTAs in proportion to
+//            its estimated work (plan_gangs); with group_blocks or
+//            group_min_nodes given, queries on graphs of at least
+//            group_min_nodes vertices run on groups of group_blocks CTAs;
 //   phase 2: the rest run on ONE CTA each (CtaMode: control block in shared
 //            memory, __syncthreads as the barrier, no grid-wide atomics).
 // Both phases take queries from a device job table, largest first (longest
@@ -33,10 +35,12 @@
 namespace gft {
 namespace dev {
 
-// jobs[0, nbig) are large queries, run in phase 1 by groups of `group`
-// CTAs (consecutive blockIdx; the launch is cooperative whenever nbig > 0,
-// so a group is co-resident); jobs[nbig, njobs) run in phase 2, one CTA
-// each.  A CTA joins phase 2 as soon as its group finds no large job left,
+// jobs[0, nbig) are large queries, run in phase 1 by groups of CTAs
+// (consecutive blockIdx; the launch is cooperative whenever nbig > 0, so a
+// group is co-resident): with `gangs` NULL groups of `group` CTAs that take
+// jobs from cursors[1], else group k runs job k alone and gangs[b] is CTA b's
+// (group, rank in it, size), group ~0 for none.  jobs[nbig, njobs) run in
+// phase 2, one CTA each.  A CTA joins phase 2 as soon as its group finds no large job left,
 // so large and small queries overlap.  cursors[0] / cursors[1] hand out
 // small / large jobs; gctl holds one zeroed control block per group.
 // Per-warp push buffers: 256 entries up to 512 threads per CTA (32 KB of
@@ -46,8 +50,9 @@ constexpr unsigned kBatchQueueBuf = BLOCK <= 512 ? 256 : kQueueBuf;
 
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
-    batch_kernel(BatchJob *jobs, unsigned njobs, unsigned nbig, unsigned group, unsigned *cursors, char *scratch,
-                 uint32_t hub_degree, TraversalCtl *gctl, unsigned long long timeout_ns)
+    batch_kernel(BatchJob *jobs, unsigned njobs, unsigned nbig, unsigned group, const uint4 *gangs,
+                 unsigned *cursors, char *scratch, uint32_t hub_degree, TraversalCtl *gctl,
+                 unsigned long long timeout_ns)
 {
     __shared__ TraversalCtl s_ctl;
     constexpr unsigned QB = kBatchQueueBuf<BLOCK>;
@@ -62,13 +67,22 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     const unsigned w = threadIdx.x >> 5;
 
     // Phase 1: large jobs on CTA groups.
-    const unsigned ngroups = (nbig > 0 && group > 1) ? gridDim.x / group : 0;
-    const unsigned g = blockIdx.x / max(group, 1u), rank = blockIdx.x % max(group, 1u);
+    const unsigned ngroups = gangs ? nbig : (nbig > 0 && group > 1) ? gridDim.x / group : 0;
+    unsigned g = blockIdx.x / max(group, 1u), rank = blockIdx.x % max(group, 1u);
+    if (gangs) {
+        const uint4 mine = gangs[blockIdx.x];
+        g = mine.x;
+        rank = mine.y;
+        group = mine.z;
+    }
     if (g < ngroups) {
         TraversalCtl *ctl = gctl + g;
+        bool first = true;
         GridSync gs{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, group, 0, timeout_ns};
         for (;;) {
-            if (rank == 0 && threadIdx.x == 0) *u32_of(ctl->job) = atomicAdd(&cursors[1], 1u);
+            if (rank == 0 && threadIdx.x == 0)
+                *u32_of(ctl->job) = !gangs ? atomicAdd(&cursors[1], 1u) : first ? g : nbig;
+            first = false;
             if (!gs.sync()) break;
             const unsigned j = ld_relaxed_u32(u32_of(ctl->job));
             if (j >= nbig) break;
@@ -157,7 +171,7 @@ static const void *batch_kernel_ptr(int block)
 }
 
 gft_status launch_batch_jobs(const BatchJob *d_jobs, unsigned njobs, unsigned nbig, unsigned group,
-                             unsigned *d_cursors, char *d_scratch, uint32_t hub_degree, TraversalCtl *d_gctl,
+                             const uint4 *d_gangs, unsigned *d_cursors, char *d_scratch, uint32_t hub_degree, TraversalCtl *d_gctl,
                              int block, int blocks, cudaStream_t stream)
 {
     const void *kern = batch_kernel_ptr(block);
@@ -169,7 +183,7 @@ gft_status launch_batch_jobs(const BatchJob *d_jobs, unsigned njobs, unsigned nb
     uint32_t hub = hub_degree;
     TraversalCtl *gc = d_gctl;
     unsigned long long timeout = 20000ull * 1000000ull;
-    void *args[] = {&dj, &nj, &nb, &grp, &cur, &scr, &hub, &gc, &timeout};
+    void *args[] = {&dj, &nj, &nb, &grp, &d_gangs, &cur, &scr, &hub, &gc, &timeout};
     GFT_CUDA_TRY(cudaMemsetAsync(d_cursors, 0, 2 * sizeof(unsigned), stream));
     cudaLaunchConfig_t lc;
     memset(&lc, 0, sizeof lc);
@@ -178,7 +192,7 @@ gft_status launch_batch_jobs(const BatchJob *d_jobs, unsigned njobs, unsigned nb
     lc.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = nbig > 0 && group > 1 ? 1 : 0;
+    attr[0].val.cooperative = nbig > 0 && (group > 1 || d_gangs) ? 1 : 0;
     lc.attrs = attr;
     lc.numAttrs = 1;
     GFT_CUDA_TRY(cudaLaunchKernelExC(&lc, kern, args));
@@ -225,6 +239,55 @@ size_t batch_job_scratch(uint32_t app, uint32_t nnodes, uint32_t hub_cap)
     return 2 * qbytes + vbytes + hbytes;
 }
 
+namespace {
+
+// Estimated edge visits of a query, to share CTAs out.  Measured ratios of
+// visits to edges: SSSP re-relaxes an R-MAT edge 3.4 times and a road edge
+// 1.3 times (and a road query's many small steps use its CTAs badly); BFS
+// visits an edge once, and a small part of them where bottom-up levels run.
+double visits(const gft_query &x)
+{
+    const DeviceGraph &G = x.graph->g;
+    const bool skewed = G.max_degree > kUniformDegree;
+    const double m = G.nedges, n = G.nnodes;
+    if (x.app == 1) return n + (skewed ? 3.5 : 2.0) * m;
+    return n + (skewed && G.symmetric ? 0.15 : skewed ? 1.0 : 1.5) * m;
+}
+
+// CTAs of each query, in proportion to its estimated visits: 1 = phase 2.
+// A query of the size that a single call runs on one CTA gets one here too,
+// and none gets more CTAs than keep 32768 visits each (a barrier of the group
+// then costs less than the CTAs bring).  Groups of a fixed size left the
+// largest queries on 8 CTAs, and R-MAT graphs below the group size on one,
+// long after the rest: a batch of 48 took 31.1 ms, with these shares 8.3 ms.
+void plan_gangs(const gft_query *q, uint32_t n, uint32_t blocks, std::vector<uint32_t> &size)
+{
+    std::vector<double> w(n);
+    double total = 0;
+    for (uint32_t i = 0; i < n; i++) total += w[i] = visits(q[i]);
+    size.assign(n, 1);
+    // The largest scale at which groups and single CTAs fit the launch.
+    for (double scale = 4.0; scale > 0.02; scale *= 0.95) {
+        double used = 0;
+        uint64_t singles = 0;
+        for (uint32_t i = 0; i < n; i++) {
+            const DeviceGraph &G = q[i].graph->g;
+            const bool small = G.nnodes <= kCtaMaxNodes && G.nedges <= kCtaMaxEdges;
+            const double share = std::min(scale * w[i] / total * blocks, w[i] / 32768.0);
+            size[i] = small || share < 2.0 ? 1u : (uint32_t)share;
+            if (size[i] > 1) used += size[i];
+            else {
+                used += std::min(1.0, scale * w[i] / total * blocks);
+                singles++;
+            }
+        }
+        if (singles) used = std::max(used, 1.0);
+        if (used + (singles ? 1 : 0) <= blocks) return;
+    }
+    size.assign(n, 1);
+}
+
+}  // namespace
 }  // namespace gft
 
 struct gft_batch {
@@ -237,6 +300,7 @@ struct gft_batch {
     int blocks = 0;
     uint32_t hub_degree = 256;
     gft::TraversalCtl *d_gctl = nullptr;
+    uint4 *d_gangs = nullptr;         // per CTA, when the groups are planned (see batch_kernel)
     size_t gctl_bytes = 0;
     std::vector<uint32_t> order;      // job slot -> caller's query index
     gft::BatchJob *h_jobs = nullptr;  // pinned, caller-owned inputs: the graph's first node uploads it
@@ -273,6 +337,7 @@ void gft_batch_destroy(gft_batch *b)
     if (b->d_cursor) cudaFree(b->d_cursor);
     if (b->d_scratch) cudaFree(b->d_scratch);
     if (b->d_gctl) cudaFree(b->d_gctl);
+    if (b->d_gangs) cudaFree(b->d_gangs);
     delete b;
 }
 
@@ -304,9 +369,24 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
             return fail(GFT_ERR_INVALID_ARG, "gft_batch_create: query %u is invalid", i);
         }
     }
+    DeviceScope device_scope(e->device);
+    GFT_CUDA_TRY_OR(device_scope.err, gft_batch_destroy(b));
+    int occ = 0;
+    GFT_CUDA_TRY_OR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, b->block, 0), gft_batch_destroy(b));
+    if (occ <= 0) {
+        gft_batch_destroy(b);
+        return fail(GFT_ERR_CUDA, "gft_batch_create: kernel cannot be resident");
+    }
+    uint32_t bps = (tune && tune->blocks_per_sm) ? tune->blocks_per_sm : (uint32_t)occ;
+    b->blocks = std::max(1, std::min<int>(occ, (int)bps)) * e->sms;
     // Large queries (run on CTA groups) first, then the rest; each class
     // largest first.
-    auto big = [&](uint32_t i) { return b->group > 1 && q[i].graph->g.nnodes >= b->group_min_nodes; };
+    const bool planned = !(tune && (tune->group_blocks || tune->group_min_nodes));
+    std::vector<uint32_t> ctas(n, 1);
+    if (planned) plan_gangs(q, n, (uint32_t)b->blocks, ctas);
+    auto big = [&](uint32_t i) {
+        return planned ? ctas[i] > 1 : b->group > 1 && q[i].graph->g.nnodes >= b->group_min_nodes;
+    };
     std::stable_sort(b->order.begin(), b->order.end(), [&](uint32_t a, uint32_t c) {
         if (big(a) != big(c)) return big(a);
         const DeviceGraph &ga = q[a].graph->g, &gc = q[c].graph->g;
@@ -314,7 +394,15 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
     });
     b->nbig = 0;
     for (uint32_t i = 0; i < n; i++) b->nbig += big(i);
-    DeviceScope device_scope(e->device);
+    std::vector<uint4> gangs;
+    if (planned && b->nbig) {
+        gangs.assign((size_t)b->blocks, make_uint4(~0u, 0, 1, 0));
+        size_t at = 0;
+        for (uint32_t k = 0; k < b->nbig; k++) {
+            const uint32_t size = ctas[b->order[k]];
+            for (uint32_t r = 0; r < size; r++) gangs[at++] = make_uint4(k, r, size, 0);
+        }
+    }
     cudaError_t err = device_scope.err;
     if (err == cudaSuccess) err = cudaMallocHost(&b->h_jobs, sizeof(BatchJob) * n);
     if (err == cudaSuccess) err = cudaMallocHost(&b->h_res, sizeof(BatchJob) * n);
@@ -330,18 +418,18 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
         off += batch_job_scratch(j.app, j.nnodes, j.hub_cap);
     }
     b->scratch_bytes = off;
-    int occ = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, b->block, 0);
-    if (err == cudaSuccess && occ <= 0) err = cudaErrorInvalidConfiguration;
-    uint32_t bps = (tune && tune->blocks_per_sm) ? tune->blocks_per_sm : (uint32_t)occ;
-    b->blocks = std::max(1, std::min<int>(occ, (int)bps)) * e->sms;
     if (b->nbig && (int)b->group > b->blocks) b->group = (uint32_t)b->blocks;
-    const uint32_t ngroups = b->nbig ? (uint32_t)b->blocks / std::max(1u, b->group) : 0;
+    const uint32_t ngroups = planned ? b->nbig : b->nbig ? (uint32_t)b->blocks / std::max(1u, b->group) : 0;
     b->gctl_bytes = std::max<size_t>(1, ngroups) * sizeof(TraversalCtl);
     if (err == cudaSuccess) err = cudaMalloc(&b->d_jobs, sizeof(BatchJob) * n);
     if (err == cudaSuccess) err = cudaMalloc(&b->d_cursor, 2 * sizeof(unsigned));
     if (err == cudaSuccess) err = cudaMalloc(&b->d_gctl, b->gctl_bytes);
     if (err == cudaSuccess) err = cudaMalloc(&b->d_scratch, std::max<size_t>(off, 256));
+    if (err == cudaSuccess && !gangs.empty()) {
+        err = cudaMalloc(&b->d_gangs, gangs.size() * sizeof(uint4));
+        if (err == cudaSuccess)
+            err = cudaMemcpy(b->d_gangs, gangs.data(), gangs.size() * sizeof(uint4), cudaMemcpyHostToDevice);
+    }
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaEventCreate(&b->ev0);
     if (err == cudaSuccess) err = cudaEventCreate(&b->ev1);
@@ -357,7 +445,7 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
     if (err == cudaSuccess) {
         cudaMemcpyAsync(b->d_jobs, b->h_jobs, sizeof(BatchJob) * n, cudaMemcpyHostToDevice, cs);
         cudaMemsetAsync(b->d_gctl, 0, b->gctl_bytes, cs);
-        gft_status ls = launch_batch_jobs(b->d_jobs, n, b->nbig, b->group, b->d_cursor, b->d_scratch, b->hub_degree,
+        gft_status ls = launch_batch_jobs(b->d_jobs, n, b->nbig, b->group, b->d_gangs, b->d_cursor, b->d_scratch, b->hub_degree,
                                           b->d_gctl, b->block, b->blocks, cs);
         cudaGraph_t gph = nullptr;
         err = cudaStreamEndCapture(cs, &gph);

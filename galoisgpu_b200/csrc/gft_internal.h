@@ -28,6 +28,18 @@ gft_status fail(gft_status s, const char *fmt, ...);
                                __LINE__);                                                              \
     } while (0)
 
+// The same, running `undo` first.
+#define GFT_CUDA_TRY_OR(call, undo)                                                                    \
+    do {                                                                                               \
+        cudaError_t e_ = (call);                                                                       \
+        if (e_ != cudaSuccess) {                                                                       \
+            undo;                                                                                      \
+            return ::gft::fail(e_ == cudaErrorMemoryAllocation ? GFT_ERR_OOM : GFT_ERR_CUDA,           \
+                               "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__,       \
+                               __LINE__);                                                              \
+        }                                                                                              \
+    } while (0)
+
 #define GFT_TRY(call)                        \
     do {                                     \
         gft_status s_ = (call);              \
@@ -205,6 +217,11 @@ gft_status check_edges_device(const DeviceGraph &G, cudaStream_t stream, uint64_
 // work per frontier vertex, so a frontier is split into one static chunk
 // per warp (no shared claim cursor); others are claimed dynamically.
 constexpr uint32_t kUniformDegree = 32;
+// Graphs up to this size run on one CTA by default: their frontiers are
+// small enough for 1024 threads, and a __syncthreads per level is several
+// times cheaper than a grid barrier (BFS on the 256^2 grid: 511 levels).
+constexpr uint32_t kCtaMaxNodes = 1u << 17;
+constexpr uint32_t kCtaMaxEdges = 1u << 19;
 gft_status check_engine_graph(gft_engine *e, const gft_graph *g);
 // Runs one BFS (is_sssp false) or SSSP query; caller holds e->mu.
 gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32_t src, int32_t delta, int32_t *d_out,
@@ -214,10 +231,11 @@ gft_status pick_sources_rs(uint32_t nnodes, const uint32_t *row_start, uint64_t 
 // CTA-mode batch kernel plumbing shared by gft_batch_* and the server.
 // jobs[0, nbig) run on groups of `group` CTAs (cooperative launch, one
 // zeroed TraversalCtl per group in d_gctl), the rest on one CTA each;
-// d_cursors holds 2 counters.
+// d_cursors holds 2 counters; d_gangs: NULL, or per CTA the group planned for
+// it (see batch_kernel).
 gft_status launch_batch_jobs(const BatchJob *d_jobs, unsigned njobs, unsigned nbig, unsigned group,
-                             unsigned *d_cursors, char *d_scratch, uint32_t hub_degree, TraversalCtl *d_gctl,
-                             int block, int blocks, cudaStream_t stream);
+                             const uint4 *d_gangs, unsigned *d_cursors, char *d_scratch, uint32_t hub_degree,
+                             TraversalCtl *d_gctl, int block, int blocks, cudaStream_t stream);
 int batch_occupancy(int block);
 void fill_batch_job(BatchJob &j, const gft_query &x, uint32_t hub_degree);
 size_t batch_job_scratch(uint32_t app, uint32_t nnodes, uint32_t hub_cap);

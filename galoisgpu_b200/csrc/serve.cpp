@@ -159,7 +159,7 @@ static void launch_lane(gft_server *s, uint32_t li, std::vector<uint64_t> &big, 
     const int blocks = nbig ? (int)G : std::min((int)s->cfg.lane_blocks, (int)small.size());
     cudaError_t e = cudaMemcpyAsync(l.d_jobs, l.h_jobs, sizeof(BatchJob) * n, cudaMemcpyHostToDevice, l.stream);
     if (e == cudaSuccess && nbig) e = cudaMemsetAsync(l.d_gctl, 0, sizeof(TraversalCtl), l.stream);
-    gft_status st = e == cudaSuccess ? launch_batch_jobs(l.d_jobs, n, nbig, G, l.d_cursor, l.d_arena,
+    gft_status st = e == cudaSuccess ? launch_batch_jobs(l.d_jobs, n, nbig, G, nullptr, l.d_cursor, l.d_arena,
                                                          s->cfg.hub_degree, l.d_gctl, (int)s->cfg.block_threads,
                                                          blocks, l.stream)
                                      : GFT_ERR_CUDA;

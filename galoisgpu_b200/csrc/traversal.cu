@@ -445,11 +445,6 @@ constexpr uint32_t kDefaultCtaSmall = 256;
 // RMAT-22), where a warp's chased vertices are hubs' neighbourhoods and
 // unbalance the grid.
 constexpr uint32_t kDefaultFuse = 256;
-// Graphs up to this size run on one CTA by default: their frontiers are
-// small enough for 1024 threads, and a __syncthreads per level is several
-// times cheaper than a grid barrier (BFS on the 256^2 grid: 511 levels).
-constexpr uint32_t kCtaMaxNodes = 1u << 17;
-constexpr uint32_t kCtaMaxEdges = 1u << 19;
 
 template <int BLOCK>
 const void *bfs_kernel_tile(uint32_t tile)

@@ -95,10 +95,14 @@ typedef struct gft_tuning {
                                  and out-degrees <= 32 gives each thread a
                                  frontier vertex and always runs top-down
                                  (levels are the same either way) */
-    uint32_t group_blocks;    /* batches: CTAs that share one large query (0 = 8)   */
+    uint32_t group_blocks;    /* batches: CTAs that share one large query; 0 (and
+                                 group_min_nodes 0) = each query gets CTAs in
+                                 proportion to its estimated work             */
     uint32_t group_min_nodes; /* batches: queries on graphs with at least this many
-                                 vertices run on a CTA group (0 = 262144; set it
-                                 above every graph to run each query on one CTA) */
+                                 vertices run on a CTA group (set it above every
+                                 graph to run each query on one CTA).  When only
+                                 one of the two is given, the other is 8 CTAs or
+                                 262144 vertices                              */
     uint32_t direction;       /* BFS: 0 = direction-optimising when the graph is
                                  marked symmetric, 1 = top-down only          */
     uint32_t cta_small;       /* SSSP on the grid: iterations of at most this

@@ -83,3 +83,27 @@ def test_batch_rejects_bad_queries(gft, engine):
         gft.Batch(engine, [{"graph": d, "app": "sssp", "src": 0, "delta": 0}])
     with pytest.raises(gft.GftError):
         gft.Batch(engine, [{"graph": d, "app": "bfs", "src": 0}], tune=gft.Tune(block_threads=100))
+
+
+def test_batch_shares_ctas_by_work(gft, orc, engine):
+    """Graphs above the one-CTA size, of very different work, beside small
+    ones: planned groups of several sizes and single CTAs in one launch."""
+    hosts = [gft.CSRGraph.road(400, seed=41), gft.CSRGraph.rmat(16, 16, seed=42, max_weight=255),
+             gft.CSRGraph.rmat(14, 32, seed=43, max_weight=255), gft.CSRGraph.road(60, seed=44)]
+    devs = [h.copy_to_gpu() for h in hosts]
+    queries, want = [], []
+    for k in range(8):
+        h, d = hosts[k % 4], devs[k % 4]
+        src = h.pick_sources(50 + k, 1)[0]
+        queries.append({"graph": d, "app": "bfs" if k >= 4 else "sssp", "src": src, "delta": 20000})
+        want.append(orc.bfs(h.row_start, h.edge_dst, src) if k >= 4
+                    else orc.sssp(h.row_start, h.edge_dst, h.edge_data, src))
+    b = gft.Batch(engine, queries)
+    for rep in range(2):
+        for q in b.queries:
+            q["out"].fill_(-7)
+        b.run()
+        for q, w in zip(b.queries, want):
+            assert q["status"] == 0
+            np.testing.assert_array_equal(q["out"].cpu().numpy(), w)
+    b.close()
