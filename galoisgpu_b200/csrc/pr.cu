@@ -326,14 +326,14 @@ gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t
     // Quads of the renumbered rows: at most deg / 4 + 3/4 per row with edges,
     // padded by at most 1/8.
     const uint64_t quads = (m / 4 + std::min(n, m)) * 9 / 8 + 64;
-    if (quads >> 32) return GFT_OK;
+    if (quads >> 32 || n >> 29) return GFT_OK;  // 32-bit quad numbers and byte offsets of values
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
         off += (bytes + 255) & ~(size_t)255;
         return o;
     };
-    const size_t vec = (n + 8) * 4;
+    const size_t vec = (n + 8) * 4;  // y holds a zero beside the n values
     const size_t o_st = take(sizeof(dev::PullState)), o_perm = take(vec), o_num = take(vec), o_inv = take(vec),
                  o_x0 = take(vec), o_x1 = take(vec), o_y0 = take(vec), o_y1 = take(vec), o_quads = take(quads * 16);
     if (e->scratch.ensure(off) != GFT_OK) {
@@ -361,7 +361,7 @@ gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t
     // A small graph's sweep is a few microseconds: CTAs without work only
     // lengthen its barrier.
     const int blocks = (int)std::min<uint64_t>(e->sms, (n + m / 4) / 2048 + 1);
-    const size_t hub_bytes = dev::kPullHub * sizeof(float);
+    const size_t hub_bytes = (dev::kPullHub + 4) * sizeof(float);
     const void *kern = (const void *)dev::pr_sweeps;
     GFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hub_bytes));
     GFT_CUDA_TRY(cudaMemsetAsync(e->ctl.ptr, 0, sizeof(TraversalCtl), stream));

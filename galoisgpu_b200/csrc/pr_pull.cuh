@@ -18,13 +18,15 @@
 // residuals: no atomics, and a sum's order does not depend on the schedule.
 //
 // What bounds a sweep is the gather of y = D^-1 x, one 4-byte value per edge.
-// L1 looks up one line a cycle for lanes on different lines, and an L2 gather
-// moves a 32-byte sector per value, so vertices are renumbered by degree,
+// L1 looks up one line a cycle for lanes on different lines, an L2 gather
+// moves a 32-byte sector per value, and every edge costs the instructions of
+// its gather, so vertices are renumbered by degree,
 // largest first: the first kPullHub values of y, which on a skewed graph
 // stand behind most edges, are copied into shared memory at the start of
 // each sweep, where 32 lanes on different banks are served together.  The
-// renumbered rows are stored in 16-byte quads of edges, padded with the index
-// of a zero.  Rows of one class (8 classes per octave of quads) are padded
+// renumbered rows are stored in 16-byte quads of edges; an edge is the byte
+// offset of its value, and rows are padded with the offset of a zero that lies
+// between the values in shared memory and the rest.  Rows of one class (8 classes per octave of quads) are padded
 // to the class's largest, so a row's place follows from its number and the
 // lanes of a warp run the same trip count; the padding is at most 1/8.
 //
@@ -72,9 +74,10 @@ struct PullParams {
     uint32_t nnodes, nedges;
     float *rank;         // the caller's output
     uint32_t *perm;      // number -> vertex
-    uint32_t *number;    // vertex -> number (nnodes: no edges, the index of a zero in y)
+    uint32_t *number;    // vertex -> number (vertices without edges: not set)
     float *inv_deg;      // by number
-    float *x[2], *y[2];  // by number; y[nnodes] = 0
+    float *x[2];         // by number
+    float *y[2];         // by place (pull_place)
     uint4 *quads;
     PullState *st;
     TraversalCtl *ctl;
@@ -102,6 +105,11 @@ __host__ __device__ __forceinline__ uint32_t pull_class_quads(unsigned c)
 
 __device__ __forceinline__ uint32_t pull_quads_of(uint32_t deg) { return deg / 4u + (deg % 4u != 0u); }
 
+// Numbers below this one have their y in shared memory.
+__device__ __forceinline__ unsigned pull_hubs(unsigned active) { return min(active, kPullHub); }
+// Place of a numbered vertex's value in y: place nhub is the padding's zero.
+__device__ __forceinline__ uint32_t pull_place(uint32_t i, unsigned nhub) { return i + (i >= nhub); }
+
 // 64-bit mix of an unordered pair (SplitMix64's finaliser, Steele, Lea and
 // Flood, OOPSLA 2014, over the packed pair).
 __device__ __forceinline__ unsigned long long pull_pair_hash(uint32_t a, uint32_t b)
@@ -114,7 +122,7 @@ __device__ __forceinline__ unsigned long long pull_pair_hash(uint32_t a, uint32_
 
 // A warp per sampled edge u->v looks for u among v's edges (lists of more
 // than kPullSampleScan edges are taken on trust: pr_relabel's hash decides).
-constexpr unsigned kPullSamples = 256, kPullSampleScan = 4096;
+constexpr unsigned kPullSamples = 256, kPullSampleScan = 1024;
 
 __global__ void __launch_bounds__(256) pr_sample(PullParams p)
 {
@@ -218,7 +226,7 @@ __global__ void __launch_bounds__(1024) pr_place(PullParams p)
             const uint32_t v = tile * kPullTile + k * 1024 + threadIdx.x;
             if (v >= p.nnodes) continue;
             if (cls[k] == 0) {
-                p.number[v] = p.nnodes;
+                p.number[v] = 0;  // no row names it, or the graph is not symmetric
                 p.rank[v] = (float)(1.0 - kPullAlpha);
             } else {
                 const uint32_t i = s_base[cls[k]] + at[k];
@@ -272,23 +280,31 @@ __device__ __forceinline__ void pull_table(const PullState *st, PullTable &t)
     __syncthreads();
 }
 
-// Lanes that share a row of q quads: one quad per lane up to 8, eight lanes
-// up to 31 quads, a warp above.
-__device__ __forceinline__ unsigned pull_lanes(uint32_t q) { return q == 1 ? 1u : q == 2 ? 2u : q <= 4 ? 4u : q < 32 ? 8u : 32u; }
+// Lanes that share a row of q quads: a quad per lane up to 4, then two to four
+// quads per lane, so that few of them are padding.
+__device__ __forceinline__ unsigned pull_lanes(uint32_t q)
+{
+    return q <= 2 ? q : q <= 16 ? 4u : q <= 32 ? 8u : q <= 64 ? 16u : 32u;
+}
 
-// Calls f(row of the class) for the rows of every class, `lanes` lanes per
-// row, dealt to the grid's warps in turn: rows are sorted by size, so every
-// warp gets about the same number of edges.
+// Calls f(class, row, first quad, end, lane of the row, lanes per row) for the
+// rows of every class, a long row in segments of kPullSegment quads, dealt to
+// the grid's warps in turn: rows are sorted by size, so every warp gets about
+// the same number of edges.
+constexpr uint32_t kPullSegment = 512;
+
 template <class F>
-__device__ __forceinline__ void pull_relabel_rows(const PullTable &t, unsigned gwarp, unsigned nwarps, unsigned lane,
-                                                  F &&f)
+__device__ __forceinline__ void pull_segments(const PullTable &t, unsigned gwarp, unsigned nwarps, unsigned lane, F &&f)
 {
     unsigned dealt = 0;
     for (unsigned c = 0; c < t.n; c++) {
-        const unsigned s = pull_lanes(t.quads[c]), per = 32 / s, chunks = (t.rows[c] + per - 1) / per;
+        const uint32_t q = t.quads[c], segs = (q + kPullSegment - 1) / kPullSegment;
+        const unsigned s = pull_lanes(q), per = 32 / s;
+        const unsigned chunks = segs > 1 ? t.rows[c] * segs : (t.rows[c] + per - 1) / per;
         for (unsigned k = (gwarp + nwarps - dealt) % nwarps; k < chunks; k += nwarps) {
-            const unsigned r = k * per + lane / s;
-            if (r < t.rows[c]) f(c, r, lane % s, s);
+            const unsigned r = segs > 1 ? k / segs : k * per + lane / s;
+            const uint32_t j = segs > 1 ? k % segs * kPullSegment : 0;
+            if (r < t.rows[c]) f(c, r, j, min(q, j + kPullSegment), lane % s, s);
         }
         dealt = (dealt + chunks) % nwarps;
     }
@@ -301,21 +317,23 @@ __global__ void __launch_bounds__(512, 3) pr_relabel(PullParams p)
     pull_table(p.st, s_t);
     const unsigned lane = threadIdx.x & 31;
     const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    const unsigned nhub = pull_hubs(s_t.active);
     unsigned long long hash = 0;
     bool outside = false;
-    pull_relabel_rows(s_t, gwarp, nwarps, lane, [&](unsigned c, unsigned r, unsigned l, unsigned s) {
+    pull_segments(s_t, gwarp, nwarps, lane, [&](unsigned c, unsigned r, uint32_t j0, uint32_t j1, unsigned l,
+                                                unsigned s) {
         const uint32_t q = s_t.quads[c];
         const uint32_t u = __ldg(p.perm + s_t.first[c] + r);
         const uint32_t start = __ldg(p.row_start + u), deg = __ldg(p.row_start + u + 1) - start;
         uint4 *out = p.quads + s_t.quad0[c] + (size_t)r * q;
-        for (uint32_t j = l; j < q; j += s) {
+        for (uint32_t j = j0 + l; j < j1; j += s) {
             uint32_t d[4], e[4];
 #pragma unroll
             for (int k = 0; k < 4; k++) d[k] = 4 * j + k < deg ? __ldcs(p.edge_dst + start + 4 * j + k) : 0xFFFFFFFFu;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const bool in = d[k] < p.nnodes;
-                e[k] = in ? __ldg(p.number + d[k]) : p.nnodes;
+                e[k] = 4u * (in ? pull_place(__ldg(p.number + d[k]), nhub) : nhub);
                 if (4 * j + k < deg) {
                     outside |= !in;
                     if (d[k] != u) hash += u < d[k] ? pull_pair_hash(u, d[k]) : 0ull - pull_pair_hash(u, d[k]);
@@ -332,76 +350,133 @@ __global__ void __launch_bounds__(512, 3) pr_relabel(PullParams p)
 // Sweeps
 // ---------------------------------------------------------------------------
 struct PullSweep {
-    const uint4 *quads;
-    const float *hub;  // shared memory: y[0, nhub)
-    unsigned nhub;
-    const float *y;    // this sweep's values
+    const char *hub;   // shared memory: y[0, nhub], the last one 0
+    unsigned hub_end;  // byte offset of that zero
+    const char *y;     // this sweep's values
     float *yn, *xo;    // next values; x(k-1), replaced by x(k+1)
     const float *xc, *inv_deg;
+    unsigned nhub;
     float omega;
     bool moved;
 
-    // y changes between sweeps (the grid barrier's acquire drops the SM's L1
-    // lines), never within one.
-    __device__ __forceinline__ float at(uint32_t i) const { return i < nhub ? hub[i] : __ldca(y + i); }
+    // One of the two terms is the value and the other 0: no branch, so all
+    // of a lane's gathers are in flight together.  y changes between sweeps
+    // (the grid barrier's acquire drops the SM's L1 lines), never within one.
+    __device__ __forceinline__ float at(uint32_t off) const
+    {
+        float g = 0.f;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.u32 p, %1, %2;\n\t@p ld.global.ca.f32 %0, [%3];\n\t}"
+                     : "+f"(g)
+                     : "r"(off), "r"(hub_end), "l"(y + off));
+        return *reinterpret_cast<const float *>(hub + min(off, hub_end)) + g;
+    }
     __device__ __forceinline__ float sum(const uint4 &e) const
     {
         const float a = at(e.x), b = at(e.y), c = at(e.z), d = at(e.w);
         return (a + b) + (c + d);
     }
-    __device__ __forceinline__ void finish(uint32_t i, double s, float old, float cur, float inv)
+    __device__ __forceinline__ void finish(uint32_t i, float s, float old, float cur, float inv)
     {
-        const float xn = (float)(old + omega * ((1.0 - kPullAlpha) + kPullAlpha * s - old));
+        const float xn = old + omega * ((float)(1.0 - kPullAlpha) + (float)kPullAlpha * s - old);
         xo[i] = xn;
-        yn[i] = xn * inv;
+        yn[pull_place(i, nhub)] = xn * inv;
         moved |= fabsf(xn - cur) > kPullEpsilon * fmaxf(1.f, xn);
     }
 };
 
-// Rows of one class, S lanes per row, U rows per group of lanes and V quads
-// per lane at once: their loads, then their gathers, are in flight together.
-template <int S, int U, int V>
+// Rows of one class of q <= 4 * S quads: S lanes per row, U rows per group of
+// lanes at once, up to four quads per lane.  A lane's sum has at most 16
+// terms and a row's 256: 32-bit sums in a tree.
+template <int S, int U>
 __device__ __forceinline__ void pull_rows(PullSweep &sw, unsigned first, unsigned rows, uint32_t q, const uint4 *quads,
-                                          uint32_t zero, unsigned k0, unsigned nwarps, unsigned lane)
+                                          unsigned k0, unsigned nwarps, unsigned lane)
 {
     constexpr unsigned per = 32 / S;
     const unsigned chunks = (rows + per - 1) / per, l = lane % S;
+    const uint4 pad = make_uint4(sw.hub_end, sw.hub_end, sw.hub_end, sw.hub_end);
     for (unsigned k = k0; k < chunks; k += nwarps * U) {
         unsigned r[U];
-        double acc[U];
-        float old[U], cur[U], inv[U];
+        uint4 e[U];
+        float acc[U], old[U], cur[U], inv[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             r[u] = (k + u * nwarps) * per + lane / S;
-            acc[u] = 0;
+            const bool has = k + u * nwarps < chunks && r[u] < rows;
+            if (!has) r[u] = rows;
+            e[u] = has && l < q ? __ldcs(quads + (size_t)r[u] * q + l) : pad;
             old[u] = cur[u] = inv[u] = 0.f;
-            if (k + u * nwarps >= chunks || r[u] >= rows) r[u] = 0xFFFFFFFFu;
-            if (l == 0 && r[u] != 0xFFFFFFFFu) {
+            if (l == 0 && has) {
                 old[u] = __ldcg(sw.xo + first + r[u]);
                 cur[u] = __ldcg(sw.xc + first + r[u]);
                 inv[u] = __ldcs(sw.inv_deg + first + r[u]);
             }
         }
-        for (uint32_t j = l; j < q; j += S * V) {
-            uint4 e[U * V];
+        if (S < 4) {  // a quad per lane
 #pragma unroll
-            for (int u = 0; u < U; u++)
+            for (int u = 0; u < U; u++) acc[u] = sw.sum(e[u]);
+        } else {
+            uint4 e1[U], e2[U], e3[U];
+            const bool two = q > S, three = q > 2 * S, four = q > 3 * S;  // the same for the class
 #pragma unroll
-                for (int v = 0; v < V; v++)
-                    e[u * V + v] = r[u] != 0xFFFFFFFFu && j + v * S < q
-                                       ? __ldcs(quads + (size_t)r[u] * q + j + v * S)
-                                       : make_uint4(zero, zero, zero, zero);
+            for (int u = 0; u < U; u++) {
+                const uint4 *row = quads + (size_t)r[u] * q;
+                const bool has = r[u] < rows;
+                e1[u] = two && has && l + S < q ? __ldcs(row + l + S) : pad;
+                e2[u] = three && has && l + 2 * S < q ? __ldcs(row + l + 2 * S) : pad;
+                e3[u] = four && has && l + 3 * S < q ? __ldcs(row + l + 3 * S) : pad;
+            }
 #pragma unroll
-            for (int u = 0; u < U; u++)
+            for (int u = 0; u < U; u++) acc[u] = sw.sum(e[u]);
+            if (two) {
 #pragma unroll
-                for (int v = 0; v < V; v++) acc[u] += sw.sum(e[u * V + v]);
+                for (int u = 0; u < U; u++) acc[u] += sw.sum(e1[u]);
+            }
+            if (three) {
+#pragma unroll
+                for (int u = 0; u < U; u++) acc[u] += sw.sum(e2[u]);
+            }
+            if (four) {
+#pragma unroll
+                for (int u = 0; u < U; u++) acc[u] += sw.sum(e3[u]);
+            }
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
 #pragma unroll
             for (int o = S / 2; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(kFull, acc[u], o);
-            if (l == 0 && r[u] != 0xFFFFFFFFu) sw.finish(first + r[u], acc[u], old[u], cur[u], inv[u]);
+            if (l == 0 && r[u] < rows) sw.finish(first + r[u], acc[u], old[u], cur[u], inv[u]);
         }
+    }
+}
+
+// Rows of more quads, a warp per row, four quads per lane at once (fewer in
+// the last turn); the turns' sums are added in 64 bits.
+__device__ __forceinline__ void pull_long_rows(PullSweep &sw, unsigned first, unsigned rows, uint32_t q,
+                                               const uint4 *quads, unsigned k0, unsigned nwarps, unsigned lane)
+{
+    const uint4 pad = make_uint4(sw.hub_end, sw.hub_end, sw.hub_end, sw.hub_end);
+    for (unsigned r = k0; r < rows; r += nwarps) {
+        const uint4 *row = quads + (size_t)r * q;
+        float old = 0.f, cur = 0.f, inv = 0.f;
+        if (lane == 0) {
+            old = __ldcg(sw.xo + first + r);
+            cur = __ldcg(sw.xc + first + r);
+            inv = __ldcs(sw.inv_deg + first + r);
+        }
+        double acc = 0;
+        for (uint32_t j = 0; j < q; j += 128) {
+            uint4 e[4];
+#pragma unroll
+            for (int v = 0; v < 4; v++) e[v] = j + 32 * v + lane < q ? __ldcs(row + j + 32 * v + lane) : pad;
+            float s = sw.sum(e[0]);
+#pragma unroll
+            for (int v = 1; v < 4; v++)
+                if (j + 32 * v < q) s += sw.sum(e[v]);
+            acc += s;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+        if (lane == 0) sw.finish(first + r, (float)acc, old, cur, inv);
     }
 }
 
@@ -422,8 +497,8 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
         return;
     }
     pull_table(p.st, s_t);
-    const uint32_t n = s_t.active, zero = p.nnodes;
-    const unsigned nhub = min(n, kPullHub);
+    const uint32_t n = s_t.active;
+    const unsigned nhub = pull_hubs(n), zero = 4 * nhub;
     unsigned long long quads_total = 0;
     if (s_t.n) quads_total = (unsigned long long)s_t.quad0[s_t.n - 1] + (unsigned long long)s_t.rows[s_t.n - 1] * s_t.quads[s_t.n - 1];
     // A row of more than a quarter of a warp's share of the quads (at least
@@ -439,21 +514,29 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
         const float x = (float)(1.0 - kPullAlpha) + per_edge / inv;
         p.x[0][i] = x;
         p.x[1][i] = x;
-        p.y[0][i] = x * inv;
+        p.y[0][pull_place(i, nhub)] = x * inv;
     }
-    if (tid == 0) p.y[0][zero] = p.y[1][zero] = 0.f;
+    if (threadIdx.x == 0) s_hub[nhub] = 0.f;  // the copies below end before it
     if (!gs.sync()) return;
 
     unsigned k = 0;
     double omega = 1.0;
     while (n && k < kPullMaxSweeps) {
         const unsigned cur = k & 1;
-        PullSweep sw{p.quads, s_hub, nhub, cur ? p.y[1] : p.y[0], cur ? p.y[0] : p.y[1], cur ? p.x[0] : p.x[1],
-                     cur ? p.x[1] : p.x[0], p.inv_deg, (float)omega, false};
+        const float *y = cur ? p.y[1] : p.y[0];
+        PullSweep sw{reinterpret_cast<const char *>(s_hub), zero, reinterpret_cast<const char *>(y),
+                     cur ? p.y[0] : p.y[1], cur ? p.x[0] : p.x[1], cur ? p.x[1] : p.x[0], p.inv_deg, nhub,
+                     (float)omega, false};
         if (tid == 0) p.st->moved[(k + 1) % 3] = 0;
-        for (unsigned i = threadIdx.x * 4; i < nhub; i += kPullBlock * 4) {  // y and s_hub hold a multiple of 4
-            const float4 v = __ldcg(reinterpret_cast<const float4 *>(sw.y + i));
-            *reinterpret_cast<float4 *>(s_hub + i) = v;
+        for (unsigned i = threadIdx.x * 4; i < nhub; i += kPullBlock * 4) {
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(y + i));  // y holds a multiple of 4
+            if (i + 4 <= nhub) {
+                *reinterpret_cast<float4 *>(s_hub + i) = v;
+            } else {
+                s_hub[i] = v.x;
+                if (i + 1 < nhub) s_hub[i + 1] = v.y;
+                if (i + 2 < nhub) s_hub[i + 2] = v.z;
+            }
         }
         __syncthreads();
         unsigned c = 0, dealt = 0, buf = 0;
@@ -465,8 +548,7 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
                 for (uint32_t j = threadIdx.x; j < q; j += 2 * kPullBlock) {
                     const uint4 a = __ldcs(e + j);
                     const uint4 b = j + kPullBlock < q ? __ldcs(e + j + kPullBlock) : make_uint4(zero, zero, zero, zero);
-                    acc += sw.sum(a);
-                    acc += sw.sum(b);
+                    acc += sw.sum(a) + sw.sum(b);
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
@@ -477,7 +559,7 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
                     const uint32_t i = s_t.first[c] + r;
-                    if (lane == 0) sw.finish(i, s, __ldcg(sw.xo + i), __ldcg(sw.xc + i), __ldcg(sw.inv_deg + i));
+                    if (lane == 0) sw.finish(i, (float)s, __ldcg(sw.xo + i), __ldcg(sw.xc + i), __ldcg(sw.inv_deg + i));
                 }
                 buf ^= 1;  // the other buffer's readers passed this row's barrier
             }
@@ -489,11 +571,12 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
             const uint4 *e = p.quads + s_t.quad0[c];
             const unsigned s = pull_lanes(q), per = 32 / s, chunks = (rows + per - 1) / per;
             const unsigned k0 = (gwarp + nwarps - dealt) % nwarps;
-            if (s == 32) pull_rows<32, 1, 4>(sw, first, rows, q, e, zero, k0, nwarps, lane);
-            else if (s == 8) pull_rows<8, 2, 2>(sw, first, rows, q, e, zero, k0, nwarps, lane);
-            else if (s == 4) pull_rows<4, 4, 1>(sw, first, rows, q, e, zero, k0, nwarps, lane);
-            else if (s == 2) pull_rows<2, 4, 1>(sw, first, rows, q, e, zero, k0, nwarps, lane);
-            else pull_rows<1, 4, 1>(sw, first, rows, q, e, zero, k0, nwarps, lane);
+            if (q > 64) pull_long_rows(sw, first, rows, q, e, k0, nwarps, lane);
+            else if (s == 16) pull_rows<16, 1>(sw, first, rows, q, e, k0, nwarps, lane);
+            else if (s == 8) pull_rows<8, 1>(sw, first, rows, q, e, k0, nwarps, lane);
+            else if (s == 4) pull_rows<4, 2>(sw, first, rows, q, e, k0, nwarps, lane);
+            else if (s == 2) pull_rows<2, 4>(sw, first, rows, q, e, k0, nwarps, lane);
+            else pull_rows<1, 4>(sw, first, rows, q, e, k0, nwarps, lane);
             dealt = (dealt + chunks) % nwarps;
         }
         if (__any_sync(kFull, sw.moved) && lane == 0) *(volatile unsigned *)&p.st->moved[k % 3] = 1;
