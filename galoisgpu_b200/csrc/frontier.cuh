@@ -985,7 +985,10 @@ __device__ __forceinline__ void sssp_body(const TravParams &p, Mode &m, uint32_t
         if (kSolo && Mode::kGrid && p.cta_small && sssp_small(p, m, st, n_near)) {
             // Small iterations: the first CTA runs them alone, with
             // __syncthreads as the barrier, while the other CTAs wait at the
-            // grid barrier below; it hands the loop state over there.
+            // grid barrier below; it hands the loop state over there.  It
+            // starts once every thread has read the pile's length, which
+            // it is about to overwrite.
+            if (!m.sync()) return;
             if (blockIdx.x == 0) {
                 CtaMode cm{ctl, threadIdx.x, blockDim.x, threadIdx.x >> 5, blockDim.x >> 5, 0};
                 unsigned nn = n_near;
