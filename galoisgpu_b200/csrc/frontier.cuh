@@ -13,7 +13,11 @@
 namespace gft {
 namespace dev {
 
-constexpr uint32_t kHubChunk = 2048;  // edges of a hub handled per warp claim
+// Edges of a hub handled per warp claim.  The last chunks of a hub phase are
+// what the grid waits for, and a frontier of a few hubs has fewer chunks than
+// warps: 512 instead of 2048 took RMAT-24 BFS from 746 to 653 us, RMAT-21
+// top-down BFS from 675 to 627 us and RMAT-20 SSSP from 1785 to 1501 us.
+constexpr uint32_t kHubChunk = 512;
 constexpr unsigned kInf = 0x7FFFFFFFu;
 
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) { return __ldcs(p); }
@@ -103,6 +107,19 @@ __device__ __forceinline__ uint32_t ld_bits(const uint32_t *p)
         return __ldcg(p);
 }
 
+// First look at a vertex's bit: through L1 in global memory.  Bits are only
+// ever set during a traversal, so a set bit is final however old the line is,
+// and most edges of a large level lead to visited vertices; a clear one is
+// looked up again in L2 before the claim (RMAT-21 top-down: 630 -> 591 us).
+template <bool kLocalBits>
+__device__ __forceinline__ uint32_t probe_bits(const uint32_t *p)
+{
+    if constexpr (kLocalBits)
+        return *(const volatile uint32_t *)p;
+    else
+        return __ldca(p);
+}
+
 template <bool kLocalBits = false, unsigned kQB = kQueueBuf>
 struct BfsVisitorT {
     static constexpr int kBatch = GFT_BFS_BATCH;  // edges per lane in one flattened step
@@ -136,7 +153,12 @@ struct BfsVisitorT {
     {
         uint32_t word[K];
 #pragma unroll
-        for (int k = 0; k < K; k++) word[k] = valid[k] ? ld_bits<kLocalBits>(visited + (dst[k] >> 5)) : 0xFFFFFFFFu;
+        for (int k = 0; k < K; k++) word[k] = valid[k] ? probe_bits<kLocalBits>(visited + (dst[k] >> 5)) : 0xFFFFFFFFu;
+        if constexpr (!kLocalBits) {
+#pragma unroll
+            for (int k = 0; k < K; k++)
+                if (!(word[k] & (1u << (dst[k] & 31)))) word[k] = __ldcg(visited + (dst[k] >> 5));
+        }
         bool mine[K];
 #pragma unroll
         for (int k = 0; k < K; k++) {
@@ -498,9 +520,13 @@ __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsig
 // frontier is cut into one chunk per warp, so no warp claims work through
 // the shared cursor, whose atomics serialise in one L2 slice; on skewed
 // graphs (R-MAT) about four chunks per warp are claimed dynamically, which
-// keeps the warps balanced.
-__device__ __forceinline__ unsigned pick_grain(unsigned n, unsigned nwarps, bool uniform)
+// keeps the warps balanced.  `fine` (SSSP) claims dynamically from a quarter
+// of a 32-vertex chunk per warp on, for frontiers whose vertices cost very
+// different times: RMAT-20 SSSP 1.19x -> 1.23x beside the smaller hub chunks,
+// while the BFS cases lose 2-3% to the claims.
+__device__ __forceinline__ unsigned pick_grain(unsigned n, unsigned nwarps, bool uniform, bool fine = false)
 {
+    if (fine && !uniform && n < nwarps * 128u) return max(1u, n / (nwarps * 4u));
     if (n < nwarps * 32u) return max(1u, (n + nwarps - 1) / nwarps);
     if (uniform) return 32u * ((n + nwarps * 32u - 1) / (nwarps * 32u));
     unsigned per = n / (nwarps * 32u * 4u);
@@ -837,8 +863,8 @@ __device__ __forceinline__ int sssp_iter(const TravParams &p, Mode &m, Vis &vis,
         vis.fq.queue = sel2(p.far, P);
         vis.fq.len = u32_of(ctl->far_len[P % 3]);
         expand_frontier<Vis, SsspOwn>(vis, p, sel2(p.q, I), n_near, u32_of(ctl->claim[slot]),
-                                              &ctl->hub[slot].v, pick_grain(n_near, nwarps, p.uniform), gwarp, nwarps,
-                                              lane);
+                                              &ctl->hub[slot].v, pick_grain(n_near, nwarps, p.uniform, true), gwarp,
+                                              nwarps, lane);
         if constexpr (Vis::kFuse) {
             // Bucket fusion: expand up to p.fuse of this warp's fresh near
             // vertices now, newest first, instead of in the next iteration.
