@@ -60,7 +60,7 @@ struct DeviceGraph {
     // SSSP query and owned by the graph even when the arrays above are
     // wrapped; NULL until then.
     uint2 *edge_dw = nullptr;
-    // Small low-degree graphs (the one-CTA thread-per-vertex BFS): one
+    // Low-degree graphs (the thread-per-vertex BFS kernels): one
     // 16-byte slot per vertex with its up to 4 destinations (kBfsSlotNone
     // after them), or kBfsSlotWide first for a vertex of more edges or of
     // a destination outside the graph (read through the CSR).  Built

@@ -154,7 +154,7 @@ constexpr size_t kLaneSmemBytes = (kCtaLocalBitsNodes / 32 + 2 * (size_t)kLaneQu
 // One warp step's appends: claimed destinations v[k] (mine[k]) of frontier
 // vertex u go to the next frontier and get their level.  Each vertex is
 // claimed once, so a level appends fewer than qcap = nnodes entries.
-template <bool kParent>
+template <bool kParent, uint32_t kHead = kLaneQueueHead>
 __device__ __forceinline__ void lanes_append(const TravParams &p, const bool (&mine)[4], const uint32_t (&v)[4],
                                              uint32_t u, unsigned *len_next, uint32_t *out_head,
                                              uint32_t *out_tail, int32_t level, unsigned *err, unsigned lane,
@@ -174,7 +174,7 @@ __device__ __forceinline__ void lanes_append(const TravParams &p, const bool (&m
     }
     at = __shfl_sync(kFull, at, 0);
     const unsigned lt = lanemask_lt();
-    if (at + total <= kLaneQueueHead) {  // warp uniform
+    if (at + total <= kHead) {  // warp uniform
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             if (mine[k]) {
@@ -190,7 +190,7 @@ __device__ __forceinline__ void lanes_append(const TravParams &p, const bool (&m
     for (int k = 0; k < 4; k++) {
         if (mine[k]) {
             const unsigned slot = at + __popc(mask[k] & lt);
-            if (slot < kLaneQueueHead)
+            if (slot < kHead)
                 out_head[slot] = v[k];
             else if (slot < p.qcap)
                 out_tail[slot] = v[k];
@@ -352,11 +352,213 @@ __host__ inline const void *lanes_kernel_for(int block, bool parent)
 {
     return parent ? lanes_kernel_for<true>(block) : lanes_kernel_for<false>(block);
 }
-__host__ inline bool is_lanes_kernel(const void *k)
+template <bool kParent>
+__global__ void bfs_slots_grid(TravParams p);
+__host__ inline bool reads_bfs_slots(const void *k)
 {
+    if (k == (const void *)bfs_slots_grid<false> || k == (const void *)bfs_slots_grid<true>) return true;
     for (int b : {256, 512, 1024})
         if (k == lanes_kernel_for<false>(b) || k == lanes_kernel_for<true>(b)) return true;
     return false;
+}
+
+// ---------------------------------------------------------------------------
+// The grid, a thread per frontier vertex: BFS on larger graphs of uniform low
+// degree (at most kUniformDegree edges a vertex, at most 4 on average).  Their
+// levels are many and small, so a level costs its chain of dependent memory
+// round trips and its barrier.  A vertex's slot (16 bytes: its up to 4
+// destinations) is one round trip where its row and its edges are two, and
+// needs no balancing across the warp.  Levels of at most kSlotsSmall vertices,
+// where a grid barrier and the global queue are most of the time, run on the
+// first CTA alone, with the frontier in its shared memory and __syncthreads
+// as the barrier; the other CTAs wait at the grid barrier.  Always top-down.
+// (Road 1021^2, four queries to the host: 4.62 -> 3.29 ms.)
+// ---------------------------------------------------------------------------
+constexpr int kSlotsBlock = 1024;
+constexpr uint32_t kSlotsHead = 2048;   // frontier entries in shared memory (later ones: global queue)
+#ifndef GFT_SLOTS_SMALL
+#define GFT_SLOTS_SMALL 512
+#endif
+constexpr uint32_t kSlotsSmall = GFT_SLOTS_SMALL;
+constexpr uint32_t kSlotsCtaFlush = 8192;  // from this many vertices on, one queue reservation per CTA
+
+// Claims up to 4 destinations in the global bitmap, all in flight together;
+// kProbe: a plain read first, so that visited vertices cost no atomic.
+template <bool kProbe>
+__device__ __forceinline__ void slots_claim(uint32_t *visited, const bool (&valid)[4], const uint32_t (&v)[4],
+                                            bool (&mine)[4])
+{
+    uint32_t word[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) word[k] = valid[k] ? (kProbe ? __ldcg(visited + (v[k] >> 5)) : 0u) : 0xFFFFFFFFu;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t b = 1u << (v[k] & 31);
+        uint32_t old = b;
+        if (!(word[k] & b)) old = atomicOr(visited + (v[k] >> 5), b);
+        mine[k] = !(old & b);
+    }
+}
+
+// The destinations of frontier vertex u of each lane, four at a time: f(mine,
+// v) for its slot, then for the edges of vertices that are read through the CSR.
+template <bool kProbe, class F>
+__device__ __forceinline__ void slots_visit(const TravParams &p, bool has, uint32_t u, unsigned &edges,
+                                            unsigned *err, F &&f)
+{
+    uint4 sl = make_uint4(kBfsSlotNone, kBfsSlotNone, kBfsSlotNone, kBfsSlotNone);
+    if (has) sl = __ldg(p.bfs_slots + u);
+    const bool csr = sl.x == kBfsSlotWide;
+    {
+        const uint32_t v[4] = {sl.x, sl.y, sl.z, sl.w};
+        bool valid[4], mine[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            valid[k] = v[k] < kBfsSlotWide;
+            edges += valid[k];
+        }
+        slots_claim<kProbe>(p.visited, valid, v, mine);
+        f(mine, v);
+    }
+    if (__any_sync(kFull, csr)) {
+        uint32_t s = 0, deg = 0;
+        if (csr) {
+            s = __ldg(p.row_start + u);
+            deg = __ldg(p.row_start + u + 1) - s;
+        }
+        edges += deg;
+        const unsigned max_deg = __reduce_max_sync(kFull, deg);
+        for (unsigned j = 0; j < max_deg; j += 4) {
+            uint32_t v[4];
+            bool valid[4], mine[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                v[k] = j + k < deg ? __ldg(p.edge_dst + s + j + k) : 0u;
+                valid[k] = j + k < deg && v[k] < p.nnodes;
+                if (j + k < deg && v[k] >= p.nnodes) atomicCAS(err, 0u, (unsigned)GFT_ERR_FORMAT);
+            }
+            slots_claim<kProbe>(p.visited, valid, v, mine);
+            f(mine, v);
+        }
+    }
+}
+
+template <bool kParent>
+__global__ void __launch_bounds__(kSlotsBlock, 1) bfs_slots_grid(TravParams p)
+{
+    __shared__ uint32_t s_buf[kSlotsBlock / 32][kQueueBuf];
+    __shared__ uint32_t s_head[2][kSlotsHead];
+    __shared__ unsigned s_len[3];
+    if ((int)blockIdx.x == p.skip_block) return;  // test hook: this CTA never arrives
+    TraversalCtl *ctl = p.ctl;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned tid = blockIdx.x * kSlotsBlock + threadIdx.x, nthreads = gridDim.x * kSlotsBlock;
+    const unsigned gwarp = warp * gridDim.x + blockIdx.x, nwarps = nthreads / 32;  // neighbours on different SMs
+    GridSync gs{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, gridDim.x, 0, p.timeout_ns};
+    const uint32_t n = p.nnodes, nwords = (n + 31) >> 5;
+    for (uint32_t v = tid; v < n; v += nthreads) {
+        p.out[v] = v == p.src ? 0 : (int32_t)kInf;
+        if (kParent) p.parent[v] = v == p.src ? p.src : GFT_NO_PARENT;
+    }
+    for (uint32_t w = tid; w < nwords; w += nthreads) p.visited[w] = w == (p.src >> 5) ? 1u << (p.src & 31) : 0u;
+    if (tid == 0) {
+        p.q[0][0] = p.src;
+        *u32_of(ctl->qlen[0]) = 1;
+    }
+    if (!gs.sync()) return;
+
+    WarpQueue q{s_buf[warp], 0, nullptr, nullptr, p.qcap, &ctl->error, &ctl->error_where};
+    unsigned edges = 0;  // of one level, or of one run of small levels
+    unsigned long long edges_all = 0, claimed = 0;
+    unsigned L = 0;
+    for (;;) {
+        const unsigned n_in = ld_relaxed_u32(u32_of(ctl->qlen[L % 3]));
+        if (n_in == 0) break;
+        edges_all += edges;
+        edges = 0;
+        if (n_in <= kSlotsSmall) {
+            // Every thread has read the length before the first CTA, which is
+            // about to overwrite it, goes on.
+            if (!gs.sync()) return;
+            if (blockIdx.x == 0) {
+                uint32_t *in = s_head[0], *out = s_head[1], *in_tail = sel2(p.q, L), *out_tail = sel2(p.q, L + 1);
+                if (threadIdx.x < n_in) in[threadIdx.x] = __ldcg(in_tail + threadIdx.x);
+                if (threadIdx.x == 0) s_len[1] = 0;
+                unsigned c = 0, nx = 1, cl = 2, len = n_in, claims = 0;
+                __syncthreads();
+                for (;;) {
+                    if (threadIdx.x == 0) s_len[cl] = 0;
+                    for (unsigned base = warp * 32; base < len; base += kSlotsBlock) {  // warp uniform
+                        const unsigned i = base + lane;
+                        uint32_t u = 0;
+                        if (i < len) u = i < kSlotsHead ? in[i] : __ldcg(in_tail + i);
+                        slots_visit<false>(p, i < len, u, edges, &ctl->error,
+                                           [&](const bool(&mine)[4], const uint32_t(&v)[4]) {
+                                               lanes_append<kParent, kSlotsHead>(p, mine, v, u, &s_len[nx], out, out_tail,
+                                                                                 (int32_t)L + 1, &ctl->error, lane, claims);
+                                           });
+                    }
+                    __syncthreads();
+                    L++;
+                    len = s_len[nx];
+                    const unsigned c0 = c;
+                    c = nx;
+                    nx = cl;
+                    cl = c0;
+                    uint32_t *t = in;
+                    in = out;
+                    out = t;
+                    t = in_tail;
+                    in_tail = out_tail;
+                    out_tail = t;
+                    if (len == 0 || len > 2 * kSlotsSmall) break;
+                }
+                claimed += claims;
+                // Hand the frontier and the level over.
+                for (unsigned i = threadIdx.x; i < min(len, kSlotsHead); i += kSlotsBlock) in_tail[i] = in[i];
+                if (threadIdx.x == 0) {
+                    *u32_of(ctl->qlen[L % 3]) = len;
+                    *u32_of(ctl->qlen[(L + 1) % 3]) = 0;
+                    *u32_of(ctl->qlen[(L + 2) % 3]) = 0;
+                    ctl->handoff[0].v = L;
+                }
+            }
+            if (!gs.sync()) return;
+            L = (unsigned)ld_relaxed_u64(&ctl->handoff[0].v);
+            continue;
+        }
+        if (tid == 0) *u32_of(ctl->qlen[(L + 2) % 3]) = 0;
+        q.queue = sel2(p.q, L + 1);
+        q.len = u32_of(ctl->qlen[(L + 1) % 3]);
+        const uint32_t *in = sel2(p.q, L);
+        for (unsigned base = gwarp * 32; base < n_in; base += nwarps * 32) {  // warp uniform
+            const unsigned i = base + lane;
+            const uint32_t u = i < n_in ? __ldcg(in + i) : 0u;
+            slots_visit<true>(p, i < n_in, u, edges, &ctl->error, [&](const bool(&mine)[4], const uint32_t(&v)[4]) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (mine[k]) {
+                        p.out[v[k]] = (int32_t)L + 1;
+                        if (kParent) p.parent[v[k]] = u;
+                        claimed++;
+                    }
+                    q.push(mine[k], v[k], lane);
+                }
+            });
+        }
+        // The many warps of a large level hold a few items each; those of a
+        // small one are few, and a CTA-wide step costs more than it saves.
+        if (n_in >= kSlotsCtaFlush) cta_flush(q, lane);
+        else q.flush(lane);
+        if (!gs.sync()) return;
+        L++;
+    }
+    warp_add_u64(&ctl->edges, edges_all + edges, lane);
+    warp_add_u64(&ctl->reached, claimed, lane);
+    if (tid == 0) {
+        ctl->levels = L;
+        ctl->iterations = gs.epoch;
+    }
 }
 
 __global__ void __launch_bounds__(kCtaBlock, 1) sssp_single_cta(TravParams p)
@@ -504,12 +706,13 @@ struct Tune {
     uint32_t fuse;
     uint32_t tile;         // push-buffer entries per warp of the grid kernels (0 = default)
     uint32_t warp_degree;  // degree from which a warp expands a vertex by itself
+    bool shaped;           // the caller chose the grid kernels' launch shape or expansion
 };
 
 Tune resolve_tuning(const gft_tuning *t, bool is_sssp)
 {
     Tune r{is_sssp ? kDefaultBlockSssp : kDefaultBlockBfs, kDefaultBlocksPerSm, kDefaultHubDegree, kDefaultTimeoutMs,
-           -1, 0, 0, 0, 0, 0, dev::kDefaultWarpDegree};
+           -1, 0, 0, 0, 0, 0, dev::kDefaultWarpDegree, false};
     if (t) {
         if (t->block_threads) r.block = t->block_threads;
         if (t->blocks_per_sm) r.bps = t->blocks_per_sm;
@@ -522,6 +725,7 @@ Tune resolve_tuning(const gft_tuning *t, bool is_sssp)
         r.fuse = t->fuse_budget;
         r.tile = t->queue_tile;
         if (t->warp_degree) r.warp_degree = t->warp_degree;
+        r.shaped = t->block_threads || t->blocks_per_sm || t->hub_degree || t->queue_tile || t->warp_degree;
     }
     return r;
 }
@@ -608,6 +812,18 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
                                                        : (const void *)dev::bfs_single_cta<false>;
         }
     } else {
+        // Graphs of uniform low degree: the slot kernel, unless the caller asks
+        // for a shape of the general one.  On more than 4 edges a vertex
+        // most slots would only point to the CSR, and bottom-up levels may
+        // pay, which the general kernel runs.
+        if (!is_sssp && !t.shaped && !G.wrapped && G.max_degree <= kUniformDegree && G.nedges <= 4ull * G.nnodes) {
+            GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
+            if (G.bfs_slots) {
+                kern = d_parent ? (const void *)dev::bfs_slots_grid<true> : (const void *)dev::bfs_slots_grid<false>;
+                t.block = dev::kSlotsBlock;
+                t.bps = 1;
+            }
+        }
         GFT_TRY(resolve_shape(e, kern, (int)t.block, (int)t.bps, 0, &shape));
         if (t.max_blocks && (uint32_t)shape.blocks > t.max_blocks) shape.blocks = (int)t.max_blocks;
     }
@@ -642,7 +858,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     p.edge_dst = G.edge_dst;
     p.edge_data = G.edge_data;
     p.edge_dw = is_sssp ? G.edge_dw : nullptr;
-    p.bfs_slots = dev::is_lanes_kernel(kern) ? G.bfs_slots : nullptr;
+    p.bfs_slots = dev::reads_bfs_slots(kern) ? G.bfs_slots : nullptr;
     p.nnodes = n;
     p.src = src;
     p.out = d_out;

@@ -146,6 +146,17 @@ struct GridSync {
     }
 };
 
+// Inclusive warp prefix sum.
+__device__ __forceinline__ uint32_t warp_incl_sum(uint32_t x, unsigned lane)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        uint32_t t = __shfl_up_sync(kFull, x, o);
+        if (lane >= (unsigned)o) x += t;
+    }
+    return x;
+}
+
 // Entries of each warp's shared-memory push buffer (a multiple of 32, at
 // least 64).  A larger buffer means fewer reservations on the queue's one
 // length counter, whose atomics serialise in a single L2 slice.
@@ -174,7 +185,14 @@ struct WarpQueueT {
         __syncwarp();
         unsigned base = 0;
         if (lane == 0) base = atomicAdd(len, count);
-        base = __shfl_sync(kFull, base, 0);
+        store_at(__shfl_sync(kFull, base, 0), lane);
+    }
+
+    // Moves the buffer to the queue's entries [base, base + count).
+    __device__ __forceinline__ void store_at(unsigned base, unsigned lane)
+    {
+        if (count == 0) return;
+        __syncwarp();
         if (base + count > cap) {
             if (lane == 0) raise_error(err, err_where, GFT_ERR_OVERFLOW, base);
         } else {
@@ -195,15 +213,26 @@ struct WarpQueueT {
 };
 using WarpQueue = WarpQueueT<kQueueBuf>;
 
-// Inclusive warp prefix sum.
-__device__ __forceinline__ uint32_t warp_incl_sum(uint32_t x, unsigned lane)
+// Appends what the warps of a CTA still hold for one queue (the same in every
+// warp) with one reservation per CTA instead of one per warp: reservations on
+// a queue's one length counter serialise in L2.  Every thread of the CTA calls
+// this and synchronises the CTA before the next call.
+template <unsigned CAP>
+__device__ __forceinline__ void cta_flush(WarpQueueT<CAP> &a, unsigned lane)
 {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(kFull, x, o);
-        if (lane >= (unsigned)o) x += t;
+    __shared__ unsigned s_count[32], s_base[32];
+    const unsigned w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (lane == 0) s_count[w] = a.count;
+    __syncthreads();
+    if (w == 0) {
+        const unsigned c = lane < nw ? s_count[lane] : 0u;
+        const unsigned incl = warp_incl_sum(c, lane), total = __shfl_sync(kFull, incl, 31);
+        unsigned base = 0;
+        if (lane == 0 && total) base = atomicAdd(a.len, total);
+        s_base[lane] = __shfl_sync(kFull, base, 0) + incl - c;
     }
-    return x;
+    __syncthreads();
+    a.store_at(s_base[w], lane);
 }
 
 // Flattened expansion of the edge ranges [start, start+deg) held one per

@@ -465,3 +465,47 @@ def test_direction_optimising_on_a_uniform_low_diameter_graph(gft, orc, engine):
         assert orc.check_tree(rs, dst, None, src, got, par) == 0
         _, _, r_td = _run_bfs(gft, engine, dg, src, {"direction": 1})
         assert r["edges_scanned"] < r_td["edges_scanned"]
+
+
+def _slot_graph(kind):
+    """Graphs of more than 2^17 vertices, at most 4 edges a vertex on average
+    and 32 at most: the slot BFS on the grid."""
+    n = 150_000
+    rng = np.random.default_rng(31)
+    if kind == "tree":  # frontiers 1, 3, 9, ...: through every threshold, then the leaves
+        v = np.arange(1, n)
+        pairs = np.stack([(v - 1) // 3, v], 1)
+    elif kind == "bursts":  # a path of hubs with 29 leaves: wide vertices on tiny and on large levels
+        v = np.arange(1, n)
+        pairs = np.stack([np.where(v % 30 == 0, v - 30, v - v % 30), v], 1)
+    else:  # "random": a few levels of tens of thousands of vertices
+        pairs = rng.integers(0, n, size=(2 * n - n // 8, 2))
+        pairs = pairs[pairs[:, 0] != pairs[:, 1]]
+    a, b = np.concatenate([pairs[:, 0], pairs[:, 1]]), np.concatenate([pairs[:, 1], pairs[:, 0]])
+    order = np.argsort(a, kind="stable")
+    rs = np.concatenate([[0], np.cumsum(np.bincount(a, minlength=n))]).astype(np.uint32)
+    assert int(np.diff(rs.astype(np.int64)).max()) <= 32 and len(a) <= 4 * n
+    return rs, b[order].astype(np.uint32)
+
+
+@pytest.mark.parametrize("kind", ["tree", "bursts", "random"])
+def test_slot_bfs_on_the_grid(gft, orc, engine, kind):
+    rs, dst = _slot_graph(kind)
+    dg = gft.CSRGraph(rs, dst).copy_to_gpu()
+    for src in (0, 1, 149_999, 75_008):
+        want = orc.bfs(rs, dst, src)
+        got, par, r = _run_bfs(gft, engine, dg, src)
+        np.testing.assert_array_equal(got, want)
+        assert orc.check_tree(rs, dst, None, src, got, par) == 0
+        reached = want != np.iinfo(np.int32).max
+        assert r["levels"] == want[reached].max() + 1 and r["vertices_reached"] == reached.sum() - 1
+        assert r["edges_scanned"] == int(np.diff(rs.astype(np.int64))[reached].sum())
+
+
+def test_slot_bfs_reports_an_edge_leaving_the_graph(gft, engine):
+    rs, dst = _slot_graph("tree")
+    dst[rs[40_000]] = 150_000
+    dg = gft.CSRGraph(rs, dst).copy_to_gpu()
+    with pytest.raises(gft.GftError) as ei:
+        engine.bfs(dg, 0)
+    assert ei.value.status_name == "GFT_ERR_FORMAT"
