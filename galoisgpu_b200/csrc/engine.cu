@@ -12,6 +12,7 @@
 
 #include <algorithm>
 
+#include "frontier.cuh"
 #include "gft_internal.h"
 
 namespace gft {
@@ -63,27 +64,11 @@ __global__ void first_bad_edge(const uint32_t *__restrict__ dst, uint32_t m, uin
         }
 }
 
-// One 16-byte slot per vertex: its destinations, or kBfsSlotWide for a
-// vertex of more than 4 edges or of an edge leaving the graph.
 __global__ void build_bfs_slots(const uint32_t *__restrict__ row_start, const uint32_t *__restrict__ dst, uint32_t n,
                                 uint4 *__restrict__ slots)
 {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t s = row_start[v], d = row_start[v + 1] - s;
-        uint4 x = make_uint4(kBfsSlotNone, kBfsSlotNone, kBfsSlotNone, kBfsSlotNone);
-        if (d > 4) x.x = kBfsSlotWide;
-        else {
-            if (d > 0) x.x = dst[s];
-            if (d > 1) x.y = dst[s + 1];
-            if (d > 2) x.z = dst[s + 2];
-            if (d > 3) x.w = dst[s + 3];
-            // A destination outside the graph sends the vertex through the
-            // CSR, whose reader reports it; slot destinations are in range.
-            if ((d > 0 && x.x >= n) || (d > 1 && x.y >= n) || (d > 2 && x.z >= n) || (d > 3 && x.w >= n))
-                x = make_uint4(kBfsSlotWide, kBfsSlotNone, kBfsSlotNone, kBfsSlotNone);
-        }
-        slots[v] = x;
-    }
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        slots[v] = bfs_slot_of(dst, row_start[v], row_start[v + 1], n);
 }
 
 __global__ void interleave_edges(const uint32_t *__restrict__ dst, const int32_t *__restrict__ w, uint32_t m,

@@ -54,6 +54,7 @@ struct TravParams {
     uint32_t qcap;
     uint32_t delta;
     TraversalCtl *ctl;
+    TraversalCtl *result;  // one-CTA thread-per-vertex BFS: the host's pinned copy of the results
     unsigned long long timeout_ns;
     int skip_block;
     int vec_ok;
@@ -64,6 +65,23 @@ struct TravParams {
     uint32_t fuse;       // SSSP: near vertices a warp may expand itself in the iteration that found them (0 = none)
     uint32_t warp_degree = kDefaultWarpDegree;  // a vertex of at least this many edges is expanded by a whole warp
 };
+
+// A vertex's BFS slot from its edges [s, e): up to 4 destinations, or
+// kBfsSlotWide for a vertex of more edges or of an edge leaving the graph,
+// which goes through the CSR, whose reader reports it.
+__device__ __forceinline__ uint4 bfs_slot_of(const uint32_t *__restrict__ dst, uint32_t s, uint32_t e, uint32_t n)
+{
+    uint32_t x[4];
+    const uint32_t d = e - s;
+    bool wide = d > 4;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+        x[k] = k < d && d <= 4 ? __ldg(dst + s + k) : kBfsSlotNone;
+        wide |= k < d && x[k] >= n;
+    }
+    return wide ? make_uint4(kBfsSlotWide, kBfsSlotNone, kBfsSlotNone, kBfsSlotNone)
+                : make_uint4(x[0], x[1], x[2], x[3]);
+}
 
 // ---------------------------------------------------------------------------
 // Visitors: what happens to one edge.

@@ -150,6 +150,11 @@ __global__ void __launch_bounds__(kCtaBlock, 1) bfs_single_cta(TravParams p)
 // ---------------------------------------------------------------------------
 constexpr uint32_t kLaneQueueHead = 8192;
 constexpr size_t kLaneSmemBytes = (kCtaLocalBitsNodes / 32 + 2 * (size_t)kLaneQueueHead) * 4;
+// Graphs of at most this many vertices keep their slots in shared memory too
+// (128 KB), filled from the CSR by the kernel itself: a level's slot load
+// is then tens of cycles, and a new graph's first query builds nothing.
+constexpr uint32_t kLaneStageNodes = 8192;
+constexpr size_t kLaneStageBytes = (size_t)kLaneStageNodes * sizeof(uint4);
 
 // One warp step's appends: claimed destinations v[k] (mine[k]) of frontier
 // vertex u go to the next frontier and get their level.  Each vertex is
@@ -203,14 +208,16 @@ __device__ __forceinline__ void lanes_append(const TravParams &p, const bool (&m
     }
 }
 
-template <int BLOCK, bool kParent>
+template <int BLOCK, bool kParent, bool kStage>
 __global__ void __launch_bounds__(BLOCK, 1) bfs_cta_lanes(TravParams p)
 {
     extern __shared__ __align__(16) uint32_t s_lane[];
     uint32_t *bits = s_lane;
     uint32_t *const head0 = bits + kCtaLocalBitsNodes / 32, *const head1 = head0 + kLaneQueueHead;
+    uint4 *const s_slots = reinterpret_cast<uint4 *>(head1 + kLaneQueueHead);
     __shared__ unsigned s_len[3];
     __shared__ unsigned s_err;
+    __shared__ unsigned long long s_edges, s_reached;
     const unsigned tid = threadIdx.x, lane = tid & 31;
     const uint32_t n = p.nnodes, nwords = (n + 31) >> 5;
     for (uint32_t v = tid; v < n; v += BLOCK) {
@@ -218,12 +225,18 @@ __global__ void __launch_bounds__(BLOCK, 1) bfs_cta_lanes(TravParams p)
         if (kParent) p.parent[v] = v == p.src ? p.src : GFT_NO_PARENT;
     }
     for (uint32_t w = tid; w < nwords; w += BLOCK) bits[w] = w == (p.src >> 5) ? 1u << (p.src & 31) : 0u;
+    if (kStage) {
+        for (uint32_t v = tid; v < n; v += BLOCK)
+            s_slots[v] = bfs_slot_of(p.edge_dst, __ldg(p.row_start + v), __ldg(p.row_start + v + 1), n);
+    }
     if (tid == 0) {
         head0[0] = p.src;
         s_len[0] = 1;
         s_len[1] = 0;
         s_len[2] = 0;
         s_err = 0;
+        s_edges = 0;
+        s_reached = 0;
     }
     __syncthreads();
 
@@ -254,8 +267,9 @@ __global__ void __launch_bounds__(BLOCK, 1) bfs_cta_lanes(TravParams p)
             bool csr = false;
             if (i < n_in) {
                 u = i < kLaneQueueHead ? in_head[i] : __ldcg(in_tail + i);
-                if (slots) sl = __ldg(slots + u);
-                csr = !slots || sl.x == kBfsSlotWide;
+                if (kStage) sl = s_slots[u];
+                else if (slots) sl = __ldg(slots + u);
+                csr = (!kStage && !slots) || sl.x == kBfsSlotWide;
                 if (csr) sl = none;
             }
             // Slot destinations.  The four claims go out together, with no
@@ -320,12 +334,21 @@ __global__ void __launch_bounds__(BLOCK, 1) bfs_cta_lanes(TravParams p)
         out_head = const_cast<uint32_t *>(ih);
         out_tail = const_cast<uint32_t *>(it);
     }
-    warp_add_u64(&p.ctl->edges, edges, lane);
-    warp_add_u64(&p.ctl->reached, claimed, lane);
+    warp_add_u64(&s_edges, edges, lane);
+    warp_add_u64(&s_reached, claimed, lane);
+    __syncthreads();
     if (tid == 0) {
-        p.ctl->levels = L;
-        p.ctl->iterations = L + 1;  // barriers, as the general kernel counts them
-        if (s_err) p.ctl->error = s_err;
+        // Every field the host reads, straight into its pinned copy: the call
+        // needs no clearing before the launch and no copy after it.
+        TraversalCtl *r = p.result;
+        r->error = s_err;
+        r->error_where = 0;
+        r->levels = L;
+        r->iterations = L + 1;  // barriers, as the general kernel counts them
+        r->threshold = 0;
+        r->edges = s_edges;
+        r->pushes = 0;
+        r->reached = s_reached;
     }
 }
 
@@ -341,27 +364,18 @@ __host__ __forceinline__ int lanes_block_for(uint32_t nnodes)
     // Graphs here have at most kCtaLocalBitsNodes vertices.
     return nnodes <= (1u << 16) ? 256 : 1024;
 }
-template <bool kParent>
+template <bool kParent, bool kStage>
 __host__ inline const void *lanes_kernel_for(int block)
 {
-    return block <= 256   ? (const void *)bfs_cta_lanes<256, kParent>
-           : block <= 512 ? (const void *)bfs_cta_lanes<512, kParent>
-                          : (const void *)bfs_cta_lanes<1024, kParent>;
+    return block <= 256   ? (const void *)bfs_cta_lanes<256, kParent, kStage>
+           : block <= 512 ? (const void *)bfs_cta_lanes<512, kParent, kStage>
+                          : (const void *)bfs_cta_lanes<1024, kParent, kStage>;
 }
-__host__ inline const void *lanes_kernel_for(int block, bool parent)
+__host__ inline const void *lanes_kernel_for(int block, bool parent, bool stage)
 {
-    return parent ? lanes_kernel_for<true>(block) : lanes_kernel_for<false>(block);
+    return stage ? (parent ? lanes_kernel_for<true, true>(block) : lanes_kernel_for<false, true>(block))
+                 : (parent ? lanes_kernel_for<true, false>(block) : lanes_kernel_for<false, false>(block));
 }
-template <bool kParent>
-__global__ void bfs_slots_grid(TravParams p);
-__host__ inline bool reads_bfs_slots(const void *k)
-{
-    if (k == (const void *)bfs_slots_grid<false> || k == (const void *)bfs_slots_grid<true>) return true;
-    for (int b : {256, 512, 1024})
-        if (k == lanes_kernel_for<false>(b) || k == lanes_kernel_for<true>(b)) return true;
-    return false;
-}
-
 // ---------------------------------------------------------------------------
 // The grid, a thread per frontier vertex: BFS on larger graphs of uniform low
 // degree (at most kUniformDegree edges a vertex, at most 4 on average).  Their
@@ -732,12 +746,15 @@ Tune resolve_tuning(const gft_tuning *t, bool is_sssp)
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-gft_status finish(gft_engine *e, cudaStream_t stream, const LaunchShape &shape, gft_stats *stats, const char *what)
+// copy: bring the results back from the device's control block.
+gft_status finish(gft_engine *e, cudaStream_t stream, const LaunchShape &shape, bool copy, gft_stats *stats,
+                  const char *what)
 {
     TraversalCtl *hctl = reinterpret_cast<TraversalCtl *>(e->host_ctl);
     const size_t cold = offsetof(TraversalCtl, error);
-    GFT_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<char *>(hctl) + cold, reinterpret_cast<char *>(e->ctl.ptr) + cold,
-                                 sizeof(TraversalCtl) - cold, cudaMemcpyDeviceToHost, stream));
+    if (copy)
+        GFT_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<char *>(hctl) + cold, reinterpret_cast<char *>(e->ctl.ptr) + cold,
+                                     sizeof(TraversalCtl) - cold, cudaMemcpyDeviceToHost, stream));
     GFT_CUDA_TRY(cudaStreamSynchronize(stream));
     if (hctl->error)
         return fail((gft_status)hctl->error, "%s: device reported %s (site %u)", what,
@@ -789,6 +806,8 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
                                               G.nedges <= kCtaMaxEdges);
     LaunchShape shape;
     size_t dyn_smem = 0;
+    const uint4 *slots = nullptr;
+    bool lanes = false;  // the thread-per-vertex kernel on one CTA, which writes its results to the host itself
     if (single) {
         shape.block_threads = dev::kCtaBlock;
         shape.blocks = 1;
@@ -803,9 +822,12 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
             // these graphs stay near the square root of the vertex count.
             const int lanes_block = dev::lanes_block_for(G.nnodes);
             shape.block_threads = lanes_block;
-            kern = dev::lanes_kernel_for(lanes_block, d_parent != nullptr);
-            dyn_smem = dev::kLaneSmemBytes;
-            if (!G.wrapped) GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
+            const bool stage = G.nnodes <= dev::kLaneStageNodes;
+            lanes = true;
+            kern = dev::lanes_kernel_for(lanes_block, d_parent != nullptr, stage);
+            dyn_smem = dev::kLaneSmemBytes + (stage ? dev::kLaneStageBytes : 0);
+            if (!G.wrapped && !stage) GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
+            slots = G.bfs_slots;
             GFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem));
         } else {
             kern = G.nnodes <= dev::kCtaLocalBitsNodes ? (const void *)dev::bfs_single_cta<true>
@@ -819,6 +841,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
         if (!is_sssp && !t.shaped && !G.wrapped && G.max_degree <= kUniformDegree && G.nedges <= 4ull * G.nnodes) {
             GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
             if (G.bfs_slots) {
+                slots = G.bfs_slots;
                 kern = d_parent ? (const void *)dev::bfs_slots_grid<true> : (const void *)dev::bfs_slots_grid<false>;
                 t.block = dev::kSlotsBlock;
                 t.bps = 1;
@@ -858,7 +881,8 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     p.edge_dst = G.edge_dst;
     p.edge_data = G.edge_data;
     p.edge_dw = is_sssp ? G.edge_dw : nullptr;
-    p.bfs_slots = dev::reads_bfs_slots(kern) ? G.bfs_slots : nullptr;
+    p.bfs_slots = slots;
+    p.result = reinterpret_cast<TraversalCtl *>(e->host_ctl);
     p.nnodes = n;
     p.src = src;
     p.out = d_out;
@@ -889,7 +913,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
         p.cta_small = t.cta_small == UINT32_MAX ? 0 : t.cta_small ? t.cta_small : p.uniform ? kDefaultCtaSmall : 0;
     if (is_sssp) p.fuse = t.fuse == UINT32_MAX ? 0 : t.fuse ? t.fuse : p.uniform ? kDefaultFuse : 0;
 
-    GFT_CUDA_TRY(cudaMemsetAsync(e->ctl.ptr, 0, sizeof(TraversalCtl), stream));
+    if (!lanes) GFT_CUDA_TRY(cudaMemsetAsync(e->ctl.ptr, 0, sizeof(TraversalCtl), stream));
     void *args[] = {&p};
     GFT_CUDA_TRY(cudaEventRecord(e->ev0, stream));
     if (single)
@@ -904,7 +928,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
                                                                   n, src);
         GFT_CUDA_TRY(cudaGetLastError());
     }
-    return finish(e, stream, shape, stats, what);
+    return finish(e, stream, shape, !lanes, stats, what);
 }
 
 gft_status reach_stats(const gft_graph *g, const int32_t *d_val, cudaStream_t stream, uint64_t *v_r, uint64_t *e_r)

@@ -509,3 +509,17 @@ def test_slot_bfs_reports_an_edge_leaving_the_graph(gft, engine):
     with pytest.raises(gft.GftError) as ei:
         engine.bfs(dg, 0)
     assert ei.value.status_name == "GFT_ERR_FORMAT"
+
+
+@pytest.mark.parametrize("side", [1, 2, 90, 91])
+def test_one_cta_bfs_either_side_of_the_staged_slots(gft, orc, engine, side):
+    """Up to 8192 vertices (90^2 = 8100) the one-CTA kernel builds its slots in
+    shared memory, above (91^2 = 8281) it reads the graph's."""
+    g = gft.CSRGraph.grid(side, side)
+    dg = g.copy_to_gpu()
+    for src in {0, g.nnodes // 2, g.nnodes - 1}:
+        got, par, r = _run_bfs(gft, engine, dg, src)
+        want = orc.bfs(g.row_start, g.edge_dst, src)
+        np.testing.assert_array_equal(got, want)
+        assert orc.check_tree(g.row_start, g.edge_dst, None, src, got, par) == 0
+        assert r["levels"] == want.max() + 1 and r["vertices_reached"] == g.nnodes - 1
