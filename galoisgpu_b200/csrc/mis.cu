@@ -46,6 +46,7 @@ struct MisParams {
     unsigned long long *word;  // per vertex: priority << 32 | state
     int32_t *out;              // per vertex state, as the reference's node_data
     uint32_t prio_threads;     // priority streams (the reference's launch size)
+    uint32_t cta_small;        // grid: rounds of at most this many vertices run on one CTA (0 = never)
 };
 
 __device__ __forceinline__ uint32_t mis_state(unsigned long long w) { return (uint32_t)w; }
@@ -118,10 +119,21 @@ __device__ __forceinline__ void mis_pass(const MisParams &mp, Mode &m, const uin
                 if (lane == l) decided = found;
             }
             if (live && deg < 32) {
-                for (uint32_t e = start; e < start + deg && !decided; e++) {
-                    const uint32_t d = __ldcs(p.edge_dst + e);
-                    decided = mis_decides<MARK>(u, pu, d, __ldcg(mp.word + d));
-                    scanned++;
+                // Four neighbours at a time: their ids, then their words, are
+                // in flight together.
+                for (uint32_t e = start; e < start + deg && !decided; e += 4) {
+                    uint32_t d[4];
+                    unsigned long long w[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++) d[k] = e + k < start + deg ? __ldcs(p.edge_dst + e + k) : u;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++) w[k] = __ldcg(mp.word + d[k]);
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++)
+                        if (e + k < start + deg) {
+                            decided |= mis_decides<MARK>(u, pu, d[k], w[k]);
+                            scanned++;
+                        }
                 }
             }
             if (MARK) {
@@ -133,6 +145,31 @@ __device__ __forceinline__ void mis_pass(const MisParams &mp, Mode &m, const uin
         }
     }
     if (!MARK) q.flush(lane);
+}
+
+// Round L over its n_in worklist vertices; false when a barrier reported an
+// error.
+template <class Mode>
+__device__ __forceinline__ bool mis_round(const MisParams &mp, Mode &m, WarpQueue &q, unsigned &L, unsigned n_in,
+                                          unsigned long long &scanned, unsigned long long &pops)
+{
+    TraversalCtl *ctl = m.ctl;
+    const unsigned slot = L % 3, nslot = (L + 1) % 3, rslot = (L + 2) % 3;
+    pops += n_in;
+    if (m.tid == 0) {
+        *u32_of(ctl->qlen[rslot]) = 0;
+        *u32_of(ctl->claim[rslot]) = 0;
+        *u32_of(ctl->hub_claim[rslot]) = 0;
+    }
+    const uint32_t *in = sel2(mp.t.q, L);
+    mis_pass<true>(mp, m, in, n_in, u32_of(ctl->claim[slot]), q, scanned);
+    if (!m.sync()) return false;
+    q.queue = sel2(mp.t.q, L + 1);
+    q.len = u32_of(ctl->qlen[nslot]);
+    mis_pass<false>(mp, m, in, n_in, u32_of(ctl->hub_claim[slot]), q, scanned);
+    if (!m.sync()) return false;
+    L++;
+    return true;
 }
 
 template <class Mode>
@@ -170,25 +207,25 @@ __device__ __forceinline__ void mis_body(const MisParams &mp, Mode &m, uint32_t 
     q.err = &ctl->error;
     q.err_where = &ctl->error_where;
     unsigned long long scanned = 0, pops = 0;  // pops: thread 0's tally of worklist entries
-    unsigned L = 0;
+    unsigned L = 0, alone = 0;                 // alone: barriers of the rounds one CTA ran
     for (;;) {
-        const unsigned slot = L % 3, nslot = (L + 1) % 3, rslot = (L + 2) % 3;
-        const unsigned n_in = m.ld(u32_of(ctl->qlen[slot]));
+        const unsigned n_in = m.ld(u32_of(ctl->qlen[L % 3]));
         if (n_in == 0) break;
-        pops += n_in;
-        if (tid == 0) {
-            *u32_of(ctl->qlen[rslot]) = 0;
-            *u32_of(ctl->claim[rslot]) = 0;
-            *u32_of(ctl->hub_claim[rslot]) = 0;
+        if (Mode::kGrid && n_in <= mp.cta_small) {
+            // The worklist only shrinks: the first CTA runs all rounds that are
+            // left, while the others wait at the grid barrier.  It starts once
+            // every thread has read the length, which it is about to overwrite.
+            if (!m.sync()) return;
+            if (blockIdx.x == 0) {
+                CtaMode cm{ctl, threadIdx.x, blockDim.x, threadIdx.x >> 5, blockDim.x >> 5, 0};
+                for (unsigned nn = n_in; nn && mis_round(mp, cm, q, L, nn, scanned, pops);)
+                    nn = cm.ld(u32_of(ctl->qlen[L % 3]));
+                alone = cm.ep;
+            }
+            if (!m.sync()) return;
+            break;
         }
-        const uint32_t *in = sel2(p.q, L);
-        mis_pass<true>(mp, m, in, n_in, u32_of(ctl->claim[slot]), q, scanned);
-        if (!m.sync()) return;
-        q.queue = sel2(p.q, L + 1);
-        q.len = u32_of(ctl->qlen[nslot]);
-        mis_pass<false>(mp, m, in, n_in, u32_of(ctl->hub_claim[slot]), q, scanned);
-        if (!m.sync()) return;
-        L++;
+        if (!mis_round(mp, m, q, L, n_in, scanned, pops)) return;
     }
     // node_data for the caller, and the set's size.
     unsigned long long members = 0;
@@ -201,7 +238,7 @@ __device__ __forceinline__ void mis_body(const MisParams &mp, Mode &m, uint32_t 
     warp_add_u64(&ctl->reached, members, lane);
     if (tid == 0) {
         ctl->levels = L;
-        ctl->iterations = m.epoch();
+        ctl->iterations = m.epoch() + alone;
         ctl->pushes = pops;
     }
 }
@@ -319,6 +356,12 @@ gft_status run_mis(gft_engine *e, const gft_graph *g, int32_t *d_state, uint32_t
     mp.word = reinterpret_cast<unsigned long long *>(base + o_word);
     mp.out = d_state;
     mp.prio_threads = prio_threads;
+    // A round on the grid costs two barriers and their memory round trips,
+    // about 15 us however few vertices are left, and a mesh spends most of
+    // its rounds on the last thousand (2047^2 road grid: ~64 of 74).  With the
+    // four neighbours in flight together: 1374 -> 1173 us.  A skewed graph has few
+    // rounds, and its last vertices may have edges for the whole grid.
+    mp.cta_small = p.uniform ? 1024 : 0;
     GFT_CUDA_TRY(cudaMemsetAsync(e->ctl.ptr, 0, sizeof(TraversalCtl), stream));
     void *args[] = {&mp};
     GFT_CUDA_TRY(cudaEventRecord(e->ev0, stream));
