@@ -215,7 +215,7 @@ constexpr int kCcSamples = 1024;
 
 __global__ void __launch_bounds__(kCcSamples, 1) cc_sample_giant(const uint32_t *label, uint32_t n, uint32_t *giant)
 {
-    __shared__ uint32_t s_lab[kCcSamples];
+    __shared__ __align__(16) uint32_t s_lab[kCcSamples];
     __shared__ unsigned long long s_best;
     const uint32_t i = threadIdx.x;
     const uint32_t v = (uint32_t)(((unsigned long long)(i * 2654435761u + 12345u) * n) >> 32);
@@ -223,8 +223,13 @@ __global__ void __launch_bounds__(kCcSamples, 1) cc_sample_giant(const uint32_t 
     if (i == 0) s_best = 0;
     __syncthreads();
     uint32_t count = 0;
-    for (int j = 0; j < kCcSamples; j++) count += s_lab[j] == s_lab[i];
-    atomicMax(&s_best, ((unsigned long long)count << 32) | (0xFFFFFFFFu - s_lab[i]));
+    const uint32_t mine = s_lab[i];
+#pragma unroll 8
+    for (int j = 0; j < kCcSamples; j += 4) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(s_lab + j);
+        count += (x.x == mine) + (x.y == mine) + (x.z == mine) + (x.w == mine);
+    }
+    atomicMax(&s_best, ((unsigned long long)count << 32) | (0xFFFFFFFFu - mine));
     __syncthreads();
     if (i == 0) *giant = 0xFFFFFFFFu - (uint32_t)s_best;
 }
