@@ -390,10 +390,11 @@ __host__ inline const void *lanes_kernel_for(int block, bool parent, bool stage)
 // ---------------------------------------------------------------------------
 constexpr int kSlotsBlock = 1024;
 constexpr uint32_t kSlotsHead = 2048;   // frontier entries in shared memory (later ones: global queue)
-#ifndef GFT_SLOTS_SMALL
-#define GFT_SLOTS_SMALL 512
-#endif
-constexpr uint32_t kSlotsSmall = GFT_SLOTS_SMALL;
+constexpr uint32_t kSlotsSmall = 512;
+// Small levels the first CTA runs before the others pass a barrier: their
+// bounded wait is one of at most this many levels (about 4 ms), however long
+// the graph is.
+constexpr uint32_t kSlotsRun = 4096;
 constexpr uint32_t kSlotsCtaFlush = 8192;  // from this many vertices on, one queue reservation per CTA
 
 // Claims up to 4 destinations in the global bitmap, all in flight together;
@@ -499,6 +500,7 @@ __global__ void __launch_bounds__(kSlotsBlock, 1) bfs_slots_grid(TravParams p)
                 if (threadIdx.x < n_in) in[threadIdx.x] = __ldcg(in_tail + threadIdx.x);
                 if (threadIdx.x == 0) s_len[1] = 0;
                 unsigned c = 0, nx = 1, cl = 2, len = n_in, claims = 0;
+                const unsigned run_end = L + kSlotsRun;
                 __syncthreads();
                 for (;;) {
                     if (threadIdx.x == 0) s_len[cl] = 0;
@@ -525,7 +527,7 @@ __global__ void __launch_bounds__(kSlotsBlock, 1) bfs_slots_grid(TravParams p)
                     t = in_tail;
                     in_tail = out_tail;
                     out_tail = t;
-                    if (len == 0 || len > 2 * kSlotsSmall) break;
+                    if (len == 0 || len > 2 * kSlotsSmall || L == run_end) break;
                 }
                 claimed += claims;
                 // Hand the frontier and the level over.

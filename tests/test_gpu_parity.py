@@ -511,6 +511,22 @@ def test_slot_bfs_reports_an_edge_leaving_the_graph(gft, engine):
     assert ei.value.status_name == "GFT_ERR_FORMAT"
 
 
+def test_slot_bfs_wait_is_bounded_by_levels_not_by_the_graph(gft, engine):
+    """A path's 200,000 levels all run on the first CTA, about 0.2 s in all:
+    the other CTAs' waits stay below a 50 ms limit (a run of 4096 levels is
+    about 4 ms)."""
+    n = 200_000
+    v = np.arange(n)
+    deg = np.where((v == 0) | (v == n - 1), 1, 2)
+    rs = np.concatenate([[0], np.cumsum(deg)]).astype(np.uint32)
+    dst = np.stack([v - 1, v + 1], 1).ravel()
+    dst = dst[(dst >= 0) & (dst < n)].astype(np.uint32)
+    dg = gft.CSRGraph(rs, dst).copy_to_gpu()
+    r = engine.bfs(dg, 0, tune=gft.Tune(timeout_ms=50))
+    np.testing.assert_array_equal(r["out"].cpu().numpy(), v)
+    assert r["levels"] == n
+
+
 @pytest.mark.parametrize("side", [1, 2, 90, 91])
 def test_one_cta_bfs_either_side_of_the_staged_slots(gft, orc, engine, side):
     """Up to 8192 vertices (90^2 = 8100) the one-CTA kernel builds its slots in
