@@ -17,7 +17,9 @@
 // depends on the schedule: the set is a function of the priorities.
 //
 // Here one persistent cooperative launch runs every round (two grid
-// barriers per round), or one CTA for a small graph.  Each vertex has one
+// barriers per round), or one CTA for a small graph.  A mesh has many rounds
+// of few vertices, bound by their chains of memory round trips and barriers:
+// they run in registers (mis_resident).  Each vertex has one
 // 64-bit word, priority << 32 | state, so testing a neighbour is one 8-byte
 // load that answers both passes' questions.  Worklist vertices go one per
 // lane; a lane scans a list of fewer than 32 edges alone and stops at the
@@ -46,7 +48,6 @@ struct MisParams {
     unsigned long long *word;  // per vertex: priority << 32 | state
     int32_t *out;              // per vertex state, as the reference's node_data
     uint32_t prio_threads;     // priority streams (the reference's launch size)
-    uint32_t cta_small;        // grid: rounds of at most this many vertices run on one CTA (0 = never)
 };
 
 __device__ __forceinline__ uint32_t mis_state(unsigned long long w) { return (uint32_t)w; }
@@ -67,10 +68,10 @@ __device__ __forceinline__ bool mis_decides(uint32_t u, uint32_t pu, uint32_t d,
     return mis_state(wd) == kMisMarked;
 }
 
-// One pass over the worklist `in[0, n)`.  Mark: undecided (unbeaten)
-// vertices become MARKED.  Drop: MARKED vertices and those with a MARKED
-// neighbour leave (unmarked ones become NON_INDEPENDENT); the rest are
-// appended to q.
+// One pass over the worklist `in[0, n)` (NULL: the first n vertices).  Mark:
+// undecided (unbeaten) vertices become MARKED.  Drop: MARKED vertices and
+// those with a MARKED neighbour leave (unmarked ones become
+// NON_INDEPENDENT); the rest are appended to q.
 template <bool MARK, class Mode>
 __device__ __forceinline__ void mis_pass(const MisParams &mp, Mode &m, const uint32_t *in, uint32_t n,
                                          unsigned *claim, WarpQueue &q, unsigned long long &scanned)
@@ -88,7 +89,7 @@ __device__ __forceinline__ void mis_pass(const MisParams &mp, Mode &m, const uin
             uint32_t u = 0, start = 0, deg = 0, pu = 0;
             bool decided = false, live = has;
             if (has) {
-                u = __ldcg(in + idx);
+                u = in ? __ldcg(in + idx) : idx;
                 const unsigned long long wu = __ldcg(mp.word + u);
                 pu = mis_prio(wu);
                 if (!MARK && mis_state(wu) == kMisMarked) {
@@ -98,30 +99,11 @@ __device__ __forceinline__ void mis_pass(const MisParams &mp, Mode &m, const uin
                     deg = __ldg(p.row_start + u + 1) - start;
                 }
             }
-            // Lists of >= 32 edges: the whole warp, 32 edges a step, stops
-            // at the first deciding neighbour.
-            unsigned heavy = __ballot_sync(kFull, live && deg >= 32);
-            while (heavy) {
-                const int l = __ffs(heavy) - 1;
-                heavy &= heavy - 1;
-                const uint32_t hu = __shfl_sync(kFull, u, l), hs = __shfl_sync(kFull, start, l);
-                const uint32_t hd = __shfl_sync(kFull, deg, l), hp = __shfl_sync(kFull, pu, l);
-                bool found = false;
-                for (uint32_t e0 = 0; e0 < hd && !found; e0 += 32) {
-                    bool mine = false;
-                    if (e0 + lane < hd) {
-                        const uint32_t d = __ldcs(p.edge_dst + hs + e0 + lane);
-                        mine = mis_decides<MARK>(hu, hp, d, __ldcg(mp.word + d));
-                        scanned++;
-                    }
-                    found = __any_sync(kFull, mine);
-                }
-                if (lane == l) decided = found;
-            }
-            if (live && deg < 32) {
-                // Four neighbours at a time: their ids, then their words, are
-                // in flight together.
-                for (uint32_t e = start; e < start + deg && !decided; e += 4) {
+            // Four neighbours at a time: their ids, then their words, are in
+            // flight together.  A list of 32 edges or more has its first four
+            // looked at here too, which decide most vertices.
+            if (live) {
+                for (uint32_t e = start; e < start + deg && !decided && (deg < 32 || e == start); e += 4) {
                     uint32_t d[4];
                     unsigned long long w[4];
 #pragma unroll
@@ -136,6 +118,26 @@ __device__ __forceinline__ void mis_pass(const MisParams &mp, Mode &m, const uin
                         }
                 }
             }
+            // The rest of a list of >= 32 edges: the whole warp, 32 edges a
+            // step, stops at the first deciding neighbour.
+            unsigned heavy = __ballot_sync(kFull, live && !decided && deg >= 32);
+            while (heavy) {
+                const int l = __ffs(heavy) - 1;
+                heavy &= heavy - 1;
+                const uint32_t hu = __shfl_sync(kFull, u, l), hs = __shfl_sync(kFull, start, l);
+                const uint32_t hd = __shfl_sync(kFull, deg, l), hp = __shfl_sync(kFull, pu, l);
+                bool found = false;
+                for (uint32_t e0 = 4; e0 < hd && !found; e0 += 32) {
+                    bool mine = false;
+                    if (e0 + lane < hd) {
+                        const uint32_t d = __ldcs(p.edge_dst + hs + e0 + lane);
+                        mine = mis_decides<MARK>(hu, hp, d, __ldcg(mp.word + d));
+                        scanned++;
+                    }
+                    found = __any_sync(kFull, mine);
+                }
+                if (lane == l) decided = found;
+            }
             if (MARK) {
                 if (live && !decided) mis_set_state(mp.word, u, kMisMarked);
             } else {
@@ -144,7 +146,11 @@ __device__ __forceinline__ void mis_pass(const MisParams &mp, Mode &m, const uin
             }
         }
     }
-    if (!MARK) q.flush(lane);
+    if (!MARK) {
+        // Reservations on the one length counter serialise in L2.
+        if (Mode::kGrid && n >= kCtaFlush) cta_flush(q, lane);
+        else q.flush(lane);
+    }
 }
 
 // Round L over its n_in worklist vertices; false when a barrier reported an
@@ -161,7 +167,7 @@ __device__ __forceinline__ bool mis_round(const MisParams &mp, Mode &m, WarpQueu
         *u32_of(ctl->claim[rslot]) = 0;
         *u32_of(ctl->hub_claim[rslot]) = 0;
     }
-    const uint32_t *in = sel2(mp.t.q, L);
+    const uint32_t *in = L ? sel2(mp.t.q, L) : nullptr;  // round 0: every vertex
     mis_pass<true>(mp, m, in, n_in, u32_of(ctl->claim[slot]), q, scanned);
     if (!m.sync()) return false;
     q.queue = sel2(mp.t.q, L + 1);
@@ -170,6 +176,92 @@ __device__ __forceinline__ bool mis_round(const MisParams &mp, Mode &m, WarpQueu
     if (!m.sync()) return false;
     L++;
     return true;
+}
+
+// Rounds of a graph of uniform low degree once there is a thread for every
+// worklist vertex: a thread keeps its vertex, with its priority and first four
+// neighbours in registers, until it is decided, so a pass is one memory round
+// trip (the neighbours' words) and its barrier; the queue passes above take
+// about five trips, and a queue reservation per warp.  (2047^2 road grid,
+// rounds of 10^3 to 3 10^5 vertices: 12-21 -> 8-11 us each, the last ones, on
+// one CTA, 5.5 -> 2.2 us; all 83 rounds 1226 -> 835 us.)  Ends when at most
+// stop_at vertices are left, which then stand in the queue of round L, and
+// returns their number; ~0 when a barrier reported an error.
+template <class Mode>
+__device__ __forceinline__ unsigned mis_resident(const MisParams &mp, Mode &m, WarpQueue &q, unsigned &L, unsigned n_in,
+                                                 unsigned stop_at, unsigned long long &scanned,
+                                                 unsigned long long &pops)
+{
+    const TravParams &p = mp.t;
+    TraversalCtl *ctl = m.ctl;
+    const unsigned lane = threadIdx.x & 31;
+    // Neighbouring entries on one warp, neighbouring warps on different CTAs.
+    const unsigned i = Mode::kGrid ? ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane : threadIdx.x;
+    bool live = i < n_in;
+    uint32_t u = 0, pu = 0, start = 0, end = 0, d[4];
+    if (live) {
+        u = L ? __ldcg(sel2(p.q, L) + i) : i;
+        pu = mis_prio(__ldcg(mp.word + u));
+        start = __ldg(p.row_start + u);
+        end = __ldg(p.row_start + u + 1);
+    }
+    // u itself stands for "no neighbour": it never decides.
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) d[k] = start + k < end ? __ldg(p.edge_dst + start + k) : u;
+    for (;;) {
+        pops += n_in;
+        if (m.tid == 0) {
+            trace_iter(L, n_in);
+            *u32_of(ctl->qlen[(L + 2) % 3]) = 0;
+        }
+        bool marked = false;
+#pragma unroll
+        for (int pass = 0; pass < 2; pass++) {
+            if (live && !marked) {
+                unsigned long long w[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++) w[k] = d[k] != u ? __ldcg(mp.word + d[k]) : kMisExcluded;
+                bool decided = false;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++) {
+                    if (d[k] == u) continue;
+                    scanned++;
+                    decided |= pass == 0 ? mis_decides<true>(u, pu, d[k], w[k]) : mis_decides<false>(u, pu, d[k], w[k]);
+                    if (mis_state(w[k]) == kMisExcluded) d[k] = u;  // out for good
+                }
+                for (uint32_t e = start + 4; e < end && !decided; e++) {
+                    const uint32_t x = __ldg(p.edge_dst + e);
+                    const unsigned long long wx = __ldcg(mp.word + x);
+                    decided = pass == 0 ? mis_decides<true>(u, pu, x, wx) : mis_decides<false>(u, pu, x, wx);
+                    scanned++;
+                }
+                if (pass == 0 && !decided) {
+                    mis_set_state(mp.word, u, kMisMarked);
+                    marked = true;
+                }
+                if (pass == 1 && decided) {
+                    mis_set_state(mp.word, u, kMisExcluded);
+                    live = false;
+                }
+            }
+            if (pass == 0) {
+                if (!m.sync()) return ~0u;
+            }
+        }
+        live = live && !marked;
+        const unsigned left = __syncthreads_count(live);
+        if (threadIdx.x == 0 && left) atomicAdd(u32_of(ctl->qlen[(L + 1) % 3]), left);
+        if (!m.sync()) return ~0u;
+        L++;
+        n_in = m.ld(u32_of(ctl->qlen[L % 3]));
+        if (n_in <= stop_at) break;
+    }
+    if (n_in == 0) return 0;
+    q.queue = sel2(p.q, L);
+    q.len = u32_of(ctl->far_len[0]);  // zero until here
+    q.push(live, u, lane);
+    q.flush(lane);
+    return m.sync() ? n_in : ~0u;
 }
 
 template <class Mode>
@@ -181,8 +273,8 @@ __device__ __forceinline__ void mis_body(const MisParams &mp, Mode &m, uint32_t 
     const unsigned tid = m.tid, nthreads = m.nthreads;
     const uint32_t n = p.nnodes;
 
-    // Priorities (apps/mis/kernel.cu:18-41), state UNMARKED, and a worklist
-    // of every vertex (init_wl, :49-63).
+    // Priorities (apps/mis/kernel.cu:18-41) and state UNMARKED; the worklist of
+    // every vertex (init_wl, :49-63) is not written out.
     const uint32_t streams = min(mp.prio_threads, n);
     for (uint32_t s = tid; s < streams; s += nthreads) {
         uint32_t x = kMisSeed1 ^ s, y = kMisSeed2 ^ s, z = kMisSeed3 ^ s, w = kMisSeed4 ^ s;
@@ -196,7 +288,6 @@ __device__ __forceinline__ void mis_body(const MisParams &mp, Mode &m, uint32_t 
             mp.word[v] = ((unsigned long long)w << 32) | kMisUnmarked;
         }
     }
-    for (uint32_t v = tid; v < n; v += nthreads) p.q[0][v] = v;
     if (tid == 0) *u32_of(ctl->qlen[0]) = n;
     if (!m.sync()) return;
 
@@ -211,18 +302,19 @@ __device__ __forceinline__ void mis_body(const MisParams &mp, Mode &m, uint32_t 
     for (;;) {
         const unsigned n_in = m.ld(u32_of(ctl->qlen[L % 3]));
         if (n_in == 0) break;
-        if (Mode::kGrid && n_in <= mp.cta_small) {
-            // The worklist only shrinks: the first CTA runs all rounds that are
-            // left, while the others wait at the grid barrier.  It starts once
-            // every thread has read the length, which it is about to overwrite.
-            if (!m.sync()) return;
-            if (blockIdx.x == 0) {
-                CtaMode cm{ctl, threadIdx.x, blockDim.x, threadIdx.x >> 5, blockDim.x >> 5, 0};
-                for (unsigned nn = n_in; nn && mis_round(mp, cm, q, L, nn, scanned, pops);)
-                    nn = cm.ld(u32_of(ctl->qlen[L % 3]));
-                alone = cm.ep;
+        if (p.uniform && n_in <= nthreads) {
+            // On the grid, the last vertices go to the first CTA, whose barrier
+            // is __syncthreads, while the others wait at the grid barrier.
+            const unsigned left = mis_resident(mp, m, q, L, n_in, Mode::kGrid ? blockDim.x : 0u, scanned, pops);
+            if (left == ~0u) return;
+            if (left) {
+                if (blockIdx.x == 0) {
+                    CtaMode cm{ctl, threadIdx.x, blockDim.x, threadIdx.x >> 5, blockDim.x >> 5, 0};
+                    if (mis_resident(mp, cm, q, L, left, 0u, scanned, pops) == ~0u) return;
+                    alone = cm.ep;
+                }
+                if (!m.sync()) return;
             }
-            if (!m.sync()) return;
             break;
         }
         if (!mis_round(mp, m, q, L, n_in, scanned, pops)) return;
@@ -356,12 +448,6 @@ gft_status run_mis(gft_engine *e, const gft_graph *g, int32_t *d_state, uint32_t
     mp.word = reinterpret_cast<unsigned long long *>(base + o_word);
     mp.out = d_state;
     mp.prio_threads = prio_threads;
-    // A round on the grid costs two barriers and their memory round trips,
-    // about 15 us however few vertices are left, and a mesh spends most of
-    // its rounds on the last thousand (2047^2 road grid: ~64 of 74).  With the
-    // four neighbours in flight together: 1374 -> 1173 us.  A skewed graph has few
-    // rounds, and its last vertices may have edges for the whole grid.
-    mp.cta_small = p.uniform ? 1024 : 0;
     GFT_CUDA_TRY(cudaMemsetAsync(e->ctl.ptr, 0, sizeof(TraversalCtl), stream));
     void *args[] = {&mp};
     GFT_CUDA_TRY(cudaEventRecord(e->ev0, stream));

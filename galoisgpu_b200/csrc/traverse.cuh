@@ -213,26 +213,51 @@ struct WarpQueueT {
 };
 using WarpQueue = WarpQueueT<kQueueBuf>;
 
+// From this many frontier vertices on, a phase's last pushes take one queue
+// reservation per CTA instead of one per warp.
+constexpr unsigned kCtaFlush = 8192;
+
+// First entries of this warp's count_a and count_b entries in two queues (len_b
+// NULL: one queue), reserved for the whole CTA of at least two warps with one
+// addition per queue; the first in the low half of the result.  Every thread
+// of the CTA calls this and synchronises the CTA before the next call.  Not
+// inlined: its registers would cost the kernels' expansion loops spills.
+static __device__ __noinline__ unsigned long long cta_reserve(unsigned *len_a, unsigned count_a,
+                                                              unsigned *len_b, unsigned count_b)
+{
+    __shared__ unsigned s_count[2][32], s_base[2][32];
+    const unsigned w = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) {
+        s_count[0][w] = count_a;
+        s_count[1][w] = count_b;
+    }
+    __syncthreads();
+    if (w < 2) {
+        const unsigned c = lane < nw ? s_count[w][lane] : 0u;
+        const unsigned incl = warp_incl_sum(c, lane), total = __shfl_sync(kFull, incl, 31);
+        unsigned base = 0;
+        if (lane == 0 && total) base = atomicAdd(w ? len_b : len_a, total);
+        s_base[w][lane] = __shfl_sync(kFull, base, 0) + incl - c;
+    }
+    __syncthreads();
+    return s_base[0][w] | (unsigned long long)s_base[1][w] << 32;
+}
+
 // Appends what the warps of a CTA still hold for one queue (the same in every
 // warp) with one reservation per CTA instead of one per warp: reservations on
-// a queue's one length counter serialise in L2.  Every thread of the CTA calls
-// this and synchronises the CTA before the next call.
+// a queue's one length counter serialise in L2.
 template <unsigned CAP>
 __device__ __forceinline__ void cta_flush(WarpQueueT<CAP> &a, unsigned lane)
 {
-    __shared__ unsigned s_count[32], s_base[32];
-    const unsigned w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0) s_count[w] = a.count;
-    __syncthreads();
-    if (w == 0) {
-        const unsigned c = lane < nw ? s_count[lane] : 0u;
-        const unsigned incl = warp_incl_sum(c, lane), total = __shfl_sync(kFull, incl, 31);
-        unsigned base = 0;
-        if (lane == 0 && total) base = atomicAdd(a.len, total);
-        s_base[lane] = __shfl_sync(kFull, base, 0) + incl - c;
-    }
-    __syncthreads();
-    a.store_at(s_base[w], lane);
+    a.store_at((unsigned)cta_reserve(a.len, a.count, nullptr, 0), lane);
+}
+// The same for two queues.
+template <unsigned CAP>
+__device__ __forceinline__ void cta_flush2(WarpQueueT<CAP> &a, WarpQueueT<CAP> &b, unsigned lane)
+{
+    const unsigned long long base = cta_reserve(a.len, a.count, b.len, b.count);
+    a.store_at((unsigned)base, lane);
+    b.store_at((unsigned)(base >> 32), lane);
 }
 
 // Flattened expansion of the edge ranges [start, start+deg) held one per

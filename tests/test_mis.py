@@ -154,6 +154,35 @@ def test_gpu_mis_matches_oracle(gft, orc, engine, tune):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 1023, 1024, 1025, 3071, 3073, 20000])
+@pytest.mark.parametrize("directed", [False, True])
+def test_gpu_mis_rounds_in_registers(gft, orc, engine, n, directed):
+    """Graphs of at most 32 edges a vertex, with lists of 0, 1..4 and more
+    edges, self loops and duplicates, around the sizes at which three CTAs
+    hold every vertex in a thread, and at which one CTA holds the rest."""
+    rng = np.random.default_rng(n)
+    deg = rng.choice([0, 1, 2, 3, 4, 5, 9, 32] if directed else [0, 1, 2, 3, 4, 9], size=n)
+    a = np.repeat(np.arange(n), deg)
+    b = np.minimum(n - 1, np.maximum(0, a + rng.integers(-40, 41, size=len(a))))
+    if not directed:
+        a, b = np.concatenate([a, b]), np.concatenate([b, a])
+        keep = np.ones(len(a), bool)
+        for v in np.flatnonzero(np.bincount(a, minlength=n) > 32):
+            keep &= (a != v) & (b != v)
+        a, b = a[keep], b[keep]
+    order = np.argsort(a, kind="stable")
+    rs = np.concatenate([[0], np.cumsum(np.bincount(a, minlength=n))]).astype(np.uint32)
+    g = gft.CSRGraph(rs, b[order].astype(np.uint32))
+    dg = g.copy_to_gpu()
+    for nt in (_device_prio_threads(), 97):  # 97 streams: long chains of falling priorities, many rounds
+        want, steps = orc.mis(g.row_start, g.edge_dst, nt)
+        for tune in (None, {"max_blocks": 3, "blocks_per_sm": 1}, {"block_threads": 256, "max_blocks": 1 << 30}):
+            r = engine.mis(dg, prio_threads=nt, tune=gft.Tune(**tune) if tune else None)
+            np.testing.assert_array_equal(r["out"].cpu().numpy(), want)
+            assert r["levels"] == steps
+
+
+@pytest.mark.gpu
 def test_gpu_mis_host_variant_and_full_size_properties(gft, engine):
     dg = gft.DeviceGraph.generate("rmat", seed=5, scale=20, edge_factor=16)
     host = dg.download()
