@@ -395,7 +395,6 @@ constexpr uint32_t kSlotsSmall = 512;
 // bounded wait is one of at most this many levels (about 4 ms), however long
 // the graph is.
 constexpr uint32_t kSlotsRun = 4096;
-constexpr uint32_t kSlotsCtaFlush = 8192;  // from this many vertices on, one queue reservation per CTA
 
 // Claims up to 4 destinations in the global bitmap, all in flight together;
 // kProbe: a plain read first, so that visited vertices cost no atomic.
@@ -564,7 +563,7 @@ __global__ void __launch_bounds__(kSlotsBlock, 1) bfs_slots_grid(TravParams p)
         }
         // The many warps of a large level hold a few items each; those of a
         // small one are few, and a CTA-wide step costs more than it saves.
-        if (n_in >= kSlotsCtaFlush) cta_flush(q, lane);
+        if (n_in >= kCtaFlush) cta_flush(q, lane);
         else q.flush(lane);
         if (!gs.sync()) return;
         L++;
