@@ -45,6 +45,7 @@ struct TravParams {
     int32_t *out;       // level / dist
     uint32_t *parent;   // BFS parent or NULL
     uint32_t *visited;  // BFS bitmap
+    uint32_t *visited2;  // a second one for bottom-up levels, or NULL (see bottom_up_level)
     uint32_t *q[2];     // frontier / near pile
     uint32_t *far[2];   // SSSP far pile
     uint32_t *qstamp;   // SSSP: the last pile stamp per vertex (see SsspVisitorT); distances live in `out`
@@ -553,22 +554,32 @@ __device__ __forceinline__ unsigned pick_grain(unsigned n, unsigned nwarps, bool
 
 // One bottom-up BFS level (Beamer, Asanovic, Patterson, "Direction-Optimizing
 // Breadth-First Search", SC 2012): every unvisited vertex scans its own
-// edges, four at a time, for a neighbour in the current frontier (level ==
-// L) and stops at the first it finds.  On a symmetric graph a vertex's
-// out-edges are its in-edges, so this claims exactly the vertices a
-// top-down level would, with the same level.  Warps take 32-vertex words of
-// the visited bitmap and own them for the level, so each sets its word's
-// new bits with one plain store; claimed vertices are also queued, so a
-// top-down level can follow.
-template <bool kLocalBits, unsigned kQB>
+// edges, four at a time, for a visited neighbour and stops at the first it
+// finds.  On a symmetric graph a vertex's out-edges are its in-edges, and a
+// neighbour that was visited before the level began is in its frontier (the
+// neighbours of earlier frontiers are all visited), so this claims exactly the
+// vertices a top-down level would, with the same level.  `bits` is the visited
+// bitmap as the level began; the level writes the next one to `next`, a
+// word per warp step with a plain store.  A probe reads n / 8 bytes in all,
+// through L1, most often the hubs' words; a probe of the neighbour's level
+// is an L2 read (RMAT-24, four graphs: 582-707 -> 493-631 us a query).
+// Without kTwo (batched and served queries, whose arenas hold one bitmap, and
+// one CTA with its bitmap in shared memory) a probe reads the level and the
+// bitmap is updated in place: next == bits.  Claimed vertices are also
+// queued, so a top-down level can follow.
+template <bool kTwo, bool kLocalBits, unsigned kQB>
 __device__ __forceinline__ void bottom_up_level(BfsVisitorT<kLocalBits, kQB> &vis, const TravParams &p, unsigned L,
-                                                unsigned gwarp, unsigned nwarps, unsigned lane)
+                                                const uint32_t *bits, uint32_t *next, unsigned gwarp, unsigned nwarps,
+                                                unsigned lane)
 {
     const uint32_t n = p.nnodes, nwords = (n + 31) >> 5;
     const int32_t cur = (int32_t)L;
     for (uint32_t w = gwarp; w < nwords; w += nwarps) {
-        const uint32_t word = ld_bits<kLocalBits>(p.visited + w);
-        if (word == 0xFFFFFFFFu) continue;  // warp uniform
+        const uint32_t word = ld_bits<kLocalBits>(bits + w);
+        if (word == 0xFFFFFFFFu) {  // warp uniform
+            if (kTwo && lane == 0) next[w] = word;
+            continue;
+        }
         const uint32_t v = (w << 5) + lane;
         bool found = false;
         uint32_t par = 0, deg = 0;
@@ -577,14 +588,17 @@ __device__ __forceinline__ void bottom_up_level(BfsVisitorT<kLocalBits, kQB> &vi
             deg = e - s;
             for (uint32_t i = s; i < e && !found; i += 4) {
                 uint32_t u[4];
-                int32_t lv[4];
+                bool in[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++) u[k] = i + k < e ? ld_stream(p.edge_dst + i + k) : 0u;
 #pragma unroll
-                for (int k = 0; k < 4; k++) lv[k] = i + k < e ? __ldcg(p.out + u[k]) : -1;
+                for (int k = 0; k < 4; k++) {
+                    if constexpr (kTwo) in[k] = i + k < e && ((__ldca(bits + (u[k] >> 5)) >> (u[k] & 31)) & 1u);
+                    else in[k] = i + k < e && __ldcg(p.out + u[k]) == cur;
+                }
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    if (!found && lv[k] == cur) {
+                    if (!found && in[k]) {
                         found = true;
                         par = u[k];
                         vis.edges += k + 1;
@@ -599,7 +613,7 @@ __device__ __forceinline__ void bottom_up_level(BfsVisitorT<kLocalBits, kQB> &vi
             vis.claimed++;
             vis.mf += deg;
         }
-        if (lane == 0 && got) p.visited[w] = word | got;
+        if (lane == 0 && (got || kTwo)) next[w] = word | got;
         vis.q.push(found, v, lane);
     }
 }
@@ -651,7 +665,8 @@ constexpr unsigned kAlpha = 14, kBeta = 24, kScan = 32;
 
 // kLocalBits: p.visited points to shared memory (one CTA runs the traversal).
 // warp_buf: this warp's kQB-entry push buffer.
-template <class Mode, bool kLocalBits = false, unsigned kQB = kQueueBuf>
+// kTwo: bottom-up levels use the second bitmap p.visited2.
+template <class Mode, bool kLocalBits = false, unsigned kQB = kQueueBuf, bool kTwo = false>
 __device__ __forceinline__ void bfs_body(const TravParams &p, Mode &m, uint32_t *warp_buf)
 {
     using Vis = BfsVisitorT<kLocalBits, kQB>;
@@ -762,7 +777,9 @@ __device__ __forceinline__ void bfs_body(const TravParams &p, Mode &m, uint32_t 
         vis.q.len = u32_of(ctl->qlen[nslot]);
         unsigned *mf_next = u32_of(ctl->far_len[nslot]);
         if (bottom_up) {
-            bottom_up_level(vis, p, L, gwarp, nwarps, lane);
+            uint32_t *const next = !kTwo ? vis.visited : vis.visited == p.visited ? p.visited2 : p.visited;
+            bottom_up_level<kTwo>(vis, p, L, vis.visited, next, gwarp, nwarps, lane);
+            vis.visited = next;
         } else {
             const unsigned grain = max(min_grain, pick_grain(n_in, nwarps, p.uniform));
             expand_frontier<Vis, BfsOwn>(vis, p, sel2(p.q, L), n_in, u32_of(ctl->claim[slot]), &ctl->hub[slot].v,

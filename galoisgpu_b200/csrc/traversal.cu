@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(BLOCK, GFT_BFS_THREADS_PER_SM / BLOCK) bfs_per
     const unsigned tid = blockIdx.x * BLOCK + threadIdx.x, nthreads = gridDim.x * BLOCK;
     GridMode m{{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, gridDim.x, 0, p.timeout_ns},
                ctl, tid, nthreads, tid / 32, nthreads / 32};
-    bfs_body<GridMode, false, QB>(p, m, s_buf[threadIdx.x >> 5]);
+    bfs_body<GridMode, false, QB, true>(p, m, s_buf[threadIdx.x >> 5]);
 }
 
 // Default push buffers of the grid-wide SSSP kernel: 256 entries per warp up
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kCtaBlock, 1) bfs_single_cta(TravParams p)
     __syncthreads();
     TraversalCtl *gctl = p.ctl;
     p.ctl = &s_ctl;
-    if (kLocalBits) p.visited = s_bits;  // bfs_body clears the first (nnodes + 31) / 32 words
+    if (kLocalBits) p.visited = s_bits, p.visited2 = nullptr;  // bfs_body clears the first (nnodes + 31) / 32 words
     CtaMode m{&s_ctl, threadIdx.x, kCtaBlock, threadIdx.x >> 5, kCtaBlock / 32, 0};
     bfs_body<CtaMode, kLocalBits>(p, m, s_buf[threadIdx.x >> 5]);
     __syncthreads();
@@ -864,7 +864,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     };
     size_t o_q0 = take((size_t)qcap * 4), o_q1 = take((size_t)qcap * 4);
     size_t o_hubs = take((size_t)hub_cap * 8);
-    size_t o_vis = 0, o_f0 = 0, o_f1 = 0, o_qs = 0;
+    size_t o_vis = 0, o_vis2 = 0, o_f0 = 0, o_f1 = 0, o_qs = 0;
     if (is_sssp) {
         // Distances are computed in place in d_out; per vertex the engine
         // keeps only a pile stamp.
@@ -873,6 +873,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
         o_qs = take((size_t)n * 4);
     } else {
         o_vis = take((size_t)((n + 31) / 32) * 4);
+        o_vis2 = take((size_t)((n + 31) / 32) * 4);
     }
     GFT_TRY(e->scratch.ensure(off));
     char *base = reinterpret_cast<char *>(e->scratch.ptr);
@@ -897,6 +898,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
         p.qstamp = reinterpret_cast<uint32_t *>(base + o_qs);
     } else {
         p.visited = reinterpret_cast<uint32_t *>(base + o_vis);
+        p.visited2 = reinterpret_cast<uint32_t *>(base + o_vis2);
     }
     p.hub_cap = hub_cap;
     p.hub_degree = t.hub;
@@ -1087,7 +1089,7 @@ gft_status gft_reach_stats(const gft_graph *g, const int32_t *d_val, void *strea
 // framework that forbids allocations outside its own pool), and hot paths
 // where cudaMalloc / cudaFree are not allowed because of their implicit
 // synchronisation.  The traversal scratch (control block, two frontier
-// queues, visited bitmap, hub list) lives in one file-scope device array of
+// queues, two visited bitmaps, hub list) lives in one file-scope device array of
 // fixed size, sized for graphs of up to kNoAllocMaxNodes vertices; every GPU
 // that loads libgft holds it until the process exits.
 //
@@ -1110,7 +1112,7 @@ constexpr size_t kNoAllocCtlBytes = na_align(sizeof(TraversalCtl));
 constexpr size_t kNoAllocQueueBytes = na_align((size_t)kNoAllocMaxNodes * 4);
 constexpr size_t kNoAllocBitmapBytes = na_align((size_t)(kNoAllocMaxNodes / 32) * 4);
 constexpr size_t kNoAllocHubBytes = na_align((size_t)kNoAllocMaxNodes * 8);
-constexpr size_t kNoAllocBytes = kNoAllocCtlBytes + 2 * kNoAllocQueueBytes + kNoAllocBitmapBytes + kNoAllocHubBytes;
+constexpr size_t kNoAllocBytes = kNoAllocCtlBytes + 2 * kNoAllocQueueBytes + 2 * kNoAllocBitmapBytes + kNoAllocHubBytes;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -1174,7 +1176,8 @@ extern "C" gft_status gft_bfs_noalloc(const gft_graph *g, uint32_t src, int32_t 
     p.q[0] = reinterpret_cast<uint32_t *>(base + kNoAllocCtlBytes);
     p.q[1] = reinterpret_cast<uint32_t *>(base + kNoAllocCtlBytes + kNoAllocQueueBytes);
     p.visited = reinterpret_cast<uint32_t *>(base + kNoAllocCtlBytes + 2 * kNoAllocQueueBytes);
-    p.hubs = reinterpret_cast<uint2 *>(base + kNoAllocCtlBytes + 2 * kNoAllocQueueBytes + kNoAllocBitmapBytes);
+    p.visited2 = p.visited + kNoAllocBitmapBytes / 4;
+    p.hubs = reinterpret_cast<uint2 *>(base + kNoAllocCtlBytes + 2 * kNoAllocQueueBytes + 2 * kNoAllocBitmapBytes);
     p.hub_cap = (uint32_t)std::min<uint64_t>(G.nnodes, (uint64_t)G.nedges / hub + 1);
     p.hub_degree = hub;
     p.qcap = G.nnodes;

@@ -467,6 +467,39 @@ def test_direction_optimising_on_a_uniform_low_diameter_graph(gft, orc, engine):
         assert r["edges_scanned"] < r_td["edges_scanned"]
 
 
+@pytest.mark.parametrize("n", [60_000, 60_001, 60_031, 65_537])
+def test_bottom_up_levels_at_bitmap_edges(gft, orc, engine, n):
+    """Several bottom-up levels in a row and top-down levels after them, last
+    bitmap words of 1, 17 and 31 vertices and a full one: a core of random
+    edges (above the one-CTA size), layers of 2000 vertices behind it, a path
+    behind those, and vertices without edges at the end."""
+    rng = np.random.default_rng(n)
+    core, path = n - 25_000, 40
+    pairs = [np.stack([rng.integers(0, core, 300_000), rng.integers(0, core, 300_000)], 1)]
+    for layer in range(10):
+        lo = core + 2000 * layer
+        before = rng.integers(0, core, 6000) if layer == 0 else rng.integers(lo - 2000, lo, 6000)
+        pairs.append(np.stack([before, rng.integers(lo, lo + 2000, 6000)], 1))
+    v = core + 20_000 + np.arange(path)
+    pairs.append(np.stack([v - 1, v], 1))
+    e = np.concatenate(pairs)
+    a, b = np.concatenate([e[:, 0], e[:, 1]]), np.concatenate([e[:, 1], e[:, 0]])
+    order = np.argsort(a, kind="stable")
+    rs = np.concatenate([[0], np.cumsum(np.bincount(a, minlength=n))]).astype(np.uint32)
+    dst = b[order].astype(np.uint32)
+    dg = gft.CSRGraph(rs, dst).copy_to_gpu()
+    dg.symmetric = True
+    for src in (0, core - 1, core + 5000, core + 20_000 + path - 1):
+        want = orc.bfs(rs, dst, src)
+        got, par, r = _run_bfs(gft, engine, dg, src)
+        np.testing.assert_array_equal(got, want)
+        assert orc.check_tree(rs, dst, None, src, got, par) == 0
+        _, _, r_td = _run_bfs(gft, engine, dg, src, {"direction": 1})
+        assert r["levels"] == r_td["levels"]
+        if src == 0:  # top-down alone scans each reached edge once
+            assert r["edges_scanned"] != r_td["edges_scanned"]
+
+
 def _slot_graph(kind):
     """Graphs of more than 2^17 vertices, at most 4 edges a vertex on average
     and 32 at most: the slot BFS on the grid."""
