@@ -12,7 +12,7 @@
 //     w(1) = 1, w(2) = 2 / (2 - a^2), w(k+1) = 4 / (4 - a^2 w(k)).
 // It gains a factor (1 - sqrt(1 - a^2)) / a = 0.56 a sweep where a round of
 // pushes gains 0.85: about 25 sweeps over the edges instead of 104 rounds
-// (RMAT-22, 127 M edges: 67.0 -> 18.2 ms, and 5e-8 instead of 7e-5 from the
+// (RMAT-22, 127 M edges: 67.0 -> 14.2 ms, and 7e-8 instead of 7e-5 from the
 // 64-bit solution, as a hub's sum no longer swallows small addends).
 // A sweep reads a vertex's terms instead of adding to its neighbours'
 // residuals: no atomics, and a sum's order does not depend on the schedule.
@@ -63,7 +63,7 @@ struct PullState {
     unsigned asymmetric;      // pr_sample found an edge without its reverse; pr_sweeps: the pushes have to run
     unsigned outside;         // pr_relabel found an edge leaving the graph
     unsigned moved[3];        // per sweep, triple buffered: some rank moved by more than EPSILON
-    unsigned pad2;
+    unsigned unit[3];         // per sweep, triple buffered: units claimed beyond every warp's first
     unsigned rows[kPullClasses];    // rows of each class
     unsigned cursor[kPullClasses];  // rows of each class numbered so far
 };
@@ -384,24 +384,25 @@ struct PullSweep {
     }
 };
 
-// Rows of one class of q <= 4 * S quads: S lanes per row, U rows per group of
-// lanes at once, up to four quads per lane.  A lane's sum has at most 16
-// terms and a row's 256: 32-bit sums in a tree.
+// Chunks k0, k0 + step, ... below k1, of 32 / S rows of one class of q <= 4 * S
+// quads: S lanes per row, U rows per group of lanes at once, up to four
+// quads per lane.  A lane's sum has at most 16 terms and a row's 256: 32-bit
+// sums in a tree.
 template <int S, int U>
 __device__ __forceinline__ void pull_rows(PullSweep &sw, unsigned first, unsigned rows, uint32_t q, const uint4 *quads,
-                                          unsigned k0, unsigned nwarps, unsigned lane)
+                                          unsigned k0, unsigned k1, unsigned step, unsigned lane)
 {
     constexpr unsigned per = 32 / S;
-    const unsigned chunks = (rows + per - 1) / per, l = lane % S;
+    const unsigned l = lane % S;
     const uint4 pad = make_uint4(sw.hub_end, sw.hub_end, sw.hub_end, sw.hub_end);
-    for (unsigned k = k0; k < chunks; k += nwarps * U) {
+    for (unsigned k = k0; k < k1; k += step * U) {
         unsigned r[U];
         uint4 e[U];
         float acc[U], old[U], cur[U], inv[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            r[u] = (k + u * nwarps) * per + lane / S;
-            const bool has = k + u * nwarps < chunks && r[u] < rows;
+            r[u] = (k + u * step) * per + lane / S;
+            const bool has = k + u * step < k1 && r[u] < rows;
             if (!has) r[u] = rows;
             e[u] = has && l < q ? __ldcs(quads + (size_t)r[u] * q + l) : pad;
             old[u] = cur[u] = inv[u] = 0.f;
@@ -449,13 +450,13 @@ __device__ __forceinline__ void pull_rows(PullSweep &sw, unsigned first, unsigne
     }
 }
 
-// Rows of more quads, a warp per row, four quads per lane at once (fewer in
-// the last turn); the turns' sums are added in 64 bits.
-__device__ __forceinline__ void pull_long_rows(PullSweep &sw, unsigned first, unsigned rows, uint32_t q,
-                                               const uint4 *quads, unsigned k0, unsigned nwarps, unsigned lane)
+// Rows r0, r0 + step, ... below r1 of more quads, a warp per row, four quads per lane at once
+// (fewer in the last turn); the turns' sums are added in 64 bits.
+__device__ __forceinline__ void pull_long_rows(PullSweep &sw, unsigned first, unsigned r0, unsigned r1, unsigned step,
+                                               uint32_t q, const uint4 *quads, unsigned lane)
 {
     const uint4 pad = make_uint4(sw.hub_end, sw.hub_end, sw.hub_end, sw.hub_end);
-    for (unsigned r = k0; r < rows; r += nwarps) {
+    for (unsigned r = r0; r < r1; r += step) {
         const uint4 *row = quads + (size_t)r * q;
         float old = 0.f, cur = 0.f, inv = 0.f;
         if (lane == 0) {
@@ -480,10 +481,50 @@ __device__ __forceinline__ void pull_long_rows(PullSweep &sw, unsigned first, un
     }
 }
 
+// The sweeps' work list: the rows of the classes from c0 on, cut into units of
+// about `target` quads, a warp's claim.  Rows of one size do not cost the
+// same (their values are in shared memory, in L2 or in between), and warps
+// that were dealt equal shares waited for the slowest at each sweep's
+// barrier (22% of the warps' time, RMAT-21).
+struct PullUnits {
+    unsigned total;
+    unsigned first[kPullClasses];  // first unit of each class
+    unsigned chunks[kPullClasses];  // chunks (see pull_rows; a long row) per unit
+};
+
+__device__ __forceinline__ unsigned pull_chunks(uint32_t q, unsigned rows)
+{
+    const unsigned per = q > 64 ? 1u : 32 / pull_lanes(q);
+    return (rows + per - 1) / per;
+}
+
+__device__ __forceinline__ void pull_units(const PullTable &t, unsigned c0, uint32_t target, PullUnits &u)
+{
+    if (threadIdx.x < 32) {  // 32 classes at a time, in order
+        unsigned total = 0;
+        for (unsigned b = c0; b < t.n; b += 32) {
+            const unsigned c = b + threadIdx.x;
+            unsigned units = 0;
+            if (c < t.n) {
+                const uint32_t q = t.quads[c];
+                const unsigned size = max(1u, target / (q > 64 ? q : q * (32 / pull_lanes(q))));
+                u.chunks[c] = size;
+                units = (pull_chunks(q, t.rows[c]) + size - 1) / size;
+            }
+            const unsigned incl = warp_incl_sum(units, threadIdx.x);
+            if (c < t.n) u.first[c] = total + incl - units;
+            total += __shfl_sync(kFull, incl, 31);
+        }
+        if (threadIdx.x == 0) u.total = total;
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
 {
     extern __shared__ __align__(16) float s_hub[];
     __shared__ PullTable s_t;
+    __shared__ PullUnits s_u;
     __shared__ double s_red[2][32];
     TraversalCtl *ctl = p.ctl;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -504,6 +545,15 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
     // A row of more than a quarter of a warp's share of the quads (at least
     // 512 quads, four steps of a warp) is summed by a whole CTA.
     const uint32_t giant = max(512u, (uint32_t)(quads_total / (4ull * nwarps)));
+    // Units are claimed where rows differ.  On a graph of at most 32 edges a
+    // vertex the chunks are dealt in turn: they cost the same, and units of a
+    // few short rows would cost a claim each (1000^2 road grid: 0.48 ms
+    // dealt, 0.97 ms claimed; RMAT-22: 16.2 ms dealt, 14.1 ms claimed; RMAT-11:
+    // 0.65 and 0.23 ms).
+    const bool skewed = s_t.n && s_t.quads[0] > kUniformDegree / 4;
+    unsigned c0 = 0;
+    while (c0 < s_t.n && s_t.quads[c0] >= giant) c0++;
+    pull_units(s_t, c0, min(512u, max(32u, (uint32_t)(quads_total / (8ull * nwarps)))), s_u);
 
     // x(0): the share of a's flow that a vertex of its degree gets when every
     // vertex has the mean rank 1, a good guess for all that the
@@ -527,7 +577,10 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
         PullSweep sw{reinterpret_cast<const char *>(s_hub), zero, reinterpret_cast<const char *>(y),
                      cur ? p.y[0] : p.y[1], cur ? p.x[0] : p.x[1], cur ? p.x[1] : p.x[0], p.inv_deg, nhub,
                      (float)omega, false};
-        if (tid == 0) p.st->moved[(k + 1) % 3] = 0;
+        if (tid == 0) {
+            p.st->moved[(k + 1) % 3] = 0;
+            p.st->unit[(k + 1) % 3] = 0;
+        }
         for (unsigned i = threadIdx.x * 4; i < nhub; i += kPullBlock * 4) {
             const float4 v = __ldcg(reinterpret_cast<const float4 *>(y + i));  // y holds a multiple of 4
             if (i + 4 <= nhub) {
@@ -565,19 +618,34 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
             }
             dealt = (dealt + s_t.rows[c]) % gridDim.x;
         }
-        dealt = 0;
-        for (; c < s_t.n; c++) {
+        const auto rows_of = [&](unsigned k0, unsigned k1, unsigned step) {  // chunks of class c
             const uint32_t q = s_t.quads[c], rows = s_t.rows[c], first = s_t.first[c];
             const uint4 *e = p.quads + s_t.quad0[c];
-            const unsigned s = pull_lanes(q), per = 32 / s, chunks = (rows + per - 1) / per;
-            const unsigned k0 = (gwarp + nwarps - dealt) % nwarps;
-            if (q > 64) pull_long_rows(sw, first, rows, q, e, k0, nwarps, lane);
-            else if (s == 16) pull_rows<16, 1>(sw, first, rows, q, e, k0, nwarps, lane);
-            else if (s == 8) pull_rows<8, 1>(sw, first, rows, q, e, k0, nwarps, lane);
-            else if (s == 4) pull_rows<4, 2>(sw, first, rows, q, e, k0, nwarps, lane);
-            else if (s == 2) pull_rows<2, 4>(sw, first, rows, q, e, k0, nwarps, lane);
-            else pull_rows<1, 4>(sw, first, rows, q, e, k0, nwarps, lane);
-            dealt = (dealt + chunks) % nwarps;
+            const unsigned s = pull_lanes(q);
+            if (q > 64) pull_long_rows(sw, first, k0, k1, step, q, e, lane);
+            else if (s == 16) pull_rows<16, 1>(sw, first, rows, q, e, k0, k1, step, lane);
+            else if (s == 8) pull_rows<8, 1>(sw, first, rows, q, e, k0, k1, step, lane);
+            else if (s == 4) pull_rows<4, 2>(sw, first, rows, q, e, k0, k1, step, lane);
+            else if (s == 2) pull_rows<2, 4>(sw, first, rows, q, e, k0, k1, step, lane);
+            else pull_rows<1, 4>(sw, first, rows, q, e, k0, k1, step, lane);
+        };
+        if (skewed) {
+            for (unsigned unit = gwarp; unit < s_u.total;) {
+                while (c + 1 < s_t.n && unit >= s_u.first[c + 1]) c++;
+                const unsigned size = s_u.chunks[c], k0 = (unit - s_u.first[c]) * size;
+                rows_of(k0, min(pull_chunks(s_t.quads[c], s_t.rows[c]), k0 + size), 1);
+                if (s_u.total <= nwarps) break;
+                unsigned next = 0;
+                if (lane == 0) next = nwarps + atomicAdd(&p.st->unit[k % 3], 1u);
+                unit = __shfl_sync(kFull, next, 0);
+            }
+        } else {
+            dealt = 0;
+            for (; c < s_t.n; c++) {
+                const unsigned chunks = pull_chunks(s_t.quads[c], s_t.rows[c]);
+                rows_of((gwarp + nwarps - dealt) % nwarps, chunks, nwarps);
+                dealt = (dealt + chunks) % nwarps;
+            }
         }
         if (__any_sync(kFull, sw.moved) && lane == 0) *(volatile unsigned *)&p.st->moved[k % 3] = 1;
         if (!gs.sync()) return;
