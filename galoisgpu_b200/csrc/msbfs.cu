@@ -24,12 +24,15 @@
 //             ones together.  Uses v's out-edges as its in-edges, so it
 //             requires a symmetric graph (flag GFT_MSBFS_SYMMETRIC); without
 //             the flag every level runs top-down.
-// In either direction a vertex of kHubDegree edges or more goes to a hub list,
-// whose edges all warps of the grid then take in kHubEdges-edge chunks: with
-// one warp per vertex most of a level was the grid waiting for the largest
-// ones (256 sources on RMAT-20, levels of eight sources read back: 4.79 ->
-// 1.52 ms, with the frontier rows reduced by one instruction per word
-// instead of five shuffles, and the source set-up by a CTA instead of a thread).
+// A vertex of kHubDegree edges or more is a hub, whose edges all warps of the
+// grid take in kHubEdges-edge chunks: with one warp per vertex most of a level
+// was the grid waiting for the largest ones (256 sources on RMAT-20, levels
+// of eight sources read back: 4.79 -> 1.50 ms, with the frontier rows reduced
+// by one instruction per word instead of five shuffles, and the source set-up
+// by a CTA instead of a thread).  Top-down, a hub stands on a list from the
+// moment it joins the frontier, so its chunks are expanded beside the other
+// vertices.  Bottom-up, the level itself finds the hubs that lack sources and
+// scans them after one more barrier.
 #include <string.h>
 
 #include <algorithm>
@@ -43,6 +46,12 @@ namespace dev {
 constexpr uint32_t kThreadDegree = 32;  // bottom-up: larger vertices are scanned by the whole warp
 constexpr uint32_t kHubDegree = 1024;   // either direction: larger vertices are scanned by the whole grid
 constexpr uint32_t kHubEdges = 512;     // edges of a hub per warp step
+// Bottom-up levels split hubs from this many sources on.  A hub that lacks few
+// sources finds them among its first edges, and the split costs a barrier per
+// level (RMAT-12, 14, 16, 18, 20 split / not, us: 8 sources 131/118, 157/134,
+// 170/170, 218/231, 312/261; 32 sources 137/122, 159/146, 186/190, 236/303,
+// 547/1001).
+constexpr uint32_t kSplitSources = 16;
 
 // A row of WP words of source bits.
 template <int WP>
@@ -119,8 +128,11 @@ struct MsParams {
     uint32_t *queue[2];        // frontier vertices per level
     uint32_t *touched;         // top-down: vertices given new bits
     uint32_t *tstamp;          // top-down: level + 1 at which v was last touched
-    uint2 *hubs;               // (vertex, first chunk) of the level's hubs
+    uint2 *hubs;               // bottom-up: (vertex, first chunk) of the level's hubs
+    uint2 *fhubs[2];           // the same of the frontier's hubs, by level
     uint32_t hub_cap;
+    uint32_t split_hubs;       // bottom-up: hubs are scanned by the whole grid
+    uint32_t max_share;        // top-down: warps that at most share a frontier vertex
     uint32_t symmetric;
     uint32_t alpha;            // bottom-up when m_f * alpha > nedges
     TraversalCtl *ctl;
@@ -200,38 +212,72 @@ __device__ __forceinline__ void warp_scatter(const MsParams &p, const Bits<WP> &
     }
 }
 
-// Puts v on the level's hub list.
-__device__ __forceinline__ void list_hub(const MsParams &p, unsigned long long *hub_ctr, uint32_t v, uint32_t deg)
+// Puts the v of the lanes with `is` on a hub list, with one reservation per
+// warp: a level of a skewed graph can list thousands.  Not inlined: its
+// registers would cost the levels spills.
+static __device__ __noinline__ void append_hubs(uint2 *hubs, uint32_t hub_cap, TraversalCtl *ctl,
+                                                unsigned long long *hub_ctr, bool is, uint32_t v, uint32_t deg,
+                                                unsigned lane)
 {
-    const unsigned nch = (deg + kHubEdges - 1) / kHubEdges;
-    const unsigned long long old = atomicAdd(hub_ctr, (1ull << 32) | nch);
-    const unsigned h = (unsigned)(old >> 32);
-    if (h < p.hub_cap) p.hubs[h] = make_uint2(v, (unsigned)old);
-    else raise_error(&p.ctl->error, &p.ctl->error_where, GFT_ERR_OVERFLOW, h);
+    const unsigned mask = __ballot_sync(kFull, is);
+    const unsigned nch = is ? (deg + kHubEdges - 1) / kHubEdges : 0u;
+    const unsigned incl = warp_incl_sum(nch, lane);
+    unsigned long long old = 0;
+    if (lane == 31) old = atomicAdd(hub_ctr, ((unsigned long long)__popc(mask) << 32) | incl);
+    old = __shfl_sync(kFull, old, 31);
+    const unsigned h = (unsigned)(old >> 32) + __popc(mask & lanemask_lt());
+    if (!is) return;
+    if (h < hub_cap) hubs[h] = make_uint2(v, (unsigned)old + incl - nch);
+    else raise_error(&ctl->error, &ctl->error_where, GFT_ERR_OVERFLOW, h);
 }
 
-// Calls f(vertex, first edge, end) for each chunk of the hub list, chunks
-// dealt to the grid's warps in turn.
+__device__ __forceinline__ void list_hubs(const MsParams &p, uint2 *hubs, unsigned long long *hub_ctr, bool is,
+                                          uint32_t v, uint32_t deg, unsigned lane)
+{
+    if (__any_sync(kFull, is)) append_hubs(hubs, p.hub_cap, p.ctl, hub_ctr, is, v, deg, lane);
+}
+
+// The grid's warps dealt to n items: `share` of them to each (at most
+// max_share) while the items are fewer than the warps.
+struct WarpShare {
+    unsigned share = 1, first, step, part = 0;
+    __device__ __forceinline__ WarpShare(unsigned max_share, unsigned n, unsigned gwarp, unsigned nwarps)
+        : first(gwarp), step(nwarps)
+    {
+        if (max_share == 1 || 2 * n > nwarps || n == 0) return;
+        share = min(max_share, nwarps / n);
+        first = gwarp / share;
+        step = nwarps / share;  // at least n: the warps left over have nothing
+        part = gwarp % share;
+    }
+};
+
+// Calls f(vertex, first edge, end, ws) for the chunks of a hub list that
+// `ws` deals to this warp.
 template <class F>
-__device__ __forceinline__ void for_hub_chunks(const MsParams &p, unsigned long long hv, unsigned gwarp,
-                                               unsigned nwarps, F &&f)
+__device__ __forceinline__ void for_hub_chunks(const MsParams &p, const uint2 *hubs, unsigned long long hv,
+                                               const WarpShare &ws, F &&f)
 {
     const unsigned nh = (unsigned)(hv >> 32), nc = (unsigned)hv;
-    for (unsigned c = gwarp; c < nc; c += nwarps) {
+    for (unsigned c = ws.first; c < nc; c += ws.step) {
         unsigned lo = 0, hi = nh;
         while (hi - lo > 1) {
             const unsigned mid = (lo + hi) >> 1;
-            if (__ldcg(&p.hubs[mid].y) <= c) lo = mid;
+            if (__ldcg(&hubs[mid].y) <= c) lo = mid;
             else hi = mid;
         }
-        const uint2 hb = __ldcg(p.hubs + lo);
+        const uint2 hb = __ldcg(hubs + lo);
         const uint32_t s = __ldg(p.row_start + hb.x), e = __ldg(p.row_start + hb.x + 1);
         const uint32_t at = s + (c - hb.y) * kHubEdges;
-        f(hb.x, at, min(e, at + kHubEdges));
+        f(hb.x, at, min(e, at + kHubEdges), ws);
     }
 }
 
-template <int WP>
+// kHubs: some vertex has kHubDegree edges or more.  Without, a level has no
+// hub step: with one in every level, road 512^2 took 1.62 ms instead of 1.20
+// and grid 256^2 5.32 instead of 3.89 (one source; part of it frontiers of a
+// few vertices shared by every warp of the grid, see max_share).
+template <int WP, bool kHubs>
 __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
 {
     constexpr int BLOCK = 512;
@@ -278,6 +324,8 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                 mf = p.row_start[s + 1] - p.row_start[s];
             }
         }
+        if (kHubs)
+            list_hubs(p, p.fhubs[0], &ctl->hub_claim[0].v, mf >= kHubDegree, s_src[i % 256], (uint32_t)mf, lane);
         warp_add_u64(&ctl->hub[0].v, mf, lane);
         __syncthreads();
         if (i == 0) *u32_of(ctl->qlen[0]) = s_n;
@@ -300,8 +348,12 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
             *u32_of(ctl->claim[rslot]) = 0;
             ctl->hub[rslot].v = 0;
             ctl->handoff[rslot].v = 0;
+            ctl->hub_claim[rslot].v = 0;
         }
-        unsigned long long *hub_ctr = &ctl->handoff[slot].v;  // (hubs << 32) | chunks of this level
+        // (hubs << 32) | chunks: those a bottom-up level finds, and those of
+        // the next frontier.
+        unsigned long long *hub_ctr = &ctl->handoff[slot].v, *fhub_next = &ctl->hub_claim[nslot].v;
+        uint2 *fhubs_next = (L & 1) ? p.fhubs[0] : p.fhubs[1];
         const uint32_t *F = p.planes + (size_t)L * plane_words;
         uint32_t *Fn = p.planes + (size_t)(L + 1) * plane_words;
         nq.queue = ((L + 1) & 1) ? p.queue[1] : p.queue[0];  // no dynamic index: keeps p out of local memory
@@ -327,10 +379,11 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                         e = __ldg(p.row_start + v + 1);
                     }
                 }
-                const bool hub = e - s >= kHubDegree;
-                if (hub) {  // its row is written after the hub phase
-                    list_hub(p, hub_ctr, v, e - s);
-                    e = s;
+                bool hub = false;
+                if (kHubs && p.split_hubs) {  // a hub's row is written after the hub phase
+                    hub = e - s >= kHubDegree;
+                    list_hubs(p, p.hubs, hub_ctr, hub, v, e - s, lane);
+                    if (hub) e = s;
                 }
                 const bool heavy = e - s > kThreadDegree;
                 if (!heavy) {  // this thread's own vertex, kStep edges at a time
@@ -371,12 +424,18 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                         my_mf += e - s;
                     }
                 }
+                if (kHubs && !p.split_hubs)
+                    list_hubs(p, fhubs_next, fhub_next, got && e - s >= kHubDegree, v, e - s, lane);
                 nq.push(got, v, lane);
             }
-            if (!gs.sync()) return;
-            const unsigned long long hv = ld_relaxed_u64(hub_ctr);
+            unsigned long long hv = 0;
+            if (kHubs && p.split_hubs) {
+                if (!gs.sync()) return;
+                hv = ld_relaxed_u64(hub_ctr);
+            }
             if (hv) {
-                for_hub_chunks(p, hv, gwarp, nwarps, [&](uint32_t v, uint32_t s, uint32_t e) {
+                const WarpShare ws(1, (unsigned)hv, gwarp, nwarps);
+                for_hub_chunks(p, p.hubs, hv, ws, [&](uint32_t v, uint32_t s, uint32_t e, const WarpShare &) {
                     const Bits<WP> sv = ld_row<WP>(p.seen, v);
                     Bits<WP> need;
 #pragma unroll
@@ -390,7 +449,7 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                 const unsigned nh = (unsigned)(hv >> 32);
                 for (unsigned b = gwarp * 32; b < nh; b += nwarps * 32) {  // warp-uniform trip count
                     bool got = false;
-                    uint32_t v = 0;
+                    uint32_t v = 0, deg = 0;
                     if (b + lane < nh) {
                         v = __ldcg(&p.hubs[b + lane].x);
                         const Bits<WP> nb = ld_row<WP>(p.next, v);  // the sources it lacked
@@ -403,9 +462,11 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
 #pragma unroll
                             for (int i = 0; i < WP; i++) sv.w[i] |= nb.w[i];
                             st_row<WP>(p.seen, v, sv);
-                            my_mf += __ldg(p.row_start + v + 1) - __ldg(p.row_start + v);
+                            deg = __ldg(p.row_start + v + 1) - __ldg(p.row_start + v);
+                            my_mf += deg;
                         }
                     }
+                    list_hubs(p, fhubs_next, fhub_next, got, v, deg, lane);
                     nq.push(got, v, lane);
                 }
             }
@@ -415,28 +476,30 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
             if (!gs.sync()) return;
             const uint32_t *q = (L & 1) ? p.queue[1] : p.queue[0];
             // A frontier of fewer vertices than warps gives each vertex
-            // several warps.
-            const unsigned share = max(1u, nwarps / nf);
-            for (uint32_t qi = gwarp / share; qi < nf; qi += nwarps / share) {
+            // several warps, up to one per 32 edges.
+            const WarpShare ws(p.max_share, nf, gwarp, nwarps);
+            for (uint32_t qi = ws.first; qi < nf; qi += ws.step) {
                 const uint32_t u = __ldcg(q + qi);
                 const uint32_t s = __ldg(p.row_start + u), e = __ldg(p.row_start + u + 1);
-                if ((e - s) / kHubDegree >= share) {
-                    if (lane == 0 && gwarp % share == 0) list_hub(p, hub_ctr, u, e - s);
-                    continue;
-                }
-                warp_scatter<WP>(p, ld_row<WP>(F, u), s + gwarp % share * 32, e, 32 * share, L + 1, tq, lane);
+                if (kHubs && e - s >= kHubDegree) continue;  // on the list
+                warp_scatter<WP>(p, ld_row<WP>(F, u), s + ws.part * 32, e, 32 * ws.share, L + 1, tq, lane);
             }
-            if (!gs.sync()) return;
-            for_hub_chunks(p, ld_relaxed_u64(hub_ctr), gwarp, nwarps, [&](uint32_t u, uint32_t s, uint32_t e) {
-                warp_scatter<WP>(p, ld_row<WP>(F, u), s, e, 32, L + 1, tq, lane);
-            });
+            if (kHubs) {
+                const unsigned long long hv = ld_relaxed_u64(&ctl->hub_claim[slot].v);
+                for_hub_chunks(p, (L & 1) ? p.fhubs[1] : p.fhubs[0], hv,
+                               WarpShare(kHubEdges / 32, (unsigned)hv, nwarps - 1 - gwarp, nwarps),
+                               [&](uint32_t u, uint32_t s, uint32_t e, const WarpShare &w) {
+                                   warp_scatter<WP>(p, ld_row<WP>(F, u), s + w.part * 32, e, 32 * w.share, L + 1, tq,
+                                                    lane);
+                               });
+            }
             tq.flush(lane);
             if (!gs.sync()) return;
             const uint32_t nt = ld_relaxed_u32(u32_of(ctl->claim[slot]));
             for (uint32_t b = gwarp * 32; b < nt; b += nwarps * 32) {  // warp-uniform trip count
                 const uint32_t ti = b + lane;
                 bool got = false;
-                uint32_t v = 0;
+                uint32_t v = 0, deg = 0;
                 if (ti < nt) {
                     v = __ldcg(p.touched + ti);
                     Bits<WP> nb = ld_row<WP>(p.next, v);
@@ -453,9 +516,11 @@ __global__ void __launch_bounds__(512, 2) msbfs_kernel(MsParams p)
                         for (int w = 0; w < WP; w++) s2.w[w] = sv.w[w] | nb.w[w];
                         st_row<WP>(p.seen, v, s2);
                         got = true;
-                        my_mf += p.row_start[v + 1] - p.row_start[v];
+                        deg = p.row_start[v + 1] - p.row_start[v];
+                        my_mf += deg;
                     }
                 }
+                if (kHubs) list_hubs(p, fhubs_next, fhub_next, got && deg >= kHubDegree, v, deg, lane);
                 nq.push(got, v, lane);
             }
         }
@@ -502,13 +567,14 @@ uint32_t row_words(uint32_t k)
     return w <= 1 ? 1 : w <= 2 ? 2 : w <= 4 ? 4 : 8;
 }
 
+template <bool kHubs>
 const void *msbfs_kernel_for(uint32_t wp)
 {
     switch (wp) {
-    case 1: return (const void *)dev::msbfs_kernel<1>;
-    case 2: return (const void *)dev::msbfs_kernel<2>;
-    case 4: return (const void *)dev::msbfs_kernel<4>;
-    case 8: return (const void *)dev::msbfs_kernel<8>;
+    case 1: return (const void *)dev::msbfs_kernel<1, kHubs>;
+    case 2: return (const void *)dev::msbfs_kernel<2, kHubs>;
+    case 4: return (const void *)dev::msbfs_kernel<4, kHubs>;
+    case 8: return (const void *)dev::msbfs_kernel<8, kHubs>;
     }
     return nullptr;
 }
@@ -550,10 +616,12 @@ gft_status gft_msbfs(gft_engine *e, const gft_graph *g, const uint32_t *h_source
                  o_q1 = take((size_t)G.nnodes * 4), o_t = take((size_t)G.nnodes * 4),
                  o_ts = take((size_t)G.nnodes * 4), o_src = take((size_t)k * 4);
     const uint32_t hub_cap = G.nedges / dev::kHubDegree + 1;
-    const size_t o_hubs = take((size_t)hub_cap * sizeof(uint2));
+    const size_t o_hubs = take((size_t)hub_cap * sizeof(uint2)), o_fhubs0 = take((size_t)hub_cap * sizeof(uint2)),
+                 o_fhubs1 = take((size_t)hub_cap * sizeof(uint2));
     GFT_TRY(e->scratch.ensure(off));
     char *base = static_cast<char *>(e->scratch.ptr);
-    const void *kern = msbfs_kernel_for(WP);
+    const bool hubs = G.max_degree >= dev::kHubDegree;
+    const void *kern = hubs ? msbfs_kernel_for<true>(WP) : msbfs_kernel_for<false>(WP);
     LaunchShape shape;
     GFT_TRY(resolve_shape(e, kern, 512, 2, 0, &shape));
     dev::MsParams p{};
@@ -572,7 +640,13 @@ gft_status gft_msbfs(gft_engine *e, const gft_graph *g, const uint32_t *h_source
     p.touched = reinterpret_cast<uint32_t *>(base + o_t);
     p.tstamp = reinterpret_cast<uint32_t *>(base + o_ts);
     p.hubs = reinterpret_cast<uint2 *>(base + o_hubs);
+    p.fhubs[0] = reinterpret_cast<uint2 *>(base + o_fhubs0);
+    p.fhubs[1] = reinterpret_cast<uint2 *>(base + o_fhubs1);
     p.hub_cap = hub_cap;
+    p.split_hubs = k >= dev::kSplitSources;
+    // More warps than a vertex has 32-edge steps would all read its queue
+    // entry, row and plane row from L2 for nothing.
+    p.max_share = std::max(1u, (std::min(G.max_degree, dev::kHubDegree) + 31) / 32);
     p.symmetric = (flags & GFT_MSBFS_SYMMETRIC) ? 1u : 0u;
     // Bottom-up once the frontier's edges exceed 1/64 of the graph's: a
     // bottom-up level checks a vertex's rows only until its sources are

@@ -86,3 +86,29 @@ def test_msbfs_hub_phase(gft, orc, engine, k, symmetric):
     r = engine.msbfs(dg, srcs, max_levels=2100, symmetric=symmetric)
     for i in {0, 1, 2, k // 2, k - 1}:
         np.testing.assert_array_equal(r["levels_of"](i).cpu().numpy(), orc.bfs(rs, g.edge_dst, srcs[i]))
+
+
+@pytest.mark.parametrize("degree", [2, 1023, 1024, 3000])
+@pytest.mark.parametrize("k", [1, 15, 16, 70])
+def test_msbfs_top_down_level_takes_three_barriers(gft, orc, engine, degree, k):
+    """A path of 300 vertices with leaves on two of them, without hubs, just
+    below and at a hub's size and above: a hub on the frontier costs no
+    barrier beyond the three of a top-down level, nor does a graph without."""
+    n, leaves = 300, degree - 2
+    pairs = [(i, i + 1) for i in range(n - 1)] + [(v, n + j + leaves * w) for w, v in enumerate((5, 150))
+                                                  for j in range(leaves)]
+    a = np.array(pairs)
+    src, dst = np.concatenate([a[:, 0], a[:, 1]]), np.concatenate([a[:, 1], a[:, 0]])
+    order = np.argsort(src, kind="stable")
+    total = n + 2 * leaves
+    rs = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=total))]).astype(np.uint32)
+    g = gft.CSRGraph(rs, dst[order].astype(np.uint32))
+    assert int(np.diff(rs.astype(np.int64)).max()) == degree
+    dg = g.copy_to_gpu()
+    srcs = [int(x) for x in np.random.default_rng(k).integers(0, n, size=k)]
+    for symmetric in (False, True):
+        r = engine.msbfs(dg, srcs, max_levels=310, symmetric=symmetric)
+        if not symmetric:  # two before the first level
+            assert r["iterations"] <= 3 * r["levels"] + 2
+        for i in {0, k // 2, k - 1}:
+            np.testing.assert_array_equal(r["levels_of"](i).cpu().numpy(), orc.bfs(rs, g.edge_dst, srcs[i]))
