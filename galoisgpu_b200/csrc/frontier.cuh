@@ -126,20 +126,19 @@ __device__ __forceinline__ uint32_t ld_bits(const uint32_t *p)
         return __ldcg(p);
 }
 
-// First look at a vertex's bit: through L1 in global memory.  Bits are only
-// ever set during a traversal, so a set bit is final however old the line is,
-// and most edges of a large level lead to visited vertices; a clear one is
-// looked up again in L2 before the claim (RMAT-21 top-down: 630 -> 591 us).
-template <bool kLocalBits>
+// First look at a vertex's bit, with kL1 through L1.  Bits are only ever set
+// during a traversal, so a set bit is final however old the line is; a clear
+// one is looked up again in L2 before the claim.  It pays where most edges lead
+// to visited vertices (RMAT-21 top-down: 630 -> 591 us), and costs a second
+// read where they do not (road 2048^2: 1.46 -> 1.52 ms).
+template <bool kLocalBits, bool kL1>
 __device__ __forceinline__ uint32_t probe_bits(const uint32_t *p)
 {
-    if constexpr (kLocalBits)
-        return *(const volatile uint32_t *)p;
-    else
-        return __ldca(p);
+    if constexpr (kL1 && !kLocalBits) return __ldca(p);
+    else return ld_bits<kLocalBits>(p);
 }
 
-template <bool kLocalBits = false, unsigned kQB = kQueueBuf>
+template <bool kLocalBits = false, unsigned kQB = kQueueBuf, bool kL1 = false>
 struct BfsVisitorT {
     static constexpr int kBatch = GFT_BFS_BATCH;  // edges per lane in one flattened step
     static constexpr bool kEarlyRow = false;      // owner() loads nothing
@@ -172,8 +171,8 @@ struct BfsVisitorT {
     {
         uint32_t word[K];
 #pragma unroll
-        for (int k = 0; k < K; k++) word[k] = valid[k] ? probe_bits<kLocalBits>(visited + (dst[k] >> 5)) : 0xFFFFFFFFu;
-        if constexpr (!kLocalBits) {
+        for (int k = 0; k < K; k++) word[k] = valid[k] ? probe_bits<kLocalBits, kL1>(visited + (dst[k] >> 5)) : 0xFFFFFFFFu;
+        if constexpr (kL1 && !kLocalBits) {
 #pragma unroll
             for (int k = 0; k < K; k++)
                 if (!(word[k] & (1u << (dst[k] & 31)))) word[k] = __ldcg(visited + (dst[k] >> 5));
@@ -567,8 +566,8 @@ __device__ __forceinline__ unsigned pick_grain(unsigned n, unsigned nwarps, bool
 // one CTA with its bitmap in shared memory) a probe reads the level and the
 // bitmap is updated in place: next == bits.  Claimed vertices are also
 // queued, so a top-down level can follow.
-template <bool kTwo, bool kLocalBits, unsigned kQB>
-__device__ __forceinline__ void bottom_up_level(BfsVisitorT<kLocalBits, kQB> &vis, const TravParams &p, unsigned L,
+template <bool kTwo, bool kLocalBits, unsigned kQB, bool kL1>
+__device__ __forceinline__ void bottom_up_level(BfsVisitorT<kLocalBits, kQB, kL1> &vis, const TravParams &p, unsigned L,
                                                 const uint32_t *bits, uint32_t *next, unsigned gwarp, unsigned nwarps,
                                                 unsigned lane)
 {
@@ -665,11 +664,11 @@ constexpr unsigned kAlpha = 14, kBeta = 24, kScan = 32;
 
 // kLocalBits: p.visited points to shared memory (one CTA runs the traversal).
 // warp_buf: this warp's kQB-entry push buffer.
-// kTwo: bottom-up levels use the second bitmap p.visited2.
-template <class Mode, bool kLocalBits = false, unsigned kQB = kQueueBuf, bool kTwo = false>
+// kTwo: bottom-up levels use the second bitmap p.visited2.  kL1: see probe_bits.
+template <class Mode, bool kLocalBits = false, unsigned kQB = kQueueBuf, bool kTwo = false, bool kL1 = false>
 __device__ __forceinline__ void bfs_body(const TravParams &p, Mode &m, uint32_t *warp_buf)
 {
-    using Vis = BfsVisitorT<kLocalBits, kQB>;
+    using Vis = BfsVisitorT<kLocalBits, kQB, kL1>;
     TraversalCtl *ctl = m.ctl;
     const unsigned lane = threadIdx.x & 31;
     const unsigned tid = m.tid, nthreads = m.nthreads, nwarps = m.nwarps, gwarp = m.gwarp;

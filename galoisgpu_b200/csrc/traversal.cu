@@ -42,7 +42,8 @@ constexpr int kCtaBlock = 1024;  // threads of the single-CTA kernels
 // most 32 KB per CTA), as the grid-wide SSSP kernel.
 constexpr unsigned kBfsGridQueueBuf = 256;
 
-template <int BLOCK, unsigned QB>
+// kTwo, kL1: see bfs_body; picked by bfs_kernel_for.
+template <int BLOCK, unsigned QB, bool kTwo, bool kL1>
 // Resident threads per SM the grid BFS kernel's register budget is set for:
 // 2048 (32 registers a thread, 42 bytes spilled).  A 64-register build
 // (1024, no spills) was slower on RMAT-24 BFS: best 0.89 ms against 0.70 ms
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(BLOCK, GFT_BFS_THREADS_PER_SM / BLOCK) bfs_per
     const unsigned tid = blockIdx.x * BLOCK + threadIdx.x, nthreads = gridDim.x * BLOCK;
     GridMode m{{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, gridDim.x, 0, p.timeout_ns},
                ctl, tid, nthreads, tid / 32, nthreads / 32};
-    bfs_body<GridMode, false, QB, true>(p, m, s_buf[threadIdx.x >> 5]);
+    bfs_body<GridMode, false, QB, kTwo, kL1>(p, m, s_buf[threadIdx.x >> 5]);
 }
 
 // Default push buffers of the grid-wide SSSP kernel: 256 entries per warp up
@@ -120,9 +121,9 @@ __global__ void __launch_bounds__(kCtaBlock, 1) bfs_single_cta(TravParams p)
     __syncthreads();
     TraversalCtl *gctl = p.ctl;
     p.ctl = &s_ctl;
-    if (kLocalBits) p.visited = s_bits, p.visited2 = nullptr;  // bfs_body clears the first (nnodes + 31) / 32 words
+    if (kLocalBits) p.visited = s_bits;  // bfs_body clears the first (nnodes + 31) / 32 words
     CtaMode m{&s_ctl, threadIdx.x, kCtaBlock, threadIdx.x >> 5, kCtaBlock / 32, 0};
-    bfs_body<CtaMode, kLocalBits>(p, m, s_buf[threadIdx.x >> 5]);
+    bfs_body<CtaMode, kLocalBits, kQueueBuf, false, true>(p, m, s_buf[threadIdx.x >> 5]);
     __syncthreads();
     if (threadIdx.x == 0) publish_cta_result(s_ctl, gctl);
 }
@@ -664,25 +665,43 @@ constexpr uint32_t kDefaultCtaSmall = 256;
 constexpr uint32_t kDefaultFuse = 256;
 
 template <int BLOCK>
-const void *bfs_kernel_tile(uint32_t tile)
+const void *bfs_kernel_tile(uint32_t tile, bool l1, bool dir_opt)
 {
     switch (tile) {
-    case 64: return (const void *)dev::bfs_persistent<BLOCK, 64>;
-    case 128: return (const void *)dev::bfs_persistent<BLOCK, 128>;
-    case 256: return (const void *)dev::bfs_persistent<BLOCK, 256>;
+    case 64: return (const void *)dev::bfs_persistent<BLOCK, 64, true, true>;
+    case 128: return (const void *)dev::bfs_persistent<BLOCK, 128, true, true>;
+    case 256:
+        return l1        ? (const void *)dev::bfs_persistent<BLOCK, 256, true, true>
+               : dir_opt ? (const void *)dev::bfs_persistent<BLOCK, 256, true, false>
+                         : (const void *)dev::bfs_persistent<BLOCK, 256, false, false>;
     }
     return nullptr;
 }
 
+// Graphs whose edges mostly lead to vertices that are visited already, where
+// the grid-wide BFS looks through L1 first: skewed ones, and from about 12
+// edges a vertex on.  Elsewhere the second read, and the registers that it
+// and the second bitmap take in the main loop, cost more than they save
+// (both / second bitmap / neither, us): road 2048^2 1520 / 1461 / 1427,
+// 8-neighbour mesh 1000^2 5627 / 5450 / 5372, random of degree 8, 2^22
+// vertices 462 / 438 / 424, but of degree 16, 2^18 vertices 142 / 164 / 158;
+// with bottom-up levels, degree 6, 2^20: 181 / 185 / 194, degree 8: 305 / 298 /
+// 318.
+bool bfs_probes_l1(const DeviceGraph &G)
+{
+    return G.max_degree > kUniformDegree || G.nedges >= 12ull * G.nnodes;
+}
+
 // Grid-wide BFS kernel for a CTA size and queue tile (0: the default tile);
-// NULL for a combination that is not built.
-const void *bfs_kernel_for(int block, uint32_t tile)
+// NULL for a combination that is not built.  dir_opt: levels may run
+// bottom-up.  Tiles other than the default are built once.
+const void *bfs_kernel_for(int block, uint32_t tile, bool l1, bool dir_opt)
 {
     if (!tile) tile = dev::kBfsGridQueueBuf;
     switch (block) {
-    case 256: return bfs_kernel_tile<256>(tile);
-    case 512: return bfs_kernel_tile<512>(tile);
-    case 1024: return bfs_kernel_tile<1024>(tile);
+    case 256: return bfs_kernel_tile<256>(tile, l1, dir_opt);
+    case 512: return bfs_kernel_tile<512>(tile, l1, dir_opt);
+    case 1024: return bfs_kernel_tile<1024>(tile, l1, dir_opt);
     }
     return nullptr;
 }
@@ -792,7 +811,9 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     if (is_sssp && G.edge_data && !G.edge_dw && !G.wrapped)
         GFT_TRY(ensure_edge_pairs(const_cast<gft_graph *>(g), stream));
     Tune t = resolve_tuning(tune, is_sssp);
-    const void *kern = is_sssp ? sssp_kernel_for(t.block, t.tile) : bfs_kernel_for(t.block, t.tile);
+    const bool dir_opt = !is_sssp && G.symmetric && t.direction == 0;
+    const void *kern = is_sssp ? sssp_kernel_for(t.block, t.tile)
+                               : bfs_kernel_for(t.block, t.tile, bfs_probes_l1(G), dir_opt);
     if (!kern)
         return fail(GFT_ERR_INVALID_ARG,
                     "%s: block_threads must be 256, 512 or 1024 and queue_tile 0, 64, 128 or 256 "
@@ -910,7 +931,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     p.skip_block = t.skip;
     p.vec_ok = ((uintptr_t)G.edge_dst % 16 == 0) && (!G.edge_data || (uintptr_t)G.edge_data % 16 == 0);
     p.nedges = G.nedges;
-    p.dir_opt = !is_sssp && G.symmetric && t.direction == 0;
+    p.dir_opt = dir_opt;
     p.uniform = G.max_degree <= kUniformDegree;
     if (is_sssp && !single)
         p.cta_small = t.cta_small == UINT32_MAX ? 0 : t.cta_small ? t.cta_small : p.uniform ? kDefaultCtaSmall : 0;
@@ -1157,7 +1178,8 @@ extern "C" gft_status gft_bfs_noalloc(const gft_graph *g, uint32_t src, int32_t 
     char *base = nullptr;
     GFT_TRY(noalloc_scratch(G.device, &base));
 
-    const void *kern = (const void *)dev::bfs_persistent<kNoAllocBlock, dev::kBfsGridQueueBuf>;
+    const bool dir_opt = G.symmetric && !(tune && tune->direction != 0);
+    const void *kern = bfs_kernel_for(kNoAllocBlock, 0, bfs_probes_l1(G), dir_opt);
     int sms = 0, occ = 0;
     GFT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, G.device));
     GFT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kNoAllocBlock, 0));
@@ -1189,7 +1211,7 @@ extern "C" gft_status gft_bfs_noalloc(const gft_graph *g, uint32_t src, int32_t 
     // bitmap and queues above).
     p.nedges = G.nedges;
     p.uniform = G.max_degree <= kUniformDegree;
-    p.dir_opt = G.symmetric && !(tune && tune->direction != 0);
+    p.dir_opt = dir_opt;
 
     // The control block must start at zero for every call.
     GFT_CUDA_TRY(cudaMemsetAsync(p.ctl, 0, sizeof(TraversalCtl), stream));

@@ -572,3 +572,31 @@ def test_one_cta_bfs_either_side_of_the_staged_slots(gft, orc, engine, side):
         np.testing.assert_array_equal(got, want)
         assert orc.check_tree(g.row_start, g.edge_dst, None, src, got, par) == 0
         assert r["levels"] == want.max() + 1 and r["vertices_reached"] == g.nnodes - 1
+
+
+@pytest.mark.parametrize("degree", [4, 10, 12, 32])
+@pytest.mark.parametrize("marked", [False, True])
+def test_grid_bfs_kernels_by_degree(gft, orc, engine, degree, marked):
+    """The grid-wide BFS kernels on random graphs of one degree, below, at and
+    above 12 edges a vertex, whose large levels run bottom-up when the graph
+    is marked, and with a queue tile that has one kernel for all of them."""
+    n = 70_001
+    rng = np.random.default_rng(degree)
+    a = np.tile(np.arange(n), degree // 2)
+    b = np.concatenate([rng.permutation(n) for _ in range(degree // 2)])
+    src = np.concatenate([a, b])
+    order = np.argsort(src, kind="stable")
+    rs = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint32)
+    dst = np.concatenate([b, a])[order].astype(np.uint32)
+    assert int(np.diff(rs.astype(np.int64)).max()) == degree
+    dg = gft.CSRGraph(rs, dst).copy_to_gpu()
+    dg.symmetric = marked
+    for src in (0, n - 1):
+        want = orc.bfs(rs, dst, src)
+        for tune in ({"max_blocks": 1 << 30, "warp_degree": 32}, {"max_blocks": 1 << 30, "queue_tile": 128}):
+            got, par, r = _run_bfs(gft, engine, dg, src, tune)
+            np.testing.assert_array_equal(got, want)
+            assert orc.check_tree(rs, dst, None, src, got, par) == 0
+            if not marked:
+                reached = want != np.iinfo(np.int32).max
+                assert r["edges_scanned"] == int(np.diff(rs.astype(np.int64))[reached].sum())
