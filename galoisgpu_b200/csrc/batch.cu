@@ -10,9 +10,10 @@
 //            launch is cooperative whenever there are such queries, so a group
 //            is co-resident and its bounded barrier cannot wait on a CTA that
 //            never starts.  By default each query gets CTAs in proportion to
-//            its estimated work (plan_gangs); with group_blocks or
-//            group_min_nodes given, queries on graphs of at least
-//            group_min_nodes vertices run on groups of group_blocks CTAs;
+//            its estimated work (plan_gangs), or, in batches of many large
+//            queries, groups of one size take them in turn (kTurnGroup); with
+//            group_blocks or group_min_nodes given, queries on graphs of at
+//            least group_min_nodes vertices run on groups of group_blocks CTAs;
 //   phase 2: the rest run on ONE CTA each (CtaMode: control block in shared
 //            memory, __syncthreads as the barrier, no grid-wide atomics).
 // Both phases take queries from a device job table, largest first (longest
@@ -68,17 +69,25 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 
     // Phase 1: large jobs on CTA groups.
     const unsigned ngroups = gangs ? nbig : (nbig > 0 && group > 1) ? gridDim.x / group : 0;
-    unsigned g = blockIdx.x / max(group, 1u), rank = blockIdx.x % max(group, 1u);
-    if (gangs) {
-        const uint4 mine = gangs[blockIdx.x];
-        g = mine.x;
-        rank = mine.y;
-        group = mine.z;
+    // This CTA's group, its rank in it and the group's size stay in shared
+    // memory: kept in registers they are spilled inside the traversal loops (512
+    // queries, groups of 8: 75.2 -> 73.0 ms; 256 threads, groups of 16: 82.2 ->
+    // 78.9 ms).
+    __shared__ volatile unsigned s_gang[3];
+    if (threadIdx.x == 0) {
+        uint4 mine = make_uint4(blockIdx.x / max(group, 1u), blockIdx.x % max(group, 1u), group, 0);
+        if (gangs) mine = gangs[blockIdx.x];
+        s_gang[0] = mine.x;
+        s_gang[1] = mine.y;
+        s_gang[2] = mine.z;
     }
+    __syncthreads();
+    const unsigned g = s_gang[0];
+    volatile unsigned &rank = s_gang[1], &size = s_gang[2];
     if (g < ngroups) {
         TraversalCtl *ctl = gctl + g;
         bool first = true;
-        GridSync gs{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, group, 0, timeout_ns};
+        GridSync gs{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, size, 0, timeout_ns};
         for (;;) {
             if (rank == 0 && threadIdx.x == 0)
                 *u32_of(ctl->job) = !gangs ? atomicAdd(&cursors[1], 1u) : first ? g : nbig;
@@ -114,7 +123,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
             __syncthreads();
             const unsigned long long t0 = s_t0;
             const unsigned tid = rank * BLOCK + threadIdx.x;
-            GridMode m{gs, ctl, tid, group * BLOCK, tid / 32, group * BLOCK / 32};
+            GridMode m{gs, ctl, tid, size * BLOCK, tid / 32, size * BLOCK / 32};
             if (s_app == 1) sssp_body<GridMode, false, QB>(s_p, m, s_near[w], s_far[w]);
             else bfs_body<GridMode, false, QB>(s_p, m, s_near[w]);
             gs.epoch = m.gs.epoch;
@@ -254,6 +263,15 @@ double visits(const gft_query &x)
     return n + (skewed && G.symmetric ? 0.15 : skewed ? 1.0 : 1.5) * m;
 }
 
+// From three rounds of large queries on, groups of kTurnGroup CTAs take them in
+// turn instead of all of them running at once on their shares: the graphs in
+// work at a time then fit L2, and the last round's idle groups no longer count.
+// (The package's mixed batches, 512 threads a CTA, shares / groups of 16 / of
+// 8 from 2^18 vertices: 48 queries 10.0 / 16.4 / 30.6 ms, 128: 18.4 / 19.2 /
+// 35.0, 256: 47.4 / 36.0 / 51.1, 512: 87.0 / 63.4 / 73.0; 17, 46, 92 and 184 of
+// them large.)
+constexpr uint32_t kTurnGroup = 16, kTurnNodes = 1u << 17;
+
 // CTAs of each query, in proportion to its estimated visits: 1 = phase 2.
 // A query of the size that a single call runs on one CTA gets one here too,
 // and none gets more CTAs than keep 32768 visits each (a barrier of the group
@@ -381,7 +399,16 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
     b->blocks = std::max(1, std::min<int>(occ, (int)bps)) * e->sms;
     // Large queries (run on CTA groups) first, then the rest; each class
     // largest first.
-    const bool planned = !(tune && (tune->group_blocks || tune->group_min_nodes));
+    bool planned = !(tune && (tune->group_blocks || tune->group_min_nodes));
+    if (planned) {
+        uint64_t large = 0;
+        for (uint32_t i = 0; i < n; i++) large += q[i].graph->g.nnodes >= kTurnNodes;
+        if (large * kTurnGroup >= 3ull * b->blocks) {
+            planned = false;
+            b->group = kTurnGroup;
+            b->group_min_nodes = kTurnNodes;
+        }
+    }
     std::vector<uint32_t> ctas(n, 1);
     if (planned) plan_gangs(q, n, (uint32_t)b->blocks, ctas);
     auto big = [&](uint32_t i) {

@@ -13,11 +13,13 @@
 namespace gft {
 namespace dev {
 
-// Edges of a hub handled per warp claim.  The last chunks of a hub phase are
-// what the grid waits for, and a frontier of a few hubs has fewer chunks than
-// warps: 512 instead of 2048 took RMAT-24 BFS from 746 to 653 us, RMAT-21
-// top-down BFS from 675 to 627 us and RMAT-20 SSSP from 1785 to 1501 us.
-constexpr uint32_t kHubChunk = 512;
+// Edges of a hub handled per warp claim (a visitor's kHubChunk).  The last
+// chunks of a hub phase are what the grid waits for, and a frontier of a few
+// hubs has fewer chunks than warps: 512 instead of 2048 took RMAT-24 BFS from
+// 746 to 653 us, RMAT-21 top-down BFS from 675 to 627 us and RMAT-20 SSSP from
+// 1785 to 1501 us.  The few warps of a batched or served query only pay the
+// claims (512 queries, groups of 8: 77.4 ms with 512, 75.2 ms with 2048).
+constexpr uint32_t kGridHubChunk = 512, kGroupHubChunk = 2048;
 constexpr unsigned kInf = 0x7FFFFFFFu;
 
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) { return __ldcs(p); }
@@ -142,6 +144,7 @@ template <bool kLocalBits = false, unsigned kQB = kQueueBuf, bool kL1 = false>
 struct BfsVisitorT {
     static constexpr int kBatch = GFT_BFS_BATCH;  // edges per lane in one flattened step
     static constexpr bool kEarlyRow = false;      // owner() loads nothing
+    static constexpr uint32_t kHubChunk = kL1 ? kGridHubChunk : kGroupHubChunk;  // without kL1: no hubs, or a group
     const uint32_t *__restrict__ edge_dst;
     const uint32_t *__restrict__ row_start;  // non-NULL: sum the out-degrees of claimed vertices
     unsigned long long mf;                    // that sum, per lane
@@ -256,6 +259,7 @@ template <bool kSolo, unsigned kQB = kQueueBuf>
 struct SsspVisitorT {
     static constexpr int kBatch = GFT_SSSP_BATCH;  // edges per lane in one flattened step
     static constexpr bool kEarlyRow = kSolo;       // owner() loads the distance
+    static constexpr uint32_t kHubChunk = kSolo ? kGridHubChunk : kGroupHubChunk;
     static constexpr bool kFuse = kSolo;           // warps may expand the near vertices they found
     const uint32_t *__restrict__ edge_dst;
     const int32_t *__restrict__ edge_data;
@@ -469,7 +473,7 @@ __device__ __forceinline__ void expand_lanes(Vis &vis, const TravParams &p, bool
     }
     if (!(has && vis.active(o))) deg = 0;
     if (deg >= p.hub_degree) {
-        unsigned nch = (deg + kHubChunk - 1) / kHubChunk;
+        unsigned nch = (deg + Vis::kHubChunk - 1) / Vis::kHubChunk;
         unsigned long long old = atomicAdd(hub_ctr, (1ull << 32) | nch);
         unsigned h = (unsigned)(old >> 32);
         if (h < p.hub_cap) p.hubs[h] = make_uint2(v, (unsigned)old);
@@ -507,7 +511,7 @@ __device__ __forceinline__ void expand_frontier(Vis &vis, const TravParams &p, c
 }
 
 // Grid-wide processing of the hub list of one iteration: warps claim
-// kHubChunk-edge chunks; hub h owns chunks [hubs[h].y, hubs[h+1].y).
+// Vis::kHubChunk-edge chunks; hub h owns chunks [hubs[h].y, hubs[h+1].y).
 template <class Vis, class Own>
 __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsigned nh, unsigned nc,
                                             unsigned *hub_claim, unsigned gwarp, unsigned nwarps, unsigned lane)
@@ -526,8 +530,8 @@ __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsig
         if (!vis.active(o)) continue;  // warp uniform: every lane read the same hub
         const uint32_t start = __ldg(p.row_start + u);
         const uint32_t deg = __ldg(p.row_start + u + 1) - start;
-        const uint32_t off = (c - hb.y) * kHubChunk;
-        const uint32_t len = min(kHubChunk, deg - off);
+        const uint32_t off = (c - hb.y) * Vis::kHubChunk;
+        const uint32_t len = min(Vis::kHubChunk, deg - off);
         warp_range(vis, start + off, len, o, lane);
     }
 }

@@ -59,6 +59,7 @@ struct PrOwn {
 struct PrInitVisitor {
     static constexpr int kBatch = 2;
     static constexpr bool kEarlyRow = false;  // owner() reads only the degree
+    static constexpr uint32_t kHubChunk = kGridHubChunk;
     const uint32_t *__restrict__ row_start;
     const uint32_t *__restrict__ edge_dst;
     float *residual;
@@ -121,6 +122,7 @@ struct PrInitVisitor {
 struct PrVisitor {
     static constexpr int kBatch = 4;
     static constexpr bool kEarlyRow = true;  // owner() pops the residual
+    static constexpr uint32_t kHubChunk = kGridHubChunk;
     const uint32_t *__restrict__ row_start;
     const uint32_t *__restrict__ edge_dst;
     float *rank, *residual, *hub_upd;

@@ -107,3 +107,28 @@ def test_batch_shares_ctas_by_work(gft, orc, engine):
             assert q["status"] == 0
             np.testing.assert_array_equal(q["out"].cpu().numpy(), w)
     b.close()
+
+
+@pytest.mark.parametrize("n", [27, 28, 61])
+def test_batch_of_many_large_queries_takes_them_in_turn(gft, orc, engine, n):
+    """Queries on a graph of just over 2^17 vertices around the number (three
+    rounds of groups of 16 CTAs: 28 on 148 CTAs) from which groups take them
+    in turn, beside small ones."""
+    large, small = gft.CSRGraph.road(363, seed=51), gft.CSRGraph.road(40, seed=52)
+    assert large.nnodes >= 1 << 17
+    dl, ds = large.copy_to_gpu(), small.copy_to_gpu()
+    srcs = large.pick_sources(53, 4)
+    want = [orc.bfs(large.row_start, large.edge_dst, s) if i % 2 else
+            orc.sssp(large.row_start, large.edge_dst, large.edge_data, s) for i, s in enumerate(srcs)]
+    queries = [{"graph": dl, "app": "bfs" if i % 2 else "sssp", "src": srcs[i % 4], "delta": 20000} for i in range(n)]
+    queries += [{"graph": ds, "app": "sssp", "src": 0, "delta": 20000} for _ in range(5)]
+    want_small = orc.sssp(small.row_start, small.edge_dst, small.edge_data, 0)
+    b = gft.Batch(engine, queries, tune=gft.Tune(block_threads=1024, blocks_per_sm=1))
+    for rep in range(2):
+        for q in b.queries:
+            q["out"].fill_(-7)
+        b.run()
+        for i, q in enumerate(b.queries):
+            assert q["status"] == 0
+            np.testing.assert_array_equal(q["out"].cpu().numpy(), want[i % 4] if i < n else want_small)
+    b.close()
