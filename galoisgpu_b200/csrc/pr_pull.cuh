@@ -41,7 +41,9 @@
 // Launches, on the caller's stream, none of which the host waits for:
 //   pr_sample   looks for the reverse of a few hundred edges; a directed
 //               graph is given up at once (the host then runs the pushes)
-//   pr_classes  counts the rows of each class
+//   pr_classes  counts the rows of each class, and refuses a graph whose rows
+//               do not lie in its edges (a wrapped one can): the buffers are
+//               sized by its number of edges
 //   pr_place    numbers the vertices, class by class
 //   pr_relabel  writes the renumbered rows, and sums over all edges u->v a
 //               64-bit hash of {u, v}, added for u < v and subtracted for
@@ -69,7 +71,7 @@ constexpr float kPullEpsilon = 0.000001f;  // apps/pr/kernel.cu:20
 struct PullState {
     unsigned long long hash;  // pr_relabel's sum: 0 for a symmetric graph
     unsigned asymmetric;      // pr_sample found an edge without its reverse; pr_sweeps: the pushes have to run
-    unsigned outside;         // pr_relabel found an edge leaving the graph
+    unsigned outside;         // pr_classes found a row, or pr_relabel an edge, leaving the graph
     unsigned moved[3];        // per sweep, triple buffered: some residual or move was above EPSILON
     unsigned unit[3];         // per sweep, triple buffered: units claimed beyond every warp's first
     unsigned rows[kPullClasses];    // rows of each class
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(256) pr_sample(PullParams p)
     bool found = false;
     if (v < p.nnodes) {
         const uint32_t s = p.row_start[v], d = p.row_start[v + 1] - s;
-        found = d > kPullSampleScan;
+        found = d > kPullSampleScan || s > p.nedges || d > p.nedges - s;
         for (uint32_t i = lane; i < d && !found; i += 32) found = p.edge_dst[s + i] == lo;
     }
     if (!__any_sync(kFull, found) && lane == 0) p.st->asymmetric = 1;
@@ -162,16 +164,22 @@ __global__ void __launch_bounds__(1024) pr_classes(PullParams p)
     __syncthreads();
     const unsigned lane = threadIdx.x & 31;
     const uint32_t step = gridDim.x * blockDim.x;
+    bool outside = false;
     for (uint32_t v0 = blockIdx.x * blockDim.x + threadIdx.x - lane; v0 < p.nnodes; v0 += step) {  // warp uniform
         const uint32_t v = v0 + lane;
-        const unsigned c =
-            v < p.nnodes ? pull_class(pull_quads_of(p.row_start[v + 1] - p.row_start[v])) : kPullClasses;
+        unsigned c = kPullClasses;
+        if (v < p.nnodes) {
+            const uint32_t s = p.row_start[v], e = p.row_start[v + 1];
+            outside |= e < s || e > p.nedges;
+            c = pull_class(pull_quads_of(e - s));
+        }
         const unsigned peers = __match_any_sync(kFull, c);
         if (c < kPullClasses && lane == __ffs(peers) - 1) atomicAdd(&s_rows[c], __popc(peers));
     }
     __syncthreads();
     for (unsigned c = threadIdx.x; c < kPullClasses; c += blockDim.x)
         if (s_rows[c]) atomicAdd(&p.st->rows[c], s_rows[c]);
+    if (outside) p.st->outside = 1;
 }
 
 // First number of each class, largest rows first (class 0 stays unnumbered):
@@ -201,7 +209,7 @@ __device__ __forceinline__ void pull_class_firsts(const PullState *st, unsigned 
 __global__ void __launch_bounds__(1024) pr_place(PullParams p)
 {
     __shared__ unsigned s_first[kPullClasses], s_rows[kPullClasses], s_base[kPullClasses];
-    if (__ldcg(&p.st->asymmetric)) return;
+    if (__ldcg(&p.st->asymmetric) || __ldcg(&p.st->outside)) return;
     pull_class_firsts(p.st, s_first);
     constexpr int kPer = kPullTile / 1024;
     const unsigned lane = threadIdx.x & 31, lt = lanemask_lt();
@@ -321,7 +329,8 @@ __device__ __forceinline__ void pull_segments(const PullTable &t, unsigned gwarp
 __global__ void __launch_bounds__(512, 3) pr_relabel(PullParams p)
 {
     __shared__ PullTable s_t;
-    if (__ldcg(&p.st->asymmetric)) return;
+    // pr_classes' finding; one of this launch may already be seen, and ends it.
+    if (__syncthreads_or(__ldcg(&p.st->asymmetric) || __ldcg(&p.st->outside))) return;
     pull_table(p.st, s_t);
     const unsigned lane = threadIdx.x & 31;
     const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;

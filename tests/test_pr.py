@@ -220,3 +220,28 @@ def test_gpu_pr_pushes_on_graphs_that_are_not_symmetric(gft, orc, engine):
         r = engine.pr(dg)
         want, _ = orc.pr(graph.row_start, graph.edge_dst)
         assert close(r["out"].cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("claimed", [-6000, -1, 0, 100])
+def test_gpu_pr_wrapped_graph_with_a_wrong_edge_count(gft, engine, claimed):
+    """A wrapped symmetric graph whose edge count says fewer than its rows
+    hold (every row's edges are there): the sweeps, whose buffers are sized by
+    the count, leave it to the pushes.  With spare entries behind the edges,
+    and with the right count, the ranks are the same."""
+    import ctypes as C
+
+    import torch
+
+    g = gft.CSRGraph.grid(80, 80)
+    want = engine.pr(g.copy_to_gpu())["out"].cpu().numpy()
+    rs = torch.from_numpy(g.row_start.astype(np.int32)).cuda()
+    dst = torch.zeros(g.nedges + 128, dtype=torch.int32, device="cuda")
+    dst[: g.nedges] = torch.from_numpy(g.edge_dst.astype(np.int32))
+    h = C.c_void_p()
+    assert gft.load().gft_graph_wrap(0, g.nnodes, g.nedges + claimed, C.c_void_p(rs.data_ptr()),
+                                     C.c_void_p(dst.data_ptr()), None, C.byref(h)) == 0
+    r = engine.pr(gft.DeviceGraph(h, 0))
+    assert close(r["out"].cpu().numpy(), want)
+    swept = r["pushes"] == r["levels"] * g.nnodes
+    assert claimed > 0 or swept == (claimed == 0)
