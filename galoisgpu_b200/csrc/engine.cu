@@ -36,6 +36,23 @@ gft_status Scratch::ensure(size_t want)
     return GFT_OK;
 }
 
+bool Scratch::grow(size_t want)
+{
+    if (want <= bytes && ptr) return true;
+    size_t room = want, total = 0;
+    void *p = nullptr;
+    if (refused && cudaMemGetInfo(&room, &total) != cudaSuccess) room = 0;
+    refused = room < want || cudaMalloc(&p, want) != cudaSuccess;
+    if (refused) {
+        cudaGetLastError();
+        return false;
+    }
+    if (ptr) cudaFree(ptr);
+    ptr = p;
+    bytes = want;
+    return true;
+}
+
 void Scratch::release()
 {
     if (ptr) cudaFree(ptr);

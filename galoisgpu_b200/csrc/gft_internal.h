@@ -76,6 +76,10 @@ struct Scratch {
     void *ptr = nullptr;
     size_t bytes = 0;
     gft_status ensure(size_t want);
+    // The same for a workspace that a call can do without: false, with the
+    // present allocation kept, when device memory has no room for it.
+    bool grow(size_t want);
+    bool refused = false;  // the last grow found no room: the next one asks for the free bytes first
     void release();
 };
 

@@ -319,7 +319,10 @@ const void *pr_kernel_for(int block)
 
 // The pull path (pr_pull.cuh).  *done says whether it has written the ranks:
 // a graph that is not symmetric, or whose renumbered rows find no room in
-// device memory, is left to the pushes.
+// device memory, is left to the pushes.  The workspace is several times
+// theirs, so it is taken only when a sample of the edges has found their
+// reverses; an engine that already holds one as large does not wait for the
+// sample.
 gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t timeout_ms, cudaStream_t stream,
                     gft_stats *stats, bool *done)
 {
@@ -338,17 +341,30 @@ gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t
     const size_t vec = (n + 8) * 4;  // y holds a zero beside the n values
     const size_t o_st = take(sizeof(dev::PullState)), o_perm = take(vec), o_num = take(vec), o_inv = take(vec),
                  o_x0 = take(vec), o_x1 = take(vec), o_y0 = take(vec), o_y1 = take(vec), o_quads = take(quads * 16);
-    if (e->scratch.ensure(off) != GFT_OK) {
-        clear_error();
-        return GFT_OK;
-    }
-    char *base = static_cast<char *>(e->scratch.ptr);
     dev::PullParams p{};
     p.row_start = G.row_start;
     p.edge_dst = G.edge_dst;
     p.nnodes = G.nnodes;
     p.nedges = G.nedges;
     p.rank = d_rank;
+    p.ctl = reinterpret_cast<TraversalCtl *>(e->ctl.ptr);
+    p.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
+    TraversalCtl *h = reinterpret_cast<TraversalCtl *>(e->host_ctl);
+    unsigned asymmetric = 0;
+    const bool sample_first = e->scratch.bytes < off;
+    if (sample_first) {
+        GFT_TRY(e->scratch.ensure(sizeof(dev::PullState)));  // every other call needs more
+        p.st = static_cast<dev::PullState *>(e->scratch.ptr);
+        GFT_CUDA_TRY(cudaMemsetAsync(p.st, 0, sizeof(dev::PullState), stream));
+        dev::pr_sample<<<dev::kPullSamples / 8, 256, 0, stream>>>(p);
+        GFT_CUDA_TRY(cudaGetLastError());
+        GFT_CUDA_TRY(cudaMemcpyAsync(h, &p.st->asymmetric, sizeof asymmetric, cudaMemcpyDeviceToHost, stream));
+        GFT_CUDA_TRY(cudaStreamSynchronize(stream));
+        memcpy(&asymmetric, h, sizeof asymmetric);
+        if (asymmetric || !e->scratch.grow(off)) return GFT_OK;
+    }
+    char *base = static_cast<char *>(e->scratch.ptr);
+    p.st = reinterpret_cast<dev::PullState *>(base + o_st);
     p.perm = reinterpret_cast<uint32_t *>(base + o_perm);
     p.number = reinterpret_cast<uint32_t *>(base + o_num);
     p.inv_deg = reinterpret_cast<float *>(base + o_inv);
@@ -357,9 +373,6 @@ gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t
     p.y[0] = reinterpret_cast<float *>(base + o_y0);
     p.y[1] = reinterpret_cast<float *>(base + o_y1);
     p.quads = reinterpret_cast<uint4 *>(base + o_quads);
-    p.st = reinterpret_cast<dev::PullState *>(base + o_st);
-    p.ctl = reinterpret_cast<TraversalCtl *>(e->ctl.ptr);
-    p.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
     // A small graph's sweep is a few microseconds: CTAs without work only
     // lengthen its barrier.
     const int blocks = (int)std::min<uint64_t>(e->sms, (n + m / 4) / 2048 + 1);
@@ -369,8 +382,10 @@ gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t
     GFT_CUDA_TRY(cudaMemsetAsync(e->ctl.ptr, 0, sizeof(TraversalCtl), stream));
     GFT_CUDA_TRY(cudaMemsetAsync(p.st, 0, sizeof(dev::PullState), stream));
     GFT_CUDA_TRY(cudaEventRecord(e->ev0, stream));
-    dev::pr_sample<<<dev::kPullSamples / 8, 256, 0, stream>>>(p);
-    GFT_CUDA_TRY(cudaGetLastError());
+    if (!sample_first) {
+        dev::pr_sample<<<dev::kPullSamples / 8, 256, 0, stream>>>(p);
+        GFT_CUDA_TRY(cudaGetLastError());
+    }
     const int vblocks = (int)std::min<uint64_t>(2 * (uint64_t)e->sms, n / dev::kPullTile + 1);
     dev::pr_classes<<<vblocks, 1024, 0, stream>>>(p);
     GFT_CUDA_TRY(cudaGetLastError());
@@ -381,9 +396,7 @@ gft_status run_pull(gft_engine *e, const DeviceGraph &G, float *d_rank, uint32_t
     void *args[] = {&p};
     GFT_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(dev::kPullBlock), args, hub_bytes, stream));
     GFT_CUDA_TRY(cudaEventRecord(e->ev1, stream));
-    TraversalCtl *h = reinterpret_cast<TraversalCtl *>(e->host_ctl);
     const size_t cold = offsetof(TraversalCtl, error);
-    unsigned asymmetric = 0;
     GFT_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<char *>(h) + cold, reinterpret_cast<char *>(e->ctl.ptr) + cold,
                                  sizeof(TraversalCtl) - cold, cudaMemcpyDeviceToHost, stream));
     GFT_CUDA_TRY(cudaMemcpyAsync(h, &p.st->asymmetric, sizeof asymmetric, cudaMemcpyDeviceToHost, stream));

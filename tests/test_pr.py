@@ -245,3 +245,52 @@ def test_gpu_pr_wrapped_graph_with_a_wrong_edge_count(gft, engine, claimed):
     assert close(r["out"].cpu().numpy(), want)
     swept = r["pushes"] == r["levels"] * g.nnodes
     assert claimed > 0 or swept == (claimed == 0)
+
+
+@pytest.mark.gpu
+def test_gpu_pr_on_a_directed_graph_takes_no_sweep_workspace(gft):
+    """The pushes need 16 bytes a vertex and the hub list; the sweeps 28 and
+    4.5 to 18 an edge."""
+    rng = np.random.default_rng(7)
+    n, m = 30000, 600000
+    rs, ed = _csr(n, rng.integers(0, n, m), rng.integers(0, n, m))
+    e = gft.Engine(0)
+    try:
+        before = e.scratch_bytes()
+        e.pr(gft.CSRGraph(rs, ed).copy_to_gpu())
+        assert e.scratch_bytes() - before <= 16 * n + 8 * (m // 256 + 1) + 4096
+    finally:
+        e.close()
+
+
+@pytest.mark.gpu
+def test_gpu_pr_without_room_for_the_sweeps(gft, engine):
+    """With device memory all but full a symmetric graph takes the pushes, and
+    the engine keeps the scratch that it had."""
+    import torch
+
+    dg = gft.DeviceGraph.generate("rmat", seed=3, scale=20, edge_factor=16)  # sweeps: about 230 MB, pushes: 17 MB
+    want = engine.pr(dg)
+    assert want["edges_scanned"] == want["levels"] * dg.nedges  # swept
+    e = gft.Engine(0)
+    out = torch.empty(dg.nnodes, dtype=torch.float32, device="cuda")
+    e.sssp(dg)  # 20 bytes a vertex and more of scratch; the pushes need 16
+    e.pr(dg, out=out, max_iterations=2)  # the pushes' kernel is loaded
+    had = e.scratch_bytes()
+    assert had < 100 << 20
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (128 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        for _ in range(2):
+            r = e.pr(dg, out=out)
+            assert r["edges_scanned"] != r["levels"] * dg.nedges
+            assert e.scratch_bytes() == had
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    # The pushes' 32-bit sums: 7.6e-5 (2-norm) from the solution on RMAT-22.
+    a, b = r["out"].double(), want["out"].double()
+    assert float((a - b).norm() / b.norm()) <= 3e-4
+    r = e.pr(dg, out=out)
+    assert r["edges_scanned"] == r["levels"] * dg.nedges
+    e.close()
