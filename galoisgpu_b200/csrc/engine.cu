@@ -82,10 +82,10 @@ __global__ void first_bad_edge(const uint32_t *__restrict__ dst, uint32_t m, uin
 }
 
 __global__ void build_bfs_slots(const uint32_t *__restrict__ row_start, const uint32_t *__restrict__ dst, uint32_t n,
-                                uint4 *__restrict__ slots)
+                                uint32_t m, uint4 *__restrict__ slots)
 {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        slots[v] = bfs_slot_of(dst, row_start[v], row_start[v + 1], n);
+        slots[v] = bfs_slot_of(dst, row_start[v], row_start[v + 1], m, n);
 }
 
 __global__ void interleave_edges(const uint32_t *__restrict__ dst, const int32_t *__restrict__ w, uint32_t m,
@@ -135,7 +135,7 @@ gft_status ensure_bfs_slots(gft_graph *g, cudaStream_t stream)
         cudaGetLastError();  // no room: the BFS reads the CSR
         return GFT_OK;
     }
-    dev::build_bfs_slots<<<148 * 4, 256, 0, stream>>>(G.row_start, G.edge_dst, G.nnodes, p);
+    dev::build_bfs_slots<<<148 * 4, 256, 0, stream>>>(G.row_start, G.edge_dst, G.nnodes, G.nedges, p);
     cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
     if (err != cudaSuccess) {

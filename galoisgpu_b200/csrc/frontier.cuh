@@ -69,19 +69,24 @@ struct TravParams {
     uint32_t warp_degree = kDefaultWarpDegree;  // a vertex of at least this many edges is expanded by a whole warp
 };
 
-// A vertex's BFS slot from its edges [s, e): up to 4 destinations, or
-// kBfsSlotWide for a vertex of more edges or of an edge leaving the graph,
-// which goes through the CSR, whose reader reports it.
-__device__ __forceinline__ uint4 bfs_slot_of(const uint32_t *__restrict__ dst, uint32_t s, uint32_t e, uint32_t n)
+// A vertex's BFS slot from its edges [s, e) of the graph's m: up to 4
+// destinations, or kBfsSlotWide for a vertex of more edges or of an edge
+// leaving the graph, which goes through the CSR, whose reader reports it.  A
+// row outside the m edges (an unreached one of a wrapped graph, say) is not
+// read either.
+__device__ __forceinline__ uint4 bfs_slot_of(const uint32_t *__restrict__ dst, uint32_t s, uint32_t e, uint32_t m,
+                                             uint32_t n)
 {
     uint32_t x[4];
     const uint32_t d = e - s;
-    bool wide = d > 4;
+    bool wide = d > 4 || e > m;
 #pragma unroll
     for (uint32_t k = 0; k < 4; k++) {
-        x[k] = k < d && d <= 4 ? __ldg(dst + s + k) : kBfsSlotNone;
-        wide |= k < d && x[k] >= n;
+        const bool has = !wide && k < d;
+        x[k] = has ? __ldg(dst + s + k) : kBfsSlotNone;
     }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) wide |= k < d && x[k] >= n;
     return wide ? make_uint4(kBfsSlotWide, kBfsSlotNone, kBfsSlotNone, kBfsSlotNone)
                 : make_uint4(x[0], x[1], x[2], x[3]);
 }

@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(BLOCK, 1) bfs_cta_lanes(TravParams p)
     for (uint32_t w = tid; w < nwords; w += BLOCK) bits[w] = w == (p.src >> 5) ? 1u << (p.src & 31) : 0u;
     if (kStage) {
         for (uint32_t v = tid; v < n; v += BLOCK)
-            s_slots[v] = bfs_slot_of(p.edge_dst, __ldg(p.row_start + v), __ldg(p.row_start + v + 1), n);
+            s_slots[v] = bfs_slot_of(p.edge_dst, __ldg(p.row_start + v), __ldg(p.row_start + v + 1), p.nedges, n);
     }
     if (tid == 0) {
         head0[0] = p.src;

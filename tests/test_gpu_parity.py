@@ -600,3 +600,24 @@ def test_grid_bfs_kernels_by_degree(gft, orc, engine, degree, marked):
             if not marked:
                 reached = want != np.iinfo(np.int32).max
                 assert r["edges_scanned"] == int(np.diff(rs.astype(np.int64))[reached].sum())
+
+
+@pytest.mark.parametrize("claimed", [-5000, -1, 0])
+def test_one_cta_bfs_on_a_wrapped_graph_with_a_wrong_edge_count(gft, orc, engine, claimed):
+    """The one-CTA kernel stages the slots of every vertex, reached or not: rows
+    that end behind the edges the caller claims are left to the CSR, which only
+    reads those of reached vertices (here every row's edges are there)."""
+    import ctypes as C
+
+    g = gft.CSRGraph.grid(60, 60)
+    dg, keep = _wrap(gft, g.row_start, g.edge_dst)
+    h = C.c_void_p()
+    assert gft.load().gft_graph_wrap(0, g.nnodes, g.nedges + claimed, C.c_void_p(keep[0].data_ptr()),
+                                     C.c_void_p(keep[1].data_ptr()), None, C.byref(h)) == 0
+    understated = gft.DeviceGraph(h, 0)
+    for src in (0, 1799, 3599):
+        want = orc.bfs(g.row_start, g.edge_dst, src)
+        for graph in (dg, understated):
+            got, par, r = _run_bfs(gft, engine, graph, src)
+            np.testing.assert_array_equal(got, want)
+            assert r["edges_scanned"] == g.nedges
