@@ -59,6 +59,7 @@ struct TravParams {
     TraversalCtl *ctl;
     TraversalCtl *result;  // one-CTA thread-per-vertex BFS: the host's pinned copy of the results
     unsigned long long timeout_ns;
+    uint32_t slots_run;    // BFS by slots: levels the first CTA runs alone at most
     int skip_block;
     int vec_ok;
     uint32_t nedges;

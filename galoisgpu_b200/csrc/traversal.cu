@@ -393,9 +393,12 @@ constexpr int kSlotsBlock = 1024;
 constexpr uint32_t kSlotsHead = 2048;   // frontier entries in shared memory (later ones: global queue)
 constexpr uint32_t kSlotsSmall = 512;
 // Small levels the first CTA runs before the others pass a barrier: their
-// bounded wait is one of at most this many levels (about 4 ms), however long
-// the graph is.
-constexpr uint32_t kSlotsRun = 4096;
+// bounded wait is one of at most this many levels, however long the graph is.
+// A level takes 1 us on a path and 4 us with a few vertices of 7 edges, which
+// are read through the CSR; one of 1024 vertices of 32 edges may take several
+// times that, so the host cuts a run to a quarter of the wait's limit at kSlotsLevelNs
+// a level.
+constexpr uint32_t kSlotsRun = 4096, kSlotsLevelNs = 32000;
 
 // Claims up to 4 destinations in the global bitmap, all in flight together;
 // kProbe: a plain read first, so that visited vertices cost no atomic.
@@ -500,7 +503,7 @@ __global__ void __launch_bounds__(kSlotsBlock, 1) bfs_slots_grid(TravParams p)
                 if (threadIdx.x < n_in) in[threadIdx.x] = __ldcg(in_tail + threadIdx.x);
                 if (threadIdx.x == 0) s_len[1] = 0;
                 unsigned c = 0, nx = 1, cl = 2, len = n_in, claims = 0;
-                const unsigned run_end = L + kSlotsRun;
+                const unsigned run_end = L + p.slots_run;
                 __syncthreads();
                 for (;;) {
                     if (threadIdx.x == 0) s_len[cl] = 0;
@@ -928,6 +931,8 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     p.delta = (uint32_t)delta;
     p.ctl = reinterpret_cast<TraversalCtl *>(e->ctl.ptr);
     p.timeout_ns = (unsigned long long)t.timeout_ms * 1000000ull;
+    p.slots_run =
+        (uint32_t)std::clamp<unsigned long long>(p.timeout_ns / 4 / dev::kSlotsLevelNs, 1ull, dev::kSlotsRun);
     p.skip_block = t.skip;
     p.vec_ok = ((uintptr_t)G.edge_dst % 16 == 0) && (!G.edge_data || (uintptr_t)G.edge_data % 16 == 0);
     p.nedges = G.nedges;

@@ -546,8 +546,8 @@ def test_slot_bfs_reports_an_edge_leaving_the_graph(gft, engine):
 
 def test_slot_bfs_wait_is_bounded_by_levels_not_by_the_graph(gft, engine):
     """A path's 200,000 levels all run on the first CTA, about 0.2 s in all:
-    the other CTAs' waits stay below a 50 ms limit (a run of 4096 levels is
-    about 4 ms)."""
+    the other CTAs' waits stay below a 50 ms limit (a run ends after a quarter
+    of it)."""
     n = 200_000
     v = np.arange(n)
     deg = np.where((v == 0) | (v == n - 1), 1, 2)
@@ -621,3 +621,28 @@ def test_one_cta_bfs_on_a_wrapped_graph_with_a_wrong_edge_count(gft, orc, engine
             got, par, r = _run_bfs(gft, engine, graph, src)
             np.testing.assert_array_equal(got, want)
             assert r["edges_scanned"] == g.nedges
+
+
+def test_slot_bfs_wait_is_bounded_by_time(gft, orc, engine):
+    """A ladder of 5000 levels of 500 vertices, every tenth with 7 edges, read
+    through the CSR: a level of the first CTA takes 4 us, all of them 20 ms,
+    and the other CTAs wait for at most 5 ms at a time."""
+    width, depth = 500, 5000
+    n = width * depth
+    v = np.arange(n)
+    src = [v[:-width], v[width:]]
+    dst = [v[width:], v[:-width]]
+    wide = v[::10]
+    for k in range(1, 6):  # five more edges, to the same level
+        a, b = wide, wide // width * width + (wide + k) % width
+        src += [a, b]
+        dst += [b, a]
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    order = np.argsort(src, kind="stable")
+    rs = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint32)
+    dst = dst[order].astype(np.uint32)
+    assert int(np.diff(rs.astype(np.int64)).max()) <= 32 and len(dst) <= 4 * n
+    dg = gft.CSRGraph(rs, dst).copy_to_gpu()
+    want = orc.bfs(rs, dst, 0)
+    r = engine.bfs(dg, 0, tune=gft.Tune(timeout_ms=5))
+    np.testing.assert_array_equal(r["out"].cpu().numpy(), want)
