@@ -61,14 +61,21 @@ void Scratch::release()
 }
 
 namespace dev {
-__global__ void max_degree_kernel(const uint32_t *__restrict__ row_start, uint32_t n, unsigned *out)
+// out[0]: the largest out-degree; out[1]: vertices of more than 4 edges.
+__global__ void degree_stats_kernel(const uint32_t *__restrict__ row_start, uint32_t n, unsigned *out)
 {
-    unsigned m = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        m = max(m, row_start[v + 1] - row_start[v]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+    unsigned m = 0, wide = 0;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const uint32_t d = row_start[v + 1] - row_start[v];
+        m = max(m, d);
+        wide += d > 4;
+    }
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    wide = __reduce_add_sync(0xFFFFFFFFu, wide);
+    if ((threadIdx.x & 31) == 0) {
+        if (m) atomicMax(out, m);
+        if (wide) atomicAdd(out + 1, wide);
+    }
 }
 
 // Lowest index of an edge whose destination is >= n, into *first.
@@ -148,18 +155,19 @@ gft_status ensure_bfs_slots(gft_graph *g, cudaStream_t stream)
 
 gft_status graph_degree_stats(DeviceGraph &G, cudaStream_t stream)
 {
-    unsigned *d = nullptr, h = 0;
-    GFT_CUDA_TRY(cudaMallocAsync(&d, sizeof(unsigned), stream));
-    cudaError_t err = cudaMemsetAsync(d, 0, sizeof(unsigned), stream);
+    unsigned *d = nullptr, h[2] = {0, 0};
+    GFT_CUDA_TRY(cudaMallocAsync(&d, sizeof h, stream));
+    cudaError_t err = cudaMemsetAsync(d, 0, sizeof h, stream);
     if (err == cudaSuccess && G.nnodes) {
-        dev::max_degree_kernel<<<592, 256, 0, stream>>>(G.row_start, G.nnodes, d);
+        dev::degree_stats_kernel<<<592, 256, 0, stream>>>(G.row_start, G.nnodes, d);
         err = cudaGetLastError();
     }
-    if (err == cudaSuccess) err = cudaMemcpyAsync(&h, d, sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, stream);
     cudaFreeAsync(d, stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
     GFT_CUDA_TRY(err);
-    G.max_degree = h;
+    G.max_degree = h[0];
+    G.wide = h[1];
     return GFT_OK;
 }
 
@@ -308,7 +316,11 @@ gft_status gft_graph_upload(int device, const gft_csr *h, void *stream_, gft_gra
         return fail(err == cudaErrorMemoryAllocation ? GFT_ERR_OOM : GFT_ERR_CUDA, "gft_graph_upload: %s",
                     cudaGetErrorString(err));
     }
-    for (uint32_t v = 0; v < h->nnodes; v++) G.max_degree = std::max(G.max_degree, h->row_start[v + 1] - h->row_start[v]);
+    for (uint32_t v = 0; v < h->nnodes; v++) {
+        const uint32_t d = h->row_start[v + 1] - h->row_start[v];
+        G.max_degree = std::max(G.max_degree, d);
+        G.wide += d > 4;
+    }
     *out = g;
     return GFT_OK;
 }

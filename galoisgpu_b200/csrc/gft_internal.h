@@ -56,6 +56,7 @@ struct DeviceGraph {
     bool wrapped = false;
     bool symmetric = false;  // every out-edge is also an in-edge: BFS may run bottom-up
     uint32_t max_degree = 0;  // largest out-degree (set when the graph is created)
+    uint32_t wide = 0;        // vertices of more than 4 edges (likewise)
     // (edge_dst[e], edge_data[e]) interleaved, built on the first weighted
     // SSSP query and owned by the graph even when the arrays above are
     // wrapped; NULL until then.
@@ -195,8 +196,6 @@ struct DeviceScope {
     DeviceScope &operator=(const DeviceScope &) = delete;
 };
 
-// Largest out-degree of a device graph, stored in G.max_degree (one small
-// reduction kernel on `stream`, then a wait).
 // Builds g->g.edge_dw on `stream` if the graph is weighted and it is not
 // there yet, and waits for it; on an allocation failure, or while `stream`
 // is being captured, the graph keeps the separate arrays only.
@@ -204,6 +203,8 @@ gft_status ensure_edge_pairs(gft_graph *g, cudaStream_t stream);
 // Builds g->g.bfs_slots on `stream` (not under stream capture; no room:
 // left NULL, and the BFS reads the CSR).
 gft_status ensure_bfs_slots(gft_graph *g, cudaStream_t stream);
+// Sets G.max_degree and G.wide (one small reduction kernel on `stream`, then a
+// wait).
 gft_status graph_degree_stats(DeviceGraph &G, cudaStream_t stream);
 // Resident-kernel serving (resident.cu), behind gft_serve_* when
 // gft_serve_config.resident is set.

@@ -379,7 +379,7 @@ __host__ inline const void *lanes_kernel_for(int block, bool parent, bool stage)
 }
 // ---------------------------------------------------------------------------
 // The grid, a thread per frontier vertex: BFS on larger graphs of uniform low
-// degree (at most kUniformDegree edges a vertex, at most 4 on average).  Their
+// degree (bfs_by_slots).  Their
 // levels are many and small, so a level costs its chain of dependent memory
 // round trips and its barrier.  A vertex's slot (16 bytes: its up to 4
 // destinations) is one round trip where its row and its edges are two, and
@@ -695,6 +695,20 @@ bool bfs_probes_l1(const DeviceGraph &G)
     return G.max_degree > kUniformDegree || G.nedges >= 12ull * G.nnodes;
 }
 
+// Graphs whose grid-wide BFS goes by slots: of uniform low degree, with few
+// vertices whose slot only points to the CSR.  (Random graphs by the share of
+// those, slots / general kernel, unmarked, us: 2^22 vertices 2% 609 / 709, 11%
+// 515 / 506, 18% 509 / 469, 36% 525 / 431; 2^20 vertices 18% 262 / 301, 28%
+// 249 / 251, 36% 249 / 250.  Marked ones, whose large levels the general kernel
+// runs bottom-up, at 36%: 525 / 367 and 250 / 227.  No such vertex, marked: 2^22
+// with 3 edges a vertex 325 / 446, with 4 324 / 374; 2^24 with 4 1065 / 972, the
+// one case found where the degrees say too little.)
+bool bfs_by_slots(const DeviceGraph &G)
+{
+    return G.max_degree <= kUniformDegree && G.nedges <= 4ull * G.nnodes &&
+           G.wide <= G.nnodes / (G.nnodes <= 1u << 20 ? 5 : 8);
+}
+
 // Grid-wide BFS kernel for a CTA size and queue tile (0: the default tile);
 // NULL for a combination that is not built.  dir_opt: levels may run
 // bottom-up.  Tiles other than the default are built once.
@@ -859,11 +873,8 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
                                                        : (const void *)dev::bfs_single_cta<false>;
         }
     } else {
-        // Graphs of uniform low degree: the slot kernel, unless the caller asks
-        // for a shape of the general one.  On more than 4 edges a vertex
-        // most slots would only point to the CSR, and bottom-up levels may
-        // pay, which the general kernel runs.
-        if (!is_sssp && !t.shaped && !G.wrapped && G.max_degree <= kUniformDegree && G.nedges <= 4ull * G.nnodes) {
+        // Unless the caller asks for a shape of the general kernel.
+        if (!is_sssp && !t.shaped && !G.wrapped && bfs_by_slots(G)) {
             GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
             if (G.bfs_slots) {
                 slots = G.bfs_slots;

@@ -502,7 +502,8 @@ def test_bottom_up_levels_at_bitmap_edges(gft, orc, engine, n):
 
 def _slot_graph(kind):
     """Graphs of more than 2^17 vertices, at most 4 edges a vertex on average
-    and 32 at most: the slot BFS on the grid."""
+    and 32 at most: the slot BFS on the grid, except for "random", of whose
+    vertices a third have more than 4."""
     n = 150_000
     rng = np.random.default_rng(31)
     if kind == "tree":  # frontiers 1, 3, 9, ...: through every threshold, then the leaves
@@ -511,8 +512,8 @@ def _slot_graph(kind):
     elif kind == "bursts":  # a path of hubs with 29 leaves: wide vertices on tiny and on large levels
         v = np.arange(1, n)
         pairs = np.stack([np.where(v % 30 == 0, v - 30, v - v % 30), v], 1)
-    else:  # "random": a few levels of tens of thousands of vertices
-        pairs = rng.integers(0, n, size=(2 * n - n // 8, 2))
+    else:  # "random", "sparse": a few levels of tens of thousands of vertices
+        pairs = rng.integers(0, n, size=(2 * n - n // 8 if kind == "random" else 5 * n // 4, 2))
         pairs = pairs[pairs[:, 0] != pairs[:, 1]]
     a, b = np.concatenate([pairs[:, 0], pairs[:, 1]]), np.concatenate([pairs[:, 1], pairs[:, 0]])
     order = np.argsort(a, kind="stable")
@@ -521,10 +522,14 @@ def _slot_graph(kind):
     return rs, b[order].astype(np.uint32)
 
 
-@pytest.mark.parametrize("kind", ["tree", "bursts", "random"])
+@pytest.mark.parametrize("kind", ["tree", "bursts", "sparse", "random"])
 def test_slot_bfs_on_the_grid(gft, orc, engine, kind):
+    import torch
+
     rs, dst = _slot_graph(kind)
     dg = gft.CSRGraph(rs, dst).copy_to_gpu()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count  # one CTA per SM by slots, else two
+    assert engine.bfs(dg, 0)["grid_blocks"] == (2 * sms if kind == "random" else sms)
     for src in (0, 1, 149_999, 75_008):
         want = orc.bfs(rs, dst, src)
         got, par, r = _run_bfs(gft, engine, dg, src)
