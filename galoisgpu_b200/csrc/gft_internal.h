@@ -4,6 +4,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -65,7 +66,8 @@ struct DeviceGraph {
     // 16-byte slot per vertex with its up to 4 destinations (kBfsSlotNone
     // after them), or kBfsSlotWide first for a vertex of more edges or of
     // a destination outside the graph (read through the CSR).  Built
-    // on the first such BFS, owned by the graph; NULL until then.
+    // on the first such BFS on one CTA, the second one on the grid or the
+    // first call of several, owned by the graph; NULL until then.
     uint4 *bfs_slots = nullptr;
 };
 
@@ -154,7 +156,8 @@ struct LaunchShape {
 
 struct gft_graph {
     gft::DeviceGraph g;
-    std::mutex pair_mu;  // guards the lazy build of g.edge_dw
+    std::mutex pair_mu;  // guards the lazy builds of g.edge_dw and g.bfs_slots
+    std::atomic<bool> asked{false};  // a BFS by slots has run
 };
 
 struct gft_engine {
@@ -228,9 +231,11 @@ constexpr uint32_t kUniformDegree = 32;
 constexpr uint32_t kCtaMaxNodes = 1u << 17;
 constexpr uint32_t kCtaMaxEdges = 1u << 19;
 gft_status check_engine_graph(gft_engine *e, const gft_graph *g);
-// Runs one BFS (is_sssp false) or SSSP query; caller holds e->mu.
+// Runs one BFS (is_sssp false) or SSSP query; caller holds e->mu.  many: one of
+// several on this graph in the same call.
 gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32_t src, int32_t delta, int32_t *d_out,
-                         uint32_t *d_parent, const gft_tuning *tune, cudaStream_t stream, gft_stats *stats);
+                         uint32_t *d_parent, const gft_tuning *tune, cudaStream_t stream, gft_stats *stats,
+                         bool many = false);
 gft_status reach_stats(const gft_graph *g, const int32_t *d_val, cudaStream_t stream, uint64_t *v_r, uint64_t *e_r);
 gft_status pick_sources_rs(uint32_t nnodes, const uint32_t *row_start, uint64_t seed, uint32_t k, uint32_t *out);
 // CTA-mode batch kernel plumbing shared by gft_batch_* and the server.

@@ -425,7 +425,7 @@ __device__ __forceinline__ void slots_visit(const TravParams &p, bool has, uint3
                                             unsigned *err, F &&f)
 {
     uint4 sl = make_uint4(kBfsSlotNone, kBfsSlotNone, kBfsSlotNone, kBfsSlotNone);
-    if (has) sl = __ldg(p.bfs_slots + u);
+    if (has) sl = __ldca(p.bfs_slots + u);  // not __ldg: this kernel may have written them
     const bool csr = sl.x == kBfsSlotWide;
     {
         const uint32_t v[4] = {sl.x, sl.y, sl.z, sl.w};
@@ -477,6 +477,8 @@ __global__ void __launch_bounds__(kSlotsBlock, 1) bfs_slots_grid(TravParams p)
     for (uint32_t v = tid; v < n; v += nthreads) {
         p.out[v] = v == p.src ? 0 : (int32_t)kInf;
         if (kParent) p.parent[v] = v == p.src ? p.src : GFT_NO_PARENT;
+        if (p.own_slots)
+            p.own_slots[v] = bfs_slot_of(p.edge_dst, __ldg(p.row_start + v), __ldg(p.row_start + v + 1), p.nedges, n);
     }
     for (uint32_t w = tid; w < nwords; w += nthreads) p.visited[w] = w == (p.src >> 5) ? 1u << (p.src & 31) : 0u;
     if (tid == 0) {
@@ -814,7 +816,7 @@ gft_status finish(gft_engine *e, cudaStream_t stream, const LaunchShape &shape, 
 }  // namespace
 
 gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32_t src, int32_t delta, int32_t *d_out,
-                         uint32_t *d_parent, const gft_tuning *tune, cudaStream_t stream, gft_stats *stats)
+                         uint32_t *d_parent, const gft_tuning *tune, cudaStream_t stream, gft_stats *stats, bool many)
 {
     const char *what = is_sssp ? "gft_sssp" : "gft_bfs";
     GFT_TRY(check_engine_graph(e, g));
@@ -839,6 +841,29 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     if (t.hub < 32) t.hub = 32;
     DeviceScope device_scope(e->device);
     GFT_CUDA_TRY(device_scope.err);
+    // Scratch layout.
+    const uint32_t n = G.nnodes;
+    const uint32_t qcap = n;
+    const uint32_t hub_cap = std::min<uint64_t>(n, (uint64_t)G.nedges / t.hub + 1);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        size_t o = off;
+        off += align256(bytes);
+        return o;
+    };
+    size_t o_q0 = take((size_t)qcap * 4), o_q1 = take((size_t)qcap * 4);
+    size_t o_hubs = take((size_t)hub_cap * 8);
+    size_t o_vis = 0, o_vis2 = 0, o_f0 = 0, o_f1 = 0, o_qs = 0;
+    if (is_sssp) {
+        // Distances are computed in place in d_out; per vertex the engine
+        // keeps only a pile stamp.
+        o_f0 = take((size_t)qcap * 4);
+        o_f1 = take((size_t)qcap * 4);
+        o_qs = take((size_t)n * 4);
+    } else {
+        o_vis = take((size_t)((n + 31) / 32) * 4);
+        o_vis2 = take((size_t)((n + 31) / 32) * 4);
+    }
     // One CTA for small graphs (max_blocks 0 = automatic) or on request
     // (max_blocks 1); the whole cooperative grid otherwise.
     const bool single = t.max_blocks == 1 || (t.max_blocks == 0 && t.skip < 0 && G.nnodes <= kCtaMaxNodes &&
@@ -846,6 +871,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     LaunchShape shape;
     size_t dyn_smem = 0;
     const uint4 *slots = nullptr;
+    bool own_slots = false;  // the slot kernel fills slots in the engine's scratch
     bool lanes = false;  // the thread-per-vertex kernel on one CTA, which writes its results to the host itself
     if (single) {
         shape.block_threads = dev::kCtaBlock;
@@ -875,8 +901,16 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     } else {
         // Unless the caller asks for a shape of the general kernel.
         if (!is_sssp && !t.shaped && !G.wrapped && bfs_by_slots(G)) {
-            GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
-            if (G.bfs_slots) {
+            // A graph's first query fills them in the engine's scratch: the
+            // graph's own copy costs an allocation, a build and a wait, 0.4 ms,
+            // which the second query pays (first / later queries, road 400^2: 0.60 /
+            // 0.58 ms, 1.01 with the copy, 0.82 / 0.80 by the general kernel;
+            // 4096^2: 2.11 / 1.92, 2.69, 2.50 / 2.44).  Filling them each time would
+            // cost 2% at 400^2 and 7% at 4096^2.
+            own_slots = !G.bfs_slots && !many && !const_cast<gft_graph *>(g)->asked.exchange(true) &&
+                        e->scratch.grow(off + align256((size_t)n * sizeof(uint4)));
+            if (!own_slots) GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
+            if (own_slots || G.bfs_slots) {
                 slots = G.bfs_slots;
                 kern = d_parent ? (const void *)dev::bfs_slots_grid<true> : (const void *)dev::bfs_slots_grid<false>;
                 t.block = dev::kSlotsBlock;
@@ -887,29 +921,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
         if (t.max_blocks && (uint32_t)shape.blocks > t.max_blocks) shape.blocks = (int)t.max_blocks;
     }
 
-    // Scratch layout.
-    const uint32_t n = G.nnodes;
-    const uint32_t qcap = n;
-    const uint32_t hub_cap = std::min<uint64_t>(n, (uint64_t)G.nedges / t.hub + 1);
-    size_t off = 0;
-    auto take = [&](size_t bytes) {
-        size_t o = off;
-        off += align256(bytes);
-        return o;
-    };
-    size_t o_q0 = take((size_t)qcap * 4), o_q1 = take((size_t)qcap * 4);
-    size_t o_hubs = take((size_t)hub_cap * 8);
-    size_t o_vis = 0, o_vis2 = 0, o_f0 = 0, o_f1 = 0, o_qs = 0;
-    if (is_sssp) {
-        // Distances are computed in place in d_out; per vertex the engine
-        // keeps only a pile stamp.
-        o_f0 = take((size_t)qcap * 4);
-        o_f1 = take((size_t)qcap * 4);
-        o_qs = take((size_t)n * 4);
-    } else {
-        o_vis = take((size_t)((n + 31) / 32) * 4);
-        o_vis2 = take((size_t)((n + 31) / 32) * 4);
-    }
+    const size_t o_slots = own_slots ? take((size_t)n * sizeof(uint4)) : 0;
     GFT_TRY(e->scratch.ensure(off));
     char *base = reinterpret_cast<char *>(e->scratch.ptr);
 
@@ -918,7 +930,8 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     p.edge_dst = G.edge_dst;
     p.edge_data = G.edge_data;
     p.edge_dw = is_sssp ? G.edge_dw : nullptr;
-    p.bfs_slots = slots;
+    p.own_slots = own_slots ? reinterpret_cast<uint4 *>(base + o_slots) : nullptr;
+    p.bfs_slots = own_slots ? p.own_slots : slots;
     p.result = reinterpret_cast<TraversalCtl *>(e->host_ctl);
     p.nnodes = n;
     p.src = src;
@@ -1081,7 +1094,8 @@ static gft_status run_host_many(bool is_sssp, gft_engine *e, const gft_graph *g,
         int32_t *d_out = reinterpret_cast<int32_t *>(base + b * row);
         if (i >= 2) ce = cudaStreamWaitEvent(stream, e->copy_done[b], 0);
         if (ce != cudaSuccess) break;
-        st = run_traversal(is_sssp, e, g, sources[i], delta, d_out, nullptr, tune, stream, stats ? stats + i : nullptr);
+        st = run_traversal(is_sssp, e, g, sources[i], delta, d_out, nullptr, tune, stream, stats ? stats + i : nullptr,
+                           k > 1);
         if (st != GFT_OK) break;
         ce = cudaEventRecord(e->result_ready[b], stream);
         if (ce == cudaSuccess) ce = cudaStreamWaitEvent(e->copy_stream, e->result_ready[b], 0);

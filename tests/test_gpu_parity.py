@@ -651,3 +651,28 @@ def test_slot_bfs_wait_is_bounded_by_time(gft, orc, engine):
     want = orc.bfs(rs, dst, 0)
     r = engine.bfs(dg, 0, tune=gft.Tune(timeout_ms=5))
     np.testing.assert_array_equal(r["out"].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("kind", ["tree", "bursts", "sparse"])
+def test_slot_bfs_fills_the_first_query_s_slots_in_scratch(gft, orc, engine, kind):
+    """A graph's first query by slots takes no device memory beside the engine's
+    scratch, the second builds the graph's own slots, and all agree."""
+    import torch
+
+    rs, dst = _slot_graph(kind)
+    host = gft.CSRGraph(rs, dst)
+    engine.bfs(host.copy_to_gpu(), 0)  # the scratch has its size
+    dg = host.copy_to_gpu()
+    out = torch.empty(dg.nnodes, dtype=torch.int32, device="cuda")
+    par = torch.empty_like(out)
+    free = []
+    for src in (75_008, 75_008, 149_999):
+        out.fill_(-7)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        engine.bfs(dg, src, out=out, parent=par)
+        free.append(before - torch.cuda.mem_get_info()[0])
+        want = orc.bfs(rs, dst, src)
+        np.testing.assert_array_equal(out.cpu().numpy(), want)
+        assert orc.check_tree(rs, dst, None, src, want, par.cpu().numpy().view(np.uint32)) == 0
+    assert free[0] == 0 and free[1] >= 16 * dg.nnodes and free[2] == 0
