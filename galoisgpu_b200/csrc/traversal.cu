@@ -353,37 +353,24 @@ __global__ void __launch_bounds__(BLOCK, 1) bfs_cta_lanes(TravParams p)
     }
 }
 
-#ifndef GFT_LANES_BLOCK
-#define GFT_LANES_BLOCK 0  // 0: chosen from the vertex count
-#endif
-__host__ __forceinline__ int lanes_block_for(uint32_t nnodes)
+// Idle warps still pay for every level's loop top and barrier: the 256^2 grid
+// (frontiers <= 256) is fastest at 256 threads, the 362^2 road graph (random
+// sources, frontiers of 700 and more) at 1024.  Graphs here have at most
+// kCtaLocalBitsNodes vertices, those with staged slots kLaneStageNodes.
+__host__ __forceinline__ int lanes_block_for(uint32_t nnodes) { return nnodes <= (1u << 16) ? 256 : 1024; }
+template <bool kParent>
+__host__ inline const void *lanes_kernel_for(int block, bool stage)
 {
-    if (GFT_LANES_BLOCK) return GFT_LANES_BLOCK;
-    // Idle warps still pay for every level's loop top and barrier: the
-    // 256^2 grid (frontiers <= 256) is fastest at 256 threads, the 362^2
-    // road graph (random sources, frontiers of 700 and more) at 1024.
-    // Graphs here have at most kCtaLocalBitsNodes vertices.
-    return nnodes <= (1u << 16) ? 256 : 1024;
-}
-template <bool kParent, bool kStage>
-__host__ inline const void *lanes_kernel_for(int block)
-{
-    return block <= 256   ? (const void *)bfs_cta_lanes<256, kParent, kStage>
-           : block <= 512 ? (const void *)bfs_cta_lanes<512, kParent, kStage>
-                          : (const void *)bfs_cta_lanes<1024, kParent, kStage>;
-}
-__host__ inline const void *lanes_kernel_for(int block, bool parent, bool stage)
-{
-    return stage ? (parent ? lanes_kernel_for<true, true>(block) : lanes_kernel_for<false, true>(block))
-                 : (parent ? lanes_kernel_for<true, false>(block) : lanes_kernel_for<false, false>(block));
+    return stage          ? (const void *)bfs_cta_lanes<256, kParent, true>
+           : block == 256 ? (const void *)bfs_cta_lanes<256, kParent, false>
+                          : (const void *)bfs_cta_lanes<1024, kParent, false>;
 }
 // ---------------------------------------------------------------------------
 // The grid, a thread per frontier vertex: BFS on larger graphs of uniform low
-// degree (bfs_by_slots).  Their
-// levels are many and small, so a level costs its chain of dependent memory
-// round trips and its barrier.  A vertex's slot (16 bytes: its up to 4
-// destinations) is one round trip where its row and its edges are two, and
-// needs no balancing across the warp.  Levels of at most kSlotsSmall vertices,
+// degree (bfs_by_slots).  Their levels are many and small, so a level costs its
+// chain of dependent memory round trips and its barrier.  A vertex's slot (16
+// bytes: its up to 4 destinations) is one round trip where its row and its
+// edges are two, and needs no balancing across the warp.  Levels of at most kSlotsSmall vertices,
 // where a grid barrier and the global queue are most of the time, run on the
 // first CTA alone, with the frontier in its shared memory and __syncthreads
 // as the barrier; the other CTAs wait at the grid barrier.  Always top-down.
@@ -889,7 +876,8 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
             shape.block_threads = lanes_block;
             const bool stage = G.nnodes <= dev::kLaneStageNodes;
             lanes = true;
-            kern = dev::lanes_kernel_for(lanes_block, d_parent != nullptr, stage);
+            kern = d_parent ? dev::lanes_kernel_for<true>(lanes_block, stage)
+                            : dev::lanes_kernel_for<false>(lanes_block, stage);
             dyn_smem = dev::kLaneSmemBytes + (stage ? dev::kLaneStageBytes : 0);
             if (!G.wrapped && !stage) GFT_TRY(ensure_bfs_slots(const_cast<gft_graph *>(g), stream));
             slots = G.bfs_slots;
