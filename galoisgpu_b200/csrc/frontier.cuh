@@ -13,13 +13,15 @@
 namespace gft {
 namespace dev {
 
-// Edges of a hub handled per warp claim (a visitor's kHubChunk).  The last
-// chunks of a hub phase are what the grid waits for, and a frontier of a few
-// hubs has fewer chunks than warps: 512 instead of 2048 took RMAT-24 BFS from
-// 746 to 653 us, RMAT-21 top-down BFS from 675 to 627 us and RMAT-20 SSSP from
-// 1785 to 1501 us.  The few warps of a batched or served query only pay the
-// claims (512 queries, groups of 8: 77.4 ms with 512, 75.2 ms with 2048).
-constexpr uint32_t kGridHubChunk = 512, kGroupHubChunk = 2048;
+// Edges of a hub handled per warp claim, as a power of two (a visitor's
+// hub_shift).  The last chunks of a hub phase are what the grid waits for, and
+// a frontier of a few hubs has fewer chunks than warps: 512 instead of 2048
+// edges took RMAT-24 BFS from 746 to 653 us, RMAT-21 top-down BFS from 675 to
+// 627 us and RMAT-20 SSSP from 1785 to 1501 us.  A level with many chunks for
+// every warp only pays their claims and searches (hub_shift_for), as do the few
+// warps of a batched or served query (512 queries, groups of 8: 77.4 ms with
+// 512, 75.2 ms with 2048).
+constexpr uint32_t kGridHubShift = 9, kGroupHubShift = 11;
 constexpr unsigned kInf = 0x7FFFFFFFu;
 
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) { return __ldcs(p); }
@@ -55,6 +57,7 @@ struct TravParams {
     uint2 *hubs;
     uint32_t hub_cap;
     uint32_t hub_degree;
+    uint32_t hub_shift = kGridHubShift;  // 1 << hub_shift edges of a hub per warp claim
     uint32_t qcap;
     uint32_t delta;
     TraversalCtl *ctl;
@@ -151,7 +154,11 @@ template <bool kLocalBits = false, unsigned kQB = kQueueBuf, bool kL1 = false>
 struct BfsVisitorT {
     static constexpr int kBatch = GFT_BFS_BATCH;  // edges per lane in one flattened step
     static constexpr bool kEarlyRow = false;      // owner() loads nothing
-    static constexpr uint32_t kHubChunk = kL1 ? kGridHubChunk : kGroupHubChunk;  // without kL1: no hubs, or a group
+    // Without kL1: no hubs, a group, or a graph with chunks for every warp.
+    static __device__ __forceinline__ uint32_t hub_shift(const TravParams &p)
+    {
+        return kL1 ? p.hub_shift : kGroupHubShift;
+    }
     const uint32_t *__restrict__ edge_dst;
     const uint32_t *__restrict__ row_start;  // non-NULL: sum the out-degrees of claimed vertices
     unsigned long long mf;                    // that sum, per lane
@@ -266,7 +273,10 @@ template <bool kSolo, unsigned kQB = kQueueBuf>
 struct SsspVisitorT {
     static constexpr int kBatch = GFT_SSSP_BATCH;  // edges per lane in one flattened step
     static constexpr bool kEarlyRow = kSolo;       // owner() loads the distance
-    static constexpr uint32_t kHubChunk = kSolo ? kGridHubChunk : kGroupHubChunk;
+    static __device__ __forceinline__ uint32_t hub_shift(const TravParams &p)
+    {
+        return kSolo ? p.hub_shift : kGroupHubShift;
+    }
     static constexpr bool kFuse = kSolo;           // warps may expand the near vertices they found
     const uint32_t *__restrict__ edge_dst;
     const int32_t *__restrict__ edge_data;
@@ -480,7 +490,8 @@ __device__ __forceinline__ void expand_lanes(Vis &vis, const TravParams &p, bool
     }
     if (!(has && vis.active(o))) deg = 0;
     if (deg >= p.hub_degree) {
-        unsigned nch = (deg + Vis::kHubChunk - 1) / Vis::kHubChunk;
+        const uint32_t shift = Vis::hub_shift(p);
+        unsigned nch = (deg + (1u << shift) - 1) >> shift;
         unsigned long long old = atomicAdd(hub_ctr, (1ull << 32) | nch);
         unsigned h = (unsigned)(old >> 32);
         if (h < p.hub_cap) p.hubs[h] = make_uint2(v, (unsigned)old);
@@ -518,7 +529,7 @@ __device__ __forceinline__ void expand_frontier(Vis &vis, const TravParams &p, c
 }
 
 // Grid-wide processing of the hub list of one iteration: warps claim
-// Vis::kHubChunk-edge chunks; hub h owns chunks [hubs[h].y, hubs[h+1].y).
+// chunks of 1 << Vis::hub_shift() edges; hub h owns chunks [hubs[h].y, hubs[h+1].y).
 template <class Vis, class Own>
 __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsigned nh, unsigned nc,
                                             unsigned *hub_claim, unsigned gwarp, unsigned nwarps, unsigned lane)
@@ -537,8 +548,8 @@ __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsig
         if (!vis.active(o)) continue;  // warp uniform: every lane read the same hub
         const uint32_t start = __ldg(p.row_start + u);
         const uint32_t deg = __ldg(p.row_start + u + 1) - start;
-        const uint32_t off = (c - hb.y) * Vis::kHubChunk;
-        const uint32_t len = min(Vis::kHubChunk, deg - off);
+        const uint32_t shift = Vis::hub_shift(p), off = (c - hb.y) << shift;
+        const uint32_t len = min(1u << shift, deg - off);
         warp_range(vis, start + off, len, o, lane);
     }
 }
@@ -551,7 +562,7 @@ __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsig
 // graphs (R-MAT) about four chunks per warp are claimed dynamically, which
 // keeps the warps balanced.  `fine` (SSSP) claims dynamically from a quarter
 // of a 32-vertex chunk per warp on, for frontiers whose vertices cost very
-// different times: RMAT-20 SSSP 1.19x -> 1.23x beside the smaller hub chunks,
+// different times: RMAT-20 SSSP 1.49 -> 1.44 ms beside the smaller hub chunks,
 // while the BFS cases lose 2-3% to the claims.
 __device__ __forceinline__ unsigned pick_grain(unsigned n, unsigned nwarps, bool uniform, bool fine = false)
 {

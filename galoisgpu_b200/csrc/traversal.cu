@@ -678,10 +678,22 @@ const void *bfs_kernel_tile(uint32_t tile, bool l1, bool dir_opt)
 // 8-neighbour mesh 1000^2 5627 / 5450 / 5372, random of degree 8, 2^22
 // vertices 462 / 438 / 424, but of degree 16, 2^18 vertices 142 / 164 / 158;
 // with bottom-up levels, degree 6, 2^20: 181 / 185 / 194, degree 8: 305 / 298 /
-// 318.
-bool bfs_probes_l1(const DeviceGraph &G)
+// 318.  From a bitmap of 1 MB on, too many looks miss L1: unmarked R-MAT of 2^22
+// vertices 1006 / - / 1046, 2^23 1722 / - / 1649, 2^24 2889 / - / 2737.
+bool bfs_probes_l1(const DeviceGraph &G, bool dir_opt)
 {
-    return G.max_degree > kUniformDegree || G.nedges >= 12ull * G.nnodes;
+    return (G.max_degree > kUniformDegree || G.nedges >= 12ull * G.nnodes) && (dir_opt || G.nnodes <= 1u << 22);
+}
+
+// Hub chunks of a single query on the grid: where levels run top-down, or
+// relax, along most of a large graph's hubs, every warp has chunks enough, and
+// small ones only cost (chunks of 512 / 1024 / 2048 edges, us, SSSP: RMAT-20 1408
+// / 1469 / 1655, RMAT-22 3747 / 3595 / 3774, RMAT-24 13722 / 12369 / 12357; unmarked
+// BFS: RMAT-20 366 / 387 / 427, RMAT-22 1053 / 1006 / 1024; marked BFS: RMAT-20
+// 177 / 199 / 232, RMAT-24 673 / 699 / 755).
+uint32_t hub_shift_for(const DeviceGraph &G, bool dir_opt)
+{
+    return dir_opt || G.nedges < 1u << 26 ? dev::kGridHubShift : dev::kGridHubShift + 1;
 }
 
 // Graphs whose grid-wide BFS goes by slots: of uniform low degree, with few
@@ -819,7 +831,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     Tune t = resolve_tuning(tune, is_sssp);
     const bool dir_opt = !is_sssp && G.symmetric && t.direction == 0;
     const void *kern = is_sssp ? sssp_kernel_for(t.block, t.tile)
-                               : bfs_kernel_for(t.block, t.tile, bfs_probes_l1(G), dir_opt);
+                               : bfs_kernel_for(t.block, t.tile, bfs_probes_l1(G, dir_opt), dir_opt);
     if (!kern)
         return fail(GFT_ERR_INVALID_ARG,
                     "%s: block_threads must be 256, 512 or 1024 and queue_tile 0, 64, 128 or 256 "
@@ -938,6 +950,7 @@ gft_status run_traversal(bool is_sssp, gft_engine *e, const gft_graph *g, uint32
     }
     p.hub_cap = hub_cap;
     p.hub_degree = t.hub;
+    p.hub_shift = hub_shift_for(G, dir_opt);
     p.warp_degree = t.warp_degree;
     p.qcap = qcap;
     p.delta = (uint32_t)delta;
@@ -1197,7 +1210,7 @@ extern "C" gft_status gft_bfs_noalloc(const gft_graph *g, uint32_t src, int32_t 
     GFT_TRY(noalloc_scratch(G.device, &base));
 
     const bool dir_opt = G.symmetric && !(tune && tune->direction != 0);
-    const void *kern = bfs_kernel_for(kNoAllocBlock, 0, bfs_probes_l1(G), dir_opt);
+    const void *kern = bfs_kernel_for(kNoAllocBlock, 0, bfs_probes_l1(G, dir_opt), dir_opt);
     int sms = 0, occ = 0;
     GFT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, G.device));
     GFT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kNoAllocBlock, 0));
@@ -1220,6 +1233,7 @@ extern "C" gft_status gft_bfs_noalloc(const gft_graph *g, uint32_t src, int32_t 
     p.hubs = reinterpret_cast<uint2 *>(base + kNoAllocCtlBytes + 2 * kNoAllocQueueBytes + 2 * kNoAllocBitmapBytes);
     p.hub_cap = (uint32_t)std::min<uint64_t>(G.nnodes, (uint64_t)G.nedges / hub + 1);
     p.hub_degree = hub;
+    p.hub_shift = hub_shift_for(G, dir_opt);
     p.qcap = G.nnodes;
     p.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
     p.skip_block = -1;

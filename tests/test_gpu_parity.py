@@ -676,3 +676,34 @@ def test_slot_bfs_fills_the_first_query_s_slots_in_scratch(gft, orc, engine, kin
         np.testing.assert_array_equal(out.cpu().numpy(), want)
         assert orc.check_tree(rs, dst, None, src, want, par.cpu().numpy().view(np.uint32)) == 0
     assert free[0] == 0 and free[1] >= 16 * dg.nnodes and free[2] == 0
+
+
+@pytest.mark.parametrize("leaves", [1023, 1024, 1025, 4096, 70_001])
+@pytest.mark.parametrize("marked", [False, True])
+def test_hub_chunks_of_every_kernel(gft, orc, engine, leaves, marked):
+    """Two hubs of sizes at the chunks' edges (512, 1024 and 2048), joined by a
+    leaf and followed by a path: grid, one CTA, a batch's group and its one CTA,
+    BFS and SSSP."""
+    n = 2 * leaves + 50
+    pairs = [(0, 2 + i) for i in range(leaves)] + [(1, 1 + leaves + i) for i in range(leaves)]
+    pairs += [(i, i + 1) for i in range(2 * leaves + 1, n - 1)] + [(2, 2 * leaves + 1)]
+    a = np.unique(np.array(pairs), axis=0)
+    src, dst = np.concatenate([a[:, 0], a[:, 1]]), np.concatenate([a[:, 1], a[:, 0]])
+    order = np.argsort(src, kind="stable")
+    rs = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint32)
+    w = np.random.default_rng(leaves).integers(1, 100, len(src)).astype(np.int32)
+    g = gft.CSRGraph(rs, dst[order].astype(np.uint32), w)
+    dg = g.copy_to_gpu()
+    dg.symmetric = marked
+    bfs, sssp = orc.bfs(rs, g.edge_dst, 3), orc.sssp(rs, g.edge_dst, w, 3)
+    for tune in (None, {"max_blocks": 1}, {"max_blocks": 1 << 30}):
+        t = gft.Tune(**tune) if tune else None
+        np.testing.assert_array_equal(engine.bfs(dg, 3, tune=t)["out"].cpu().numpy(), bfs)
+        np.testing.assert_array_equal(engine.sssp(dg, 3, delta=50, tune=t)["out"].cpu().numpy(), sssp)
+    for group in (1, 4):
+        b = gft.Batch(engine, [{"graph": dg, "app": "bfs", "src": 3}, {"graph": dg, "app": "sssp", "src": 3, "delta": 50}],
+                      tune=gft.Tune(group_blocks=group, group_min_nodes=1 if group > 1 else 1 << 30))
+        b.run()
+        np.testing.assert_array_equal(b.queries[0]["out"].cpu().numpy(), bfs)
+        np.testing.assert_array_equal(b.queries[1]["out"].cpu().numpy(), sssp)
+        b.close()
