@@ -49,7 +49,8 @@ namespace dev {
 template <int BLOCK>
 constexpr unsigned kBatchQueueBuf = BLOCK <= 512 ? 256 : kQueueBuf;
 
-template <int BLOCK>
+// kGangs: `gangs` is given.
+template <int BLOCK, bool kGangs>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     batch_kernel(BatchJob *jobs, unsigned njobs, unsigned nbig, unsigned group, const uint4 *gangs,
                  unsigned *cursors, char *scratch, uint32_t hub_degree, TraversalCtl *gctl,
@@ -68,34 +69,39 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     const unsigned w = threadIdx.x >> 5;
 
     // Phase 1: large jobs on CTA groups.
-    const unsigned ngroups = gangs ? nbig : (nbig > 0 && group > 1) ? gridDim.x / group : 0;
-    // This CTA's group, its rank in it and the group's size stay in shared
-    // memory: kept in registers they are spilled inside the traversal loops (512
-    // queries, groups of 8: 75.2 -> 73.0 ms; 256 threads, groups of 16: 82.2 ->
-    // 78.9 ms).
-    __shared__ volatile unsigned s_gang[3];
-    if (threadIdx.x == 0) {
-        uint4 mine = make_uint4(blockIdx.x / max(group, 1u), blockIdx.x % max(group, 1u), group, 0);
-        if (gangs) mine = gangs[blockIdx.x];
-        s_gang[0] = mine.x;
-        s_gang[1] = mine.y;
-        s_gang[2] = mine.z;
+    // A planned group's numbers stay in shared memory: kept in registers they
+    // are spilled inside the traversal loops.  Groups of one size have a kernel
+    // of their own, where the size is a launch parameter (one kernel with the
+    // numbers in registers / in shared memory / two kernels: 512 queries, groups
+    // of 8 75.2 / 73.0 / 73.7 ms; BFS requests on eight graphs, one at a time on
+    // all CTAs, 1026 / 1032 / 1096 a second).
+    const unsigned ngroups = kGangs ? nbig : (nbig > 0 && group > 1) ? gridDim.x / group : 0;
+    __shared__ volatile unsigned s_gang[3];  // group, rank in it, size
+    if (kGangs) {
+        if (threadIdx.x == 0) {
+            const uint4 mine = gangs[blockIdx.x];
+            s_gang[0] = mine.x;
+            s_gang[1] = mine.y;
+            s_gang[2] = mine.z;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    const unsigned g = s_gang[0];
-    volatile unsigned &rank = s_gang[1], &size = s_gang[2];
+    const unsigned g = kGangs ? s_gang[0] : blockIdx.x / max(group, 1u);
+    const unsigned my_rank = kGangs ? 0u : blockIdx.x % max(group, 1u);
+    const auto rank = [&] { return kGangs ? (unsigned)s_gang[1] : my_rank; };
+    const auto size = [&] { return kGangs ? (unsigned)s_gang[2] : group; };
     if (g < ngroups) {
         TraversalCtl *ctl = gctl + g;
         bool first = true;
-        GridSync gs{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, size, 0, timeout_ns};
+        GridSync gs{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, size(), 0, timeout_ns};
         for (;;) {
-            if (rank == 0 && threadIdx.x == 0)
-                *u32_of(ctl->job) = !gangs ? atomicAdd(&cursors[1], 1u) : first ? g : nbig;
+            if (rank() == 0 && threadIdx.x == 0)
+                *u32_of(ctl->job) = !kGangs ? atomicAdd(&cursors[1], 1u) : first ? g : nbig;
             first = false;
             if (!gs.sync()) break;
             const unsigned j = ld_relaxed_u32(u32_of(ctl->job));
             if (j >= nbig) break;
-            if (rank == 0) {  // per-job state; the barrier lines and the job line persist
+            if (rank() == 0) {  // per-job state; the barrier lines and the job line persist
                 for (int k = 0; k < 3; k++) {
                     if (threadIdx.x == 32 * k + 0) ctl->qlen[k].v = 0;
                     if (threadIdx.x == 32 * k + 1) ctl->claim[k].v = 0;
@@ -116,19 +122,19 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
             if (!gs.sync()) break;
             if (threadIdx.x == 0) {
                 const BatchJob jb = jobs[j];
-                s_p = job_params(jb, scratch, hub_degree, ctl);
+                s_p = job_params(jb, scratch, hub_degree, ctl, size() * (BLOCK / 32));
                 s_app = jb.app;
                 s_t0 = globaltimer_ns();
             }
             __syncthreads();
             const unsigned long long t0 = s_t0;
-            const unsigned tid = rank * BLOCK + threadIdx.x;
-            GridMode m{gs, ctl, tid, size * BLOCK, tid / 32, size * BLOCK / 32};
+            const unsigned tid = rank() * BLOCK + threadIdx.x;
+            GridMode m{gs, ctl, tid, size() * BLOCK, tid / 32, size() * BLOCK / 32};
             if (s_app == 1) sssp_body<GridMode, false, QB>(s_p, m, s_near[w], s_far[w]);
             else bfs_body<GridMode, false, QB>(s_p, m, s_near[w]);
             gs.epoch = m.gs.epoch;
             const bool ok = gs.sync();
-            if (rank == 0 && threadIdx.x == 0) {
+            if (rank() == 0 && threadIdx.x == 0) {
                 TraversalCtl c;
                 c.error = ld_relaxed_u32(&ctl->error);
                 c.error_where = ctl->error_where;
@@ -151,7 +157,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
         if (j >= njobs) return;
         if (threadIdx.x == 0) {
             const BatchJob jb = jobs[j];
-            s_p = job_params(jb, scratch, hub_degree, &s_ctl);
+            s_p = job_params(jb, scratch, hub_degree, &s_ctl, BLOCK / 32);
             s_app = jb.app;
             s_t0 = globaltimer_ns();
         }
@@ -168,13 +174,14 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 
 }  // namespace dev
 
+template <bool kGangs>
 static const void *batch_kernel_ptr(int block)
 {
     switch (block) {
-    case 128: return (const void *)dev::batch_kernel<128>;
-    case 256: return (const void *)dev::batch_kernel<256>;
-    case 512: return (const void *)dev::batch_kernel<512>;
-    case 1024: return (const void *)dev::batch_kernel<1024>;
+    case 128: return (const void *)dev::batch_kernel<128, kGangs>;
+    case 256: return (const void *)dev::batch_kernel<256, kGangs>;
+    case 512: return (const void *)dev::batch_kernel<512, kGangs>;
+    case 1024: return (const void *)dev::batch_kernel<1024, kGangs>;
     }
     return nullptr;
 }
@@ -183,7 +190,7 @@ gft_status launch_batch_jobs(const BatchJob *d_jobs, unsigned njobs, unsigned nb
                              const uint4 *d_gangs, unsigned *d_cursors, char *d_scratch, uint32_t hub_degree, TraversalCtl *d_gctl,
                              int block, int blocks, cudaStream_t stream)
 {
-    const void *kern = batch_kernel_ptr(block);
+    const void *kern = d_gangs ? batch_kernel_ptr<true>(block) : batch_kernel_ptr<false>(block);
     if (!kern) return fail(GFT_ERR_INVALID_ARG, "batch: block_threads must be 128, 256, 512 or 1024");
     BatchJob *dj = const_cast<BatchJob *>(d_jobs);
     unsigned nj = njobs, nb = nbig, grp = group;
@@ -210,7 +217,7 @@ gft_status launch_batch_jobs(const BatchJob *d_jobs, unsigned njobs, unsigned nb
 
 int batch_occupancy(int block)
 {
-    const void *kern = batch_kernel_ptr(block);
+    const void *kern = batch_kernel_ptr<false>(block);
     if (!kern) return 0;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, 0) != cudaSuccess) return 0;
@@ -371,7 +378,7 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
     if (tune && tune->hub_degree) b->hub_degree = std::max<uint32_t>(32, tune->hub_degree);
     if (tune && tune->group_blocks) b->group = tune->group_blocks;
     if (tune && tune->group_min_nodes) b->group_min_nodes = tune->group_min_nodes;
-    const void *kern = batch_kernel_ptr(b->block);
+    const void *kern = batch_kernel_ptr<false>(b->block);
     if (!kern) {
         delete b;
         return fail(GFT_ERR_INVALID_ARG, "gft_batch_create: block_threads must be 128, 256, 512 or 1024");
@@ -389,8 +396,12 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
     }
     DeviceScope device_scope(e->device);
     GFT_CUDA_TRY_OR(device_scope.err, gft_batch_destroy(b));
-    int occ = 0;
+    int occ = 0, occ_gangs = 0;
     GFT_CUDA_TRY_OR(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, b->block, 0), gft_batch_destroy(b));
+    GFT_CUDA_TRY_OR(
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_gangs, batch_kernel_ptr<true>(b->block), b->block, 0),
+        gft_batch_destroy(b));
+    occ = std::min(occ, occ_gangs);
     if (occ <= 0) {
         gft_batch_destroy(b);
         return fail(GFT_ERR_CUDA, "gft_batch_create: kernel cannot be resident");

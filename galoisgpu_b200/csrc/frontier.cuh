@@ -13,15 +13,17 @@
 namespace gft {
 namespace dev {
 
-// Edges of a hub handled per warp claim, as a power of two (a visitor's
+// Edges of a hub handled per warp claim, as a power of two (TravParams::
 // hub_shift).  The last chunks of a hub phase are what the grid waits for, and
 // a frontier of a few hubs has fewer chunks than warps: 512 instead of 2048
 // edges took RMAT-24 BFS from 746 to 653 us, RMAT-21 top-down BFS from 675 to
 // 627 us and RMAT-20 SSSP from 1785 to 1501 us.  A level with many chunks for
 // every warp only pays their claims and searches (hub_shift_for), as do the few
-// warps of a batched or served query (512 queries, groups of 8: 77.4 ms with
-// 512, 75.2 ms with 2048).
-constexpr uint32_t kGridHubShift = 9, kGroupHubShift = 11;
+// warps of a batched or served query's group or CTA (512 queries, groups of 8:
+// 77.4 ms with 512, 75.2 ms with 2048; one request at a time on all CTAs, three
+// small graphs: 1148 and 997 a second).
+constexpr uint32_t kSmallHubShift = 9, kLargeHubShift = 11;
+constexpr unsigned kManyWarps = 1024;  // a group's warps from which its chunks are small
 constexpr unsigned kInf = 0x7FFFFFFFu;
 
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) { return __ldcs(p); }
@@ -57,7 +59,7 @@ struct TravParams {
     uint2 *hubs;
     uint32_t hub_cap;
     uint32_t hub_degree;
-    uint32_t hub_shift = kGridHubShift;  // 1 << hub_shift edges of a hub per warp claim
+    uint32_t hub_shift = kSmallHubShift;  // 1 << hub_shift edges of a hub per warp claim
     uint32_t qcap;
     uint32_t delta;
     TraversalCtl *ctl;
@@ -154,11 +156,6 @@ template <bool kLocalBits = false, unsigned kQB = kQueueBuf, bool kL1 = false>
 struct BfsVisitorT {
     static constexpr int kBatch = GFT_BFS_BATCH;  // edges per lane in one flattened step
     static constexpr bool kEarlyRow = false;      // owner() loads nothing
-    // Without kL1: no hubs, a group, or a graph with chunks for every warp.
-    static __device__ __forceinline__ uint32_t hub_shift(const TravParams &p)
-    {
-        return kL1 ? p.hub_shift : kGroupHubShift;
-    }
     const uint32_t *__restrict__ edge_dst;
     const uint32_t *__restrict__ row_start;  // non-NULL: sum the out-degrees of claimed vertices
     unsigned long long mf;                    // that sum, per lane
@@ -273,10 +270,6 @@ template <bool kSolo, unsigned kQB = kQueueBuf>
 struct SsspVisitorT {
     static constexpr int kBatch = GFT_SSSP_BATCH;  // edges per lane in one flattened step
     static constexpr bool kEarlyRow = kSolo;       // owner() loads the distance
-    static __device__ __forceinline__ uint32_t hub_shift(const TravParams &p)
-    {
-        return kSolo ? p.hub_shift : kGroupHubShift;
-    }
     static constexpr bool kFuse = kSolo;           // warps may expand the near vertices they found
     const uint32_t *__restrict__ edge_dst;
     const int32_t *__restrict__ edge_data;
@@ -490,8 +483,7 @@ __device__ __forceinline__ void expand_lanes(Vis &vis, const TravParams &p, bool
     }
     if (!(has && vis.active(o))) deg = 0;
     if (deg >= p.hub_degree) {
-        const uint32_t shift = Vis::hub_shift(p);
-        unsigned nch = (deg + (1u << shift) - 1) >> shift;
+        unsigned nch = (deg + (1u << p.hub_shift) - 1) >> p.hub_shift;
         unsigned long long old = atomicAdd(hub_ctr, (1ull << 32) | nch);
         unsigned h = (unsigned)(old >> 32);
         if (h < p.hub_cap) p.hubs[h] = make_uint2(v, (unsigned)old);
@@ -529,7 +521,7 @@ __device__ __forceinline__ void expand_frontier(Vis &vis, const TravParams &p, c
 }
 
 // Grid-wide processing of the hub list of one iteration: warps claim
-// chunks of 1 << Vis::hub_shift() edges; hub h owns chunks [hubs[h].y, hubs[h+1].y).
+// chunks of 1 << p.hub_shift edges; hub h owns chunks [hubs[h].y, hubs[h+1].y).
 template <class Vis, class Own>
 __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsigned nh, unsigned nc,
                                             unsigned *hub_claim, unsigned gwarp, unsigned nwarps, unsigned lane)
@@ -548,8 +540,8 @@ __device__ __forceinline__ void expand_hubs(Vis &vis, const TravParams &p, unsig
         if (!vis.active(o)) continue;  // warp uniform: every lane read the same hub
         const uint32_t start = __ldg(p.row_start + u);
         const uint32_t deg = __ldg(p.row_start + u + 1) - start;
-        const uint32_t shift = Vis::hub_shift(p), off = (c - hb.y) << shift;
-        const uint32_t len = min(1u << shift, deg - off);
+        const uint32_t off = (c - hb.y) << p.hub_shift;
+        const uint32_t len = min(1u << p.hub_shift, deg - off);
         warp_range(vis, start + off, len, o, lane);
     }
 }

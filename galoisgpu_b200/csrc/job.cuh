@@ -9,9 +9,10 @@
 namespace gft {
 namespace dev {
 
-// Parameters of one job's traversal inside the batch scratch.
+// Parameters of one job's traversal inside the batch scratch, by a group or CTA
+// on `warps` warps.
 __device__ __forceinline__ TravParams job_params(const BatchJob &jb, char *scratch, uint32_t hub_degree,
-                                                 TraversalCtl *ctl)
+                                                 TraversalCtl *ctl, unsigned warps)
 {
     char *base = scratch + jb.scratch;
     const size_t qbytes = ((size_t)jb.nnodes * 4 + 255) & ~(size_t)255;
@@ -26,6 +27,7 @@ __device__ __forceinline__ TravParams job_params(const BatchJob &jb, char *scrat
     p.q[1] = reinterpret_cast<uint32_t *>(base + qbytes);
     p.hub_cap = jb.hub_cap;
     p.hub_degree = hub_degree;
+    p.hub_shift = warps >= kManyWarps ? kSmallHubShift : kLargeHubShift;
     p.qcap = jb.nnodes;
     p.delta = jb.delta;
     p.ctl = ctl;

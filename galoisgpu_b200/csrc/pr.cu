@@ -59,7 +59,6 @@ struct PrOwn {
 struct PrInitVisitor {
     static constexpr int kBatch = 2;
     static constexpr bool kEarlyRow = false;  // owner() reads only the degree
-    static __device__ __forceinline__ uint32_t hub_shift(const TravParams &p) { return p.hub_shift; }
     const uint32_t *__restrict__ row_start;
     const uint32_t *__restrict__ edge_dst;
     float *residual;
@@ -122,7 +121,6 @@ struct PrInitVisitor {
 struct PrVisitor {
     static constexpr int kBatch = 4;
     static constexpr bool kEarlyRow = true;  // owner() pops the residual
-    static __device__ __forceinline__ uint32_t hub_shift(const TravParams &p) { return p.hub_shift; }
     const uint32_t *__restrict__ row_start;
     const uint32_t *__restrict__ edge_dst;
     float *rank, *residual, *hub_upd;
@@ -472,7 +470,7 @@ gft_status run_pr(gft_engine *e, const gft_graph *g, float *d_rank, uint32_t max
     // warps keep busy, the claims of small ones only cost (chunks of 512 / 2048
     // edges, ms: RMAT-17 5.2 / 6.1, RMAT-20 20.6 / 20.5, RMAT-22 68.6 / 65.6, RMAT-24
     // 314 / 265; a directed graph of 2^20 vertices, 16.8 M edges 15.7 / 17.2).
-    p.hub_shift = G.nedges < 1u << 26 ? dev::kGridHubShift : dev::kGroupHubShift;
+    p.hub_shift = G.nedges < 1u << 26 ? dev::kSmallHubShift : dev::kLargeHubShift;
     p.qcap = n;
     p.ctl = reinterpret_cast<TraversalCtl *>(e->ctl.ptr);
     p.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;

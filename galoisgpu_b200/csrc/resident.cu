@@ -457,7 +457,8 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) serve_resident(ResArgs a)
         const unsigned rank_cta = s_rank * a.lane_ctas + r;
         if (threadIdx.x == 0) {
             load_job_cg(&s_jb, &T.job);
-            s_p = job_params(s_jb, a.arenas + (size_t)s_team_lane * a.arena_bytes, a.hub_degree, &T.ctl);
+            s_p = job_params(s_jb, a.arenas + (size_t)s_team_lane * a.arena_bytes, a.hub_degree, &T.ctl,
+                             team_ctas * BLOCK / 32);
             s_app = s_jb.app;
             s_t0 = globaltimer_ns();
         }

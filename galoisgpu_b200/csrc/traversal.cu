@@ -689,11 +689,12 @@ bool bfs_probes_l1(const DeviceGraph &G, bool dir_opt)
 // relax, along most of a large graph's hubs, every warp has chunks enough, and
 // small ones only cost (chunks of 512 / 1024 / 2048 edges, us, SSSP: RMAT-20 1408
 // / 1469 / 1655, RMAT-22 3747 / 3595 / 3774, RMAT-24 13722 / 12369 / 12357; unmarked
-// BFS: RMAT-20 366 / 387 / 427, RMAT-22 1053 / 1006 / 1024; marked BFS: RMAT-20
-// 177 / 199 / 232, RMAT-24 673 / 699 / 755).
+// BFS: RMAT-20 366 / 387 / 427, RMAT-22 1053 / 1006 / 1024, RMAT-24 3271 / 2889 /
+// 2852; marked BFS: RMAT-20 177 / 199 / 232, RMAT-24 673 / 699 / 755).
 uint32_t hub_shift_for(const DeviceGraph &G, bool dir_opt)
 {
-    return dir_opt || G.nedges < 1u << 26 ? dev::kGridHubShift : dev::kGridHubShift + 1;
+    if (dir_opt || G.nedges < 1u << 26) return dev::kSmallHubShift;
+    return G.nnodes <= 1u << 22 ? dev::kSmallHubShift + 1 : dev::kLargeHubShift;
 }
 
 // Graphs whose grid-wide BFS goes by slots: of uniform low degree, with few
