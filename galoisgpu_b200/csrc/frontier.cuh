@@ -18,12 +18,14 @@ namespace dev {
 // a frontier of a few hubs has fewer chunks than warps: 512 instead of 2048
 // edges took RMAT-24 BFS from 746 to 653 us, RMAT-21 top-down BFS from 675 to
 // 627 us and RMAT-20 SSSP from 1785 to 1501 us.  A level with many chunks for
-// every warp only pays their claims and searches (hub_shift_for), as do the few
-// warps of a batched or served query's group or CTA (512 queries, groups of 8:
-// 77.4 ms with 512, 75.2 ms with 2048; one request at a time on all CTAs, three
-// small graphs: 1148 and 997 a second).
+// every warp only pays their claims and searches (hub_shift_for).  A batched or
+// served query's group or CTA goes by the edges that each of its warps has
+// (512 queries, groups of 8, all chunks of 512: 77.4 ms, of 2048: 73.7, by the
+// edges 72.6; one request at a time on all CTAs, three small graphs: 1148, 997
+// and 1156 a second).
 constexpr uint32_t kSmallHubShift = 9, kLargeHubShift = 11;
-constexpr unsigned kManyWarps = 1024;  // a group's warps from which its chunks are small
+constexpr uint32_t kFewEdges = 16384;  // edges a warp below which chunks are small; three times that: large
+
 constexpr unsigned kInf = 0x7FFFFFFFu;
 
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t *p) { return __ldcs(p); }

@@ -27,7 +27,9 @@ __device__ __forceinline__ TravParams job_params(const BatchJob &jb, char *scrat
     p.q[1] = reinterpret_cast<uint32_t *>(base + qbytes);
     p.hub_cap = jb.hub_cap;
     p.hub_degree = hub_degree;
-    p.hub_shift = warps >= kManyWarps ? kSmallHubShift : kLargeHubShift;
+    p.hub_shift = jb.nedges / warps < kFewEdges       ? kSmallHubShift
+                  : jb.nedges / warps < 3 * kFewEdges ? kSmallHubShift + 1
+                                                      : kLargeHubShift;
     p.qcap = jb.nnodes;
     p.delta = jb.delta;
     p.ctl = ctl;
