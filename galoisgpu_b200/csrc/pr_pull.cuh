@@ -209,7 +209,7 @@ __device__ __forceinline__ void pull_class_firsts(const PullState *st, unsigned 
 __global__ void __launch_bounds__(1024) pr_place(PullParams p)
 {
     __shared__ unsigned s_first[kPullClasses], s_rows[kPullClasses], s_base[kPullClasses];
-    if (__ldcg(&p.st->asymmetric) || __ldcg(&p.st->outside)) return;
+    if (__ldcg(&p.st->asymmetric) | __ldcg(&p.st->outside)) return;
     pull_class_firsts(p.st, s_first);
     constexpr int kPer = kPullTile / 1024;
     const unsigned lane = threadIdx.x & 31, lt = lanemask_lt();
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(512, 3) pr_relabel(PullParams p)
 {
     __shared__ PullTable s_t;
     // pr_classes' finding; one of this launch may already be seen, and ends it.
-    if (__syncthreads_or(__ldcg(&p.st->asymmetric) || __ldcg(&p.st->outside))) return;
+    if (__syncthreads_or(__ldcg(&p.st->asymmetric) | __ldcg(&p.st->outside))) return;
     pull_table(p.st, s_t);
     const unsigned lane = threadIdx.x & 31;
     const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(kPullBlock, 1) pr_sweeps(PullParams p)
     GridSync gs{&ctl->barrier.v, u32_of(ctl->release), &ctl->error, &ctl->error_where, gridDim.x, 0, p.timeout_ns};
     // The launches before this one decided: every thread sees the same words
     // (a CTA that starts after tid 0's store still finds the cause).
-    if (__ldcg(&p.st->asymmetric) || __ldcg(&p.st->outside) || __ldcg(&p.st->hash) != 0) {
+    if ((__ldcg(&p.st->asymmetric) | __ldcg(&p.st->outside)) || __ldcg(&p.st->hash) != 0) {
         if (tid == 0) p.st->asymmetric = 1;
         return;
     }
