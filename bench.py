@@ -735,13 +735,37 @@ PR_WORKLOADS = {
 PR_SECONDARY = ("pr-rmat-24", "pr-road-4096")
 
 
+def _pr_error_bound(host, rank, dev: int) -> float:
+    """An upper bound on the ranks' relative error (1-norm), from the 64-bit
+    residual of x = (1 - a) + a * A D^-1 x: the columns of A D^-1 sum to at
+    most 1, so |x - solution| <= |residual| / (1 - a)."""
+    import torch
+
+    a = float(np.float32(0.85))
+    x = torch.as_tensor(rank, device=f"cuda:{dev}").double()
+    rows = torch.from_numpy(host.row_start.astype(np.int64)).to(x.device)
+    deg = rows[1:] - rows[:-1]
+    y = x / deg.clamp(min=1)
+    sums = torch.zeros_like(x)
+    step = 1 << 25  # edges at a time
+    for lo in range(0, host.nedges, step):
+        e = torch.arange(lo, min(host.nedges, lo + step), device=x.device)
+        src = torch.searchsorted(rows, e, right=True) - 1
+        dst = torch.from_numpy(host.edge_dst[lo:lo + step].astype(np.int64)).to(x.device)
+        sums.index_add_(0, dst, y[src])
+    r = (1 - a) + a * sums - x
+    return float(r.abs().sum() / (1 - a) / x.abs().sum())
+
+
 def bench_pr(gft, orc, name: str, dev: int, steps: int = 5, warmup: int = 3, cpu_seconds: float = 10.0) -> dict:
-    """PageRank by residual push (apps/pr on this engine) to convergence on a
-    full-size seeded graph: GTEPS = edges pushed / kernel time, end to end
-    with the ranks copied to pinned host memory, and the oracle on one host
-    core, capped at the iterations that fit in about cpu_seconds (its
-    per-edge rate is the CPU baseline; the ranks are checked against the
-    oracle in the tests, at sizes the oracle finishes in seconds)."""
+    """PageRank (apps/pr on this engine) to convergence on a full-size seeded
+    graph: milliseconds per solve, and end to end with the ranks copied to
+    pinned host memory.  The graphs are symmetric, so gft_pr takes its pulled
+    sweeps; `pushes` is the same solve by the residual pushes that a directed
+    graph takes (a call with a round limit takes them too).  Both come with an
+    upper bound on their error.  The CPU figure is the oracle's pushes on one
+    host core, extrapolated: its rate per edge over the rounds that fit in
+    about cpu_seconds, and the edges that the pushes of a whole solve push."""
     import torch
 
     spec = {**PR_WORKLOADS[name], "app": "pr"}
@@ -749,53 +773,62 @@ def bench_pr(gft, orc, name: str, dev: int, steps: int = 5, warmup: int = 3, cpu
     eng = gft.Engine(dev)
     out = torch.empty(dg.nnodes, dtype=torch.float32, device=f"cuda:{dev}")
     stream = torch.cuda.current_stream(dev)
-    for _ in range(warmup):
-        r = eng.pr(dg, out=out, stream=stream)
-    torch.cuda.synchronize(dev)
-    ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    ev0.record(stream)
-    runs = [eng.pr(dg, out=out, stream=stream) for _ in range(steps)]
-    ev1.record(stream)
-    torch.cuda.synchronize(dev)
-    total_ms = ev0.elapsed_time(ev1) / steps
+
+    def timed(**kw):
+        for _ in range(warmup):
+            eng.pr(dg, out=out, stream=stream, **kw)
+        torch.cuda.synchronize(dev)
+        ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        ev0.record(stream)
+        runs = [eng.pr(dg, out=out, stream=stream, **kw) for _ in range(steps)]
+        ev1.record(stream)
+        torch.cuda.synchronize(dev)
+        return ev0.elapsed_time(ev1) / steps, runs
+
+    host = dg.download()
+    push_ms, push_runs = timed(max_iterations=0xFFFFFFFE)
+    push_err = _pr_error_bound(host, out, dev)
+    pushed = statistics.mean(x["edges_scanned"] for x in push_runs)
+    total_ms, runs = timed()
+    err = _pr_error_bound(host, out, dev)
+    sweeps = runs[0]["levels"]
+    if runs[0]["edges_scanned"] != sweeps * dg.nedges:
+        raise RuntimeError(f"{name}: gft_pr did not take its sweeps on a symmetric graph")
     kernel_ms = statistics.mean(x["kernel_ms"] for x in runs)
-    pushed = statistics.mean(x["edges_scanned"] for x in runs)
     h_out = torch.empty(dg.nnodes, dtype=torch.float32, pin_memory=True).numpy()
     t1 = time.perf_counter()
     for _ in range(steps):
         eng.pr_host(dg, h_out)
-    e2e_s = (time.perf_counter() - t1) / steps
-    host = dg.download()
+    e2e_ms = (time.perf_counter() - t1) / steps * 1e3
     cpu = {}
     iters = 1
     while True:  # grow the capped oracle run until it takes about cpu_seconds
         t2 = time.perf_counter()
         orc.pr(host.row_start, host.edge_dst, max_iterations=iters, stats=cpu)
         dt = time.perf_counter() - t2
-        if dt * 2 > cpu_seconds or iters >= runs[0]["levels"]:
+        if dt * 2 > cpu_seconds or iters >= push_runs[0]["levels"]:
             break
         iters *= 2
     peak, peak_kind = measured_peaks()
-    pops = statistics.mean(x["pushes"] for x in runs)
-    # Bytes a push step must move per edge pushed: its destination (4 B), the
-    # residual read-modify-write (8 B); per worklist entry popped: the entry,
-    # the residual exchange, the rank update and the row pair (20 B).
-    alg = 12 * pushed + 20 * pops
+    # Bytes a sweep must move: 4 per edge for the renumbered row, and per vertex
+    # its two last ranks, its factor, its new rank and its new value (20 B).
+    alg = sweeps * (4 * dg.nedges + 20 * dg.nnodes)
     res = {
-        "metric": "GTEPS (edges pushed)", "value": pushed / (total_ms * 1e6), "unit": "GTEPS",
-        "kernel_ms_mean": kernel_ms, "iterations": runs[0]["levels"], "edges_pushed": pushed, "pops": pops,
-        "steps": steps,
-        "warmup": warmup, "nodes": dg.nnodes, "edges": dg.nedges,
-        "e2e": {"value": pushed / (e2e_s * 1e9), "unit": "GTEPS", "h2d_bytes_per_step": 0,
-                "d2h_bytes_per_step": dg.nnodes * 4},
+        "metric": "PageRank solve", "value": total_ms, "unit": "ms", "higher_is_better": False,
+        "kernel_ms_mean": kernel_ms, "sweeps": sweeps, "error_bound_rel": err,
+        "pushes": {"ms": push_ms, "rounds": push_runs[0]["levels"], "edges_pushed": pushed,
+                   "error_bound_rel": push_err},
+        "steps": steps, "warmup": warmup, "nodes": dg.nnodes, "edges": dg.nedges,
+        "e2e": {"value": e2e_ms, "unit": "ms", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": dg.nnodes * 4},
         "roofline": {"bound": "hbm", "achieved": alg / (kernel_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": alg / (kernel_ms * 1e-3) / 1e9 / peak, "traffic": None, "peak_kind": peak_kind,
-                     "alg_bytes_per_launch": alg, "kernel": "pr_persistent"},
-        "cpu_baseline": {"value": cpu["edges_pushed"] / dt / 1e9, "unit": "GTEPS", "cores": 1, "kind": "port",
-                         "sample": f"the oracle's first {iters} iterations ({cpu['edges_pushed']} edges pushed, "
-                                   f"{dt:.1f} s)"},
+                     "alg_bytes_per_launch": alg, "kernel": "pr_sweeps"},
+        "cpu_baseline": {"value": pushed / (cpu["edges_pushed"] / dt) * 1e3, "unit": "ms", "cores": 1, "kind": "port",
+                         "sample": f"extrapolated from the oracle's first {iters} rounds of pushes "
+                                   f"({cpu['edges_pushed']} edges, {dt:.1f} s) to the {pushed:.3g} edges of a solve"},
     }
-    log(f"[{name}] {res['value']:.1f} GTEPS, kernel {kernel_ms:.3f} ms, {runs[0]['levels']} iterations")
+    log(f"[{name}] {total_ms:.2f} ms a solve ({sweeps} sweeps, error <= {err:.1e}); pushes {push_ms:.2f} ms "
+        f"({push_runs[0]['levels']} rounds, error <= {push_err:.1e})")
     eng.close()
     dg.free()
     return res
@@ -824,7 +857,8 @@ def bench_batch(gft, dev: int, n_queries: int = 512, reps: int = 3, delta: int =
     queries = [{"graph": g, "app": "sssp", "src": s, "delta": delta} for g, s in zip(graphs, srcs)]
     # Batch launch shapes tried (CTA size, CTAs per large query, size from
     # which a query gets a CTA group); the fastest is reported.
-    shapes = [(512, 8, 1 << 18), (512, 16, 1 << 18), (256, 16, 1 << 17), (256, 32, 1 << 18), (512, 1, 1 << 30)]
+    # The first is the engine's own choice (no group options).
+    shapes = [(512, 0, 0), (512, 8, 1 << 18), (512, 16, 1 << 18), (256, 16, 1 << 17), (256, 32, 1 << 18), (512, 1, 1 << 30)]
     tried = []
     best = None
     for blk, grp, gmin in shapes:
@@ -1469,7 +1503,7 @@ def cc_arm(args) -> int:
     is_pr, is_mis = args.workload in PR_WORKLOADS, args.workload in MIS_WORKLOADS
     fn, table = (bench_pr, PR_WORKLOADS) if is_pr else (bench_mis, MIS_WORKLOADS) if is_mis else (bench_cc, CC_WORKLOADS)
     r = fn(gft, orc, args.workload, 0, steps=args.steps, warmup=args.warmup)
-    line = {**r, "n_gpus": 1, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+    line = {"higher_is_better": True, **r, "n_gpus": 1, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32" if is_pr else "u32",
             "data": "synthetic: seeded graph generated on the device (SplitMix64 streams)",
             "config": {"workload": args.workload, **table[args.workload]}}

@@ -41,9 +41,9 @@ constexpr uint32_t kCcHubChunk = 2048;
 
 // A vertex that was x's root.  Parent links are read through L1: every find
 // ends at a root, most of them at the giant component's, and reads of one
-// address from all SMs queue up in its L2 slice (RMAT-23, whole call: 1.39 ms
-// with reads from L2, 0.54 ms through L1).  An SM may so see a link that has changed
-// since, but it is still one to an ancestor (trees only grow at the root), and
+// address from all SMs queue up in its L2 slice (RMAT-23, whole call, whose
+// time varies from box to box: 1.10-1.39 ms with reads from L2, 0.50-0.54 ms
+// through L1).  An SM may so see a link that has changed since, but it is still one to an ancestor (trees only grow at the root), and
 // cc_union finds out by its compare-and-swap.  Links are halved on the way:
 // label[x] <- label[label[x]], an ancestor of x at the time of the read and
 // therefore forever.

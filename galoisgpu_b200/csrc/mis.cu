@@ -22,9 +22,10 @@
 // they run in registers (mis_resident).  Each vertex has one
 // 64-bit word, priority << 32 | state, so testing a neighbour is one 8-byte
 // load that answers both passes' questions.  Worklist vertices go one per
-// lane; a lane scans a list of fewer than 32 edges alone and stops at the
-// first deciding neighbour, and the whole warp scans a longer one 32 edges
-// at a time.  Survivors are appended with the warp-aggregated queue.
+// lane; a lane scans a list of fewer than 32 edges alone, four at a time, and
+// stops at the first deciding neighbour; of a longer list it looks at the
+// first four, and the whole warp at the rest, 32 at a time.  Survivors are
+// appended with the warp-aggregated queue.
 #include <string.h>
 
 #include <algorithm>

@@ -420,8 +420,9 @@ class Engine:
 
     def pr(self, graph: DeviceGraph, out=None, max_iterations: int = 0xFFFFFFFF, tune: Tune | None = None,
            stream=None) -> dict:
-        """PageRank by residual push (apps/pr): ``out`` (float32 device tensor)
-        receives the unnormalised ranks; ``levels`` = worklist rounds run."""
+        """PageRank (apps/pr): ``out`` (float32 device tensor) receives the
+        unnormalised ranks; ``levels`` = sweeps over the edges (symmetric
+        graphs without an iteration limit) or worklist rounds of pushes."""
         import torch
 
         dev = torch.device("cuda", graph.device)

@@ -94,7 +94,14 @@ typedef struct gft_tuning {
                                  says; BFS there on a graph of <= 2^17 vertices
                                  and out-degrees <= 32 gives each thread a
                                  frontier vertex and always runs top-down
-                                 (levels are the same either way) */
+                                 (levels are the same either way).  So does
+                                 grid-wide BFS on a larger graph that the
+                                 library owns, of out-degrees <= 32, at most 4
+                                 edges a vertex on average and few vertices of
+                                 more than 4, unless block_threads,
+                                 blocks_per_sm, hub_degree, queue_tile or
+                                 warp_degree is given: those shape the general
+                                 kernel, which then runs                       */
     uint32_t group_blocks;    /* batches: CTAs that share one large query; 0 (and
                                  group_min_nodes 0) = each query gets CTAs in
                                  proportion to its estimated work or, when
@@ -107,7 +114,9 @@ typedef struct gft_tuning {
                                  one of the two is given, the other is 8 CTAs or
                                  262144 vertices                              */
     uint32_t direction;       /* BFS: 0 = direction-optimising when the graph is
-                                 marked symmetric, 1 = top-down only          */
+                                 marked symmetric, 1 = top-down only (no
+                                 effect on the thread-per-vertex kernels, see
+                                 max_blocks)                                  */
     uint32_t cta_small;       /* SSSP on the grid: iterations of at most this
                                  many vertices run on one CTA while the others
                                  wait (0 = engine default: 256 on graphs of
@@ -498,13 +507,22 @@ GFT_API gft_status gft_cc_host(gft_engine *e, const gft_graph *g, int32_t *h_lab
 GFT_API gft_status gft_write_cc_output(const char *path, const gft_csr *g, const int32_t *h_label);
 
 /* ---------------------------------------------------------------------------
- * PageRank by residual push: replaces apps/pr gg_main (apps/pr/kernel.cu:
- * 362-389) with its constants ALPHA = 0.85 and EPSILON = 1e-6 (:19-20).
- * d_rank (float, nnodes entries) receives the unnormalised ranks the
- * reference prints; max_iterations bounds the worklist rounds (its -x
- * option; UINT32_MAX = until converged); stats->levels = rounds run,
- * stats->edges_scanned = edges pushed along, stats->pushes = worklist
- * entries processed over all rounds.  Float
+ * PageRank: replaces apps/pr gg_main (apps/pr/kernel.cu:362-389) with its
+ * constants ALPHA = 0.85 and EPSILON = 1e-6 (:19-20).  d_rank (float, nnodes
+ * entries) receives the unnormalised ranks the reference prints;
+ * max_iterations bounds the worklist rounds (its -x option; UINT32_MAX =
+ * until converged).
+ *
+ * A graph whose edges prove symmetric (whatever its mark says), without a
+ * bound on the rounds, is solved by sweeps over all its edges, which end once
+ * no vertex's residual is above EPSILON * max(1, rank).  stats->levels = sweeps,
+ * stats->edges_scanned = sweeps * nedges, stats->pushes = sweeps * vertices
+ * with edges; of the tuning only timeout_ms applies.  The ranks do not depend
+ * on the schedule.  The engine's scratch grows to 46 bytes a vertex and 4.5 an
+ * edge; where there is no room for it, and on every other graph, the
+ * reference's residual pushes run:
+ * stats->levels = rounds, stats->edges_scanned = edges pushed along,
+ * stats->pushes = worklist entries processed over all rounds.  Their float
  * atomicAdd makes the summation order, and so the last bits of the ranks,
  * depend on the schedule, in the reference as here.
  * ------------------------------------------------------------------------- */

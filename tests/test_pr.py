@@ -249,8 +249,8 @@ def test_gpu_pr_wrapped_graph_with_a_wrong_edge_count(gft, engine, claimed):
 
 @pytest.mark.gpu
 def test_gpu_pr_on_a_directed_graph_takes_no_sweep_workspace(gft):
-    """The pushes need 16 bytes a vertex and the hub list; the sweeps 28 and
-    4.5 to 18 an edge."""
+    """The pushes need 16 bytes a vertex and the hub list, the sweeps 46 and
+    4.5 an edge."""
     rng = np.random.default_rng(7)
     n, m = 30000, 600000
     rs, ed = _csr(n, rng.integers(0, n, m), rng.integers(0, n, m))
