@@ -11,7 +11,7 @@
 //            is co-resident and its bounded barrier cannot wait on a CTA that
 //            never starts.  By default each query gets CTAs in proportion to
 //            its estimated work (plan_gangs), or, in batches of many large
-//            queries, groups of one size take them in turn (kTurnGroup); with
+//            queries, groups of one size take them in turn (turn_group); with
 //            group_blocks or group_min_nodes given, queries on graphs of at
 //            least group_min_nodes vertices run on groups of group_blocks CTAs;
 //   phase 2: the rest run on ONE CTA each (CtaMode: control block in shared
@@ -270,14 +270,37 @@ double visits(const gft_query &x)
     return n + (skewed && G.symmetric ? 0.15 : skewed ? 1.0 : 1.5) * m;
 }
 
-// From three rounds of large queries on, groups of kTurnGroup CTAs take them in
-// turn instead of all of them running at once on their shares: the graphs in
-// work at a time then fit L2, and the last round's idle groups no longer count.
-// (The package's mixed batches, 512 threads a CTA, shares / groups of 16 / of
-// 8 from 2^18 vertices: 48 queries 10.0 / 16.4 / 30.6 ms, 128: 18.4 / 19.2 /
-// 35.0, 256: 47.4 / 36.0 / 51.1, 512: 87.0 / 63.4 / 73.0; 17, 46, 92 and 184 of
-// them large.)
-constexpr uint32_t kTurnGroup = 16, kTurnNodes = 1u << 17;
+// Large queries, those on skewed graphs of this many vertices and on others
+// with this many estimated visits (SSSP on a road 700^2).
+constexpr uint32_t kTurnNodes = 1u << 17;
+constexpr double kTurnVisits = 4e6;
+
+bool large(const gft_query &x)
+{
+    const DeviceGraph &G = x.graph->g;
+    return G.max_degree > kUniformDegree ? G.nnodes >= kTurnNodes : visits(x) >= kTurnVisits;
+}
+
+// From two rounds of large queries on skewed graphs on, groups of this many
+// CTAs take the large ones in turn instead of all running at once on their
+// shares: the graphs in work at a time then fit L2.  0: shares.  (The package's
+// mixed batches of SSSP, 512 threads a CTA, shares / groups of 16 in turn / of 8:
+// 48 queries 10.0 / 16.4 / 30.6 ms, 128: 18.4 / 19.2 / 35.0, 256: 47.4 / 36.0 /
+// 51.1, 512: 87.0 / 63.4 / 73.0; half of them on skewed graphs.  100 on RMAT-18: SSSP
+// 31.4 / 17.0 / 17.5, BFS 1.94 / 1.65 / 1.44.)  Road graphs keep little in L2 and
+// use few CTAs better than many: 40 of 600^2 3.1 ms by shares, 5.6 by 16 in turn,
+// 300 of 363^2 8.3 and 22.1.
+uint32_t turn_group(const gft_query *q, uint32_t n, uint32_t blocks)
+{
+    uint64_t skewed = 0;
+    uint32_t group = 8;
+    for (uint32_t i = 0; i < n; i++)
+        if (q[i].graph->g.max_degree > kUniformDegree && large(q[i])) {
+            skewed++;
+            if (q[i].app == 1) group = 16;
+        }
+    return skewed * group >= 2ull * blocks ? group : 0u;
+}
 
 // CTAs of each query, in proportion to its estimated visits: 1 = phase 2.
 // A query of the size that a single call runs on one CTA gets one here too,
@@ -410,20 +433,16 @@ gft_status gft_batch_create(gft_engine *e, const gft_query *q, uint32_t n, const
     b->blocks = std::max(1, std::min<int>(occ, (int)bps)) * e->sms;
     // Large queries (run on CTA groups) first, then the rest; each class
     // largest first.
-    bool planned = !(tune && (tune->group_blocks || tune->group_min_nodes));
-    if (planned) {
-        uint64_t large = 0;
-        for (uint32_t i = 0; i < n; i++) large += q[i].graph->g.nnodes >= kTurnNodes;
-        if (large * kTurnGroup >= 3ull * b->blocks) {
-            planned = false;
-            b->group = kTurnGroup;
-            b->group_min_nodes = kTurnNodes;
-        }
-    }
+    const bool free_choice = !(tune && (tune->group_blocks || tune->group_min_nodes));
+    const uint32_t turns = free_choice ? turn_group(q, n, (uint32_t)b->blocks) : 0u;
+    const bool planned = free_choice && !turns;
+    if (turns) b->group = turns;
     std::vector<uint32_t> ctas(n, 1);
     if (planned) plan_gangs(q, n, (uint32_t)b->blocks, ctas);
     auto big = [&](uint32_t i) {
-        return planned ? ctas[i] > 1 : b->group > 1 && q[i].graph->g.nnodes >= b->group_min_nodes;
+        return planned ? ctas[i] > 1
+               : turns ? large(q[i])
+                       : b->group > 1 && q[i].graph->g.nnodes >= b->group_min_nodes;
     };
     std::stable_sort(b->order.begin(), b->order.end(), [&](uint32_t a, uint32_t c) {
         if (big(a) != big(c)) return big(a);

@@ -105,9 +105,9 @@ typedef struct gft_tuning {
     uint32_t group_blocks;    /* batches: CTAs that share one large query; 0 (and
                                  group_min_nodes 0) = each query gets CTAs in
                                  proportion to its estimated work or, when
-                                 the queries on graphs of 2^17 vertices and
-                                 more make three rounds of groups of 16 CTAs,
-                                 such groups take those in turn               */
+                                 large ones on skewed graphs make two rounds
+                                 of groups of 16 CTAs (8, if all are BFS),
+                                 such groups take the large ones in turn      */
     uint32_t group_min_nodes; /* batches: queries on graphs with at least this many
                                  vertices run on a CTA group (set it above every
                                  graph to run each query on one CTA).  When only

@@ -109,26 +109,27 @@ def test_batch_shares_ctas_by_work(gft, orc, engine):
     b.close()
 
 
-@pytest.mark.parametrize("n", [27, 28, 61])
+@pytest.mark.parametrize("n", [17, 18, 40])
 def test_batch_of_many_large_queries_takes_them_in_turn(gft, orc, engine, n):
-    """Queries on a graph of just over 2^17 vertices around the number (three
-    rounds of groups of 16 CTAs: 28 on 148 CTAs) from which groups take them
-    in turn, beside small ones."""
-    large, small = gft.CSRGraph.road(363, seed=51), gft.CSRGraph.road(40, seed=52)
-    assert large.nnodes >= 1 << 17
-    dl, ds = large.copy_to_gpu(), small.copy_to_gpu()
-    srcs = large.pick_sources(53, 4)
-    want = [orc.bfs(large.row_start, large.edge_dst, s) if i % 2 else
-            orc.sssp(large.row_start, large.edge_dst, large.edge_data, s) for i, s in enumerate(srcs)]
-    queries = [{"graph": dl, "app": "bfs" if i % 2 else "sssp", "src": srcs[i % 4], "delta": 20000} for i in range(n)]
-    queries += [{"graph": ds, "app": "sssp", "src": 0, "delta": 20000} for _ in range(5)]
-    want_small = orc.sssp(small.row_start, small.edge_dst, small.edge_data, 0)
-    b = gft.Batch(engine, queries, tune=gft.Tune(block_threads=1024, blocks_per_sm=1))
+    """Large queries on a skewed graph around the number (two rounds of groups
+    of 16 CTAs: 19 on 148 CTAs, one of them BFS) from which groups take them
+    in turn, beside small ones of either application and a road graph's."""
+    rmat, road, small = gft.CSRGraph.rmat(17, 8, seed=51, max_weight=255), gft.CSRGraph.road(363, seed=53), \
+        gft.CSRGraph.road(40, seed=52)
+    graphs = [rmat.copy_to_gpu(), road.copy_to_gpu(), small.copy_to_gpu()]
+    srcs = rmat.pick_sources(53, 3)
+    want = [orc.sssp(rmat.row_start, rmat.edge_dst, rmat.edge_data, s) for s in srcs]
+    queries = [({"graph": graphs[0], "app": "sssp", "src": srcs[i % 3], "delta": 20000}, want[i % 3]) for i in range(n)]
+    queries += [({"graph": graphs[0], "app": "bfs", "src": srcs[0]}, orc.bfs(rmat.row_start, rmat.edge_dst, srcs[0])),
+                ({"graph": graphs[1], "app": "sssp", "src": 5, "delta": 20000},
+                 orc.sssp(road.row_start, road.edge_dst, road.edge_data, 5)),
+                ({"graph": graphs[2], "app": "bfs", "src": 0}, orc.bfs(small.row_start, small.edge_dst, 0))]
+    b = gft.Batch(engine, [q for q, _ in queries], tune=gft.Tune(block_threads=1024, blocks_per_sm=1))
     for rep in range(2):
         for q in b.queries:
             q["out"].fill_(-7)
         b.run()
-        for i, q in enumerate(b.queries):
+        for q, (_, w) in zip(b.queries, queries):
             assert q["status"] == 0
-            np.testing.assert_array_equal(q["out"].cpu().numpy(), want[i % 4] if i < n else want_small)
+            np.testing.assert_array_equal(q["out"].cpu().numpy(), w)
     b.close()
